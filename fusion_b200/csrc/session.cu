@@ -615,6 +615,16 @@ cudaGraphExec_t take_exec(const ExecKey& key) {
 
 namespace fb {
 
+// One image of H rows of `row` bytes into dense device memory.  Dense sources
+// go as one linear copy: the copy engine takes a 2-D copy row by row and moved
+// pinned rows of 854 to 1920 bytes at 8-27 GB/s (a 640x480 frame's two images
+// 115 us, a 427x319 frame's 86 us), a linear copy of them at PCIe rate.
+static cudaError_t copy_rows(void* dst, const void* src, size_t pitch, size_t row, size_t H, cudaMemcpyKind kind,
+                             cudaStream_t st) {
+    if (pitch == row) return cudaMemcpyAsync(dst, src, row * H, kind, st);
+    return cudaMemcpy2DAsync(dst, row, src, pitch, row, H, kind, st);
+}
+
 // Host input -> the device input buffers of fr[next].
 int copy_frame_in(fb_session* s, const uint16_t* depth, size_t depth_pitch, const uint8_t* rgb, size_t rgb_pitch,
                   int on_device, cudaStream_t st) {
@@ -622,8 +632,8 @@ int copy_frame_in(fb_session* s, const uint16_t* depth, size_t depth_pitch, cons
     if (depth_pitch < (size_t)W * 2 || rgb_pitch < (size_t)W * 3) return FB_EINVAL;
     FrameBuf& N = s->fr[s->next];
     cudaMemcpyKind kind = on_device ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice;
-    FB_CUDA(cudaMemcpy2DAsync(N.depth_in, (size_t)W * 2, depth, depth_pitch, (size_t)W * 2, H, kind, st));
-    FB_CUDA(cudaMemcpy2DAsync(N.rgb, (size_t)W * 3, rgb, rgb_pitch, (size_t)W * 3, H, kind, st));
+    FB_CUDA(copy_rows(N.depth_in, depth, depth_pitch, (size_t)W * 2, H, kind, st));
+    FB_CUDA(copy_rows(N.rgb, rgb, rgb_pitch, (size_t)W * 3, H, kind, st));
     return FB_OK;
 }
 
@@ -965,10 +975,8 @@ int fb_stage_frame(fb_session* s, const uint16_t* depth, size_t depth_pitch, con
     if (g->count == 2) return FB_EINVAL;   // two frames are waiting already
     const int k = (g->head + g->count) & 1;
     FB_CUDA(cudaStreamWaitEvent(g->copy, g->freed[k], 0));   // its previous frame has been taken
-    FB_CUDA(cudaMemcpy2DAsync(g->depth[k], (size_t)W * 2, depth, depth_pitch, (size_t)W * 2, H, cudaMemcpyHostToDevice,
-                              g->copy));
-    FB_CUDA(cudaMemcpy2DAsync(g->rgb[k], (size_t)W * 3, rgb, rgb_pitch, (size_t)W * 3, H, cudaMemcpyHostToDevice,
-                              g->copy));
+    FB_CUDA(copy_rows(g->depth[k], depth, depth_pitch, (size_t)W * 2, H, cudaMemcpyHostToDevice, g->copy));
+    FB_CUDA(copy_rows(g->rgb[k], rgb, rgb_pitch, (size_t)W * 3, H, cudaMemcpyHostToDevice, g->copy));
     FB_CUDA(cudaEventRecord(g->ready[k], g->copy));
     ++g->count;
     return FB_OK;
