@@ -12,9 +12,8 @@ namespace fb {
 // ------------------------------------------------------------------ tracking
 
 constexpr int kTrackMaxBlocks = 592;   // 4 resident blocks of 256 threads per SM
-// The per-iteration kernels run in thread-block clusters of kTrackCluster
-// blocks; each cluster reduces its blocks' sums through distributed shared
-// memory into one group sum.
+// The tracking passes add their block sums by groups of kTrackCluster blocks
+// (clusters of k_track_loop, single blocks of the kernels for shared GPUs).
 constexpr int kTrackCluster = 4;
 constexpr int kTrackMaxGroups = kTrackMaxBlocks / kTrackCluster;
 constexpr int kTrackWarps = 8;         // warps per block of the per-iteration kernels
@@ -62,18 +61,37 @@ struct TrackState {
     float2 grp_rgb2[kTrackMaxGroups][32];
 };
 
+// Exchange area of k_track_loop: the blocks of a frame's tracking hand each
+// other counts, sums and poses as 16-byte slots of three words and the number
+// of the exchange they belong to, written and read as single 128-bit accesses.
+struct __align__(16) TrackSlot {
+    uint32_t x, y, z, epoch;
+};
+constexpr int kPoseCopies = 8;       // of the pose: blocks poll one of them
+constexpr int kSumSlots = 20;        // 10 slots of ICP sums, 10 of RGB sums (29 floats each)
+struct TrackSync {
+    unsigned epoch;                  // exchanges of this frame: epoch + 1, + 2, ... (one per iteration)
+    unsigned pad[31];
+    TrackSlot count[kTrackMaxBlocks];            // {correspondences, sum of squared differences, -}
+    TrackSlot sums[kTrackMaxBlocks][kSumSlots];
+    TrackSlot pose[kPoseCopies][8];              // 21 floats of a DevPose, then {failed, -, -}
+};
+
 int track_grid(int n);
-int track_cluster_grid(int n);   // track_grid rounded up to whole clusters
-int launch_track_begin(TrackState* st, cudaStream_t s);
+int track_cluster_grid(int n);   // the passes' logical grid: track_grid in whole groups
+int launch_track_begin(TrackState* st, TrackSync* sync, const int iters[3], cudaStream_t s);
+// All Gauss-Newton iterations of a frame (lv, iters and min_count by pyramid
+// level; list: track_list_bytes of level 0) in one launch; 0 launches when the sizes do not fit it (the caller
+// then launches the iterations one by one; the results are the same).
+int launch_track_loop(const TrackLevel lv[3], const int iters[3], const int min_count[3], TrackState* st,
+                      TrackSync* sync, void* list, cudaStream_t s, bool compensated);
 // residual: per-warp compact segments of photometric correspondences
-// (int2: the pixel's Sobel derivatives dx | dy << 16, packed last pixel + difference), capacity track_list_capacity;
+// (int2: the pixel's Sobel derivatives dx | dy << 16, packed last pixel + difference), track_list_bytes;
 // counts: entries per segment (kTrackMaxBlocks * kTrackWarps ints)
-// shared_gpu: the instance with four resident blocks per SM (other sessions'
-// kernels run beside it); same results as the two-block instance
 int launch_track_iter(const TrackLevel& L, TrackState* st, unsigned int* tickets, int2* residual, int* counts,
-                      int min_count, bool is_final, cudaStream_t s, bool shared_gpu = false,
-                      bool compensated = false);
-size_t track_list_capacity(int n_pixels);
+                      int min_count, bool is_final, cudaStream_t s, bool compensated = false);
+size_t track_list_bytes(int n_pixels);
+bool track_list_global(int n_pixels);   // whether k_track_loop keeps its lists in global memory
 int launch_step_icp(const TrackLevel& L, const DevPose& cur, const DevPose& last, float* partials,
                      unsigned int* ticket, double* out, cudaStream_t s);
 int launch_step_rgb(const TrackLevel& L, const DevPose& cur, const DevPose& last, float* partials,

@@ -285,9 +285,9 @@ bool carve_session(fb_session* s, const fb_config* cfg) {
                  dalloc(s, &F.rgbok[l], n);
         }
     }
-    ok = ok && dalloc(s, &s->st, 1) && dalloc(s, &s->partials, (size_t)2 * kTrackMaxBlocks * 32) &&
+    ok = ok && dalloc(s, &s->st, 1) && dalloc(s, &s->track_sync, 1) &&
          dalloc(s, &s->tickets, 4) &&
-         dalloc(s, &s->residual, track_list_capacity(s->W[0] * s->H[0])) &&
+         dalloc(s, (char**)&s->residual, track_list_bytes(s->W[0] * s->H[0])) &&
          dalloc(s, &s->counts, (size_t)kTrackMaxBlocks * kTrackWarps) &&
          dalloc(s, &s->scratch_pose, 1) && dalloc(s, &s->d_out, 1);
     MapView& m = s->map;
@@ -333,6 +333,7 @@ int reset_session(fb_session* s) {
     launch_map_reset(s->map, s->stream);
     k_init_poses<<<1, 1, 0, s->stream>>>(s->st);
     FB_CUDA(cudaMemsetAsync(s->tickets, 0, 4 * sizeof(unsigned), s->stream));
+    FB_CUDA(cudaMemsetAsync(s->track_sync, 0, sizeof(TrackSync), s->stream));
     FB_CUDA(cudaMemsetAsync(s->map.rc_cost, 0, (size_t)s->map.rc_cap * sizeof(uint32_t), s->stream));
     FB_CUDA(cudaMemsetAsync(s->map.rc_order, 0, sizeof(int), s->stream));   // no order yet: blocks in grid order
     for (int f = 0; f < 2; ++f)
@@ -432,23 +433,26 @@ int issue_frame(fb_session* s, bool track, bool fuse, bool render, bool init, un
     } else if (track) {
         // Tracker::ComputeSE3 (Tracking.cc:296-409)
         static const int min_count[3] = {2000, 1000, 100};   // MIN_ICP_COUNT, Tracking.h:102
-        n += launch_track_begin(s->st, st);
+        n += launch_track_begin(s->st, s->track_sync, c.iters, st);
         if (start) {
             Pose16 T;
             std::memcpy(T.m, start, sizeof T.m);
             fb_launch(k_track_start, (const void*)k_track_start_fused, 1, 1, 0, st, s->st, T);
             n += 1;
         }
+        const TrackLevel lv[3] = {level_view(s, 0), level_view(s, 1), level_view(s, 2)};
+        const bool comp = c.form == FB_FORM_PRECISION;
+        const int one =
+            s->shared_gpu ? 0 : launch_track_loop(lv, c.iters, min_count, s->st, s->track_sync, s->residual, st, comp);
+        n += one;
         int last_level = -1;
         for (int l = 2; l >= 0; --l)
             if (c.iters[l] > 0) last_level = l;
-        for (int l = 2; l >= 0; --l) {
-            TrackLevel lv = level_view(s, l);
+        for (int l = 2; l >= 0 && !one; --l) {
             for (int it = 0; it < c.iters[l]; ++it) {
                 launch_slot(kSlotTrack, 2 - l, it);
-                n += launch_track_iter(lv, s->st, s->tickets, s->residual, s->counts, min_count[l],
-                                       l == last_level && it == c.iters[l] - 1, st, s->shared_gpu,
-                                       c.form == FB_FORM_PRECISION);
+                n += launch_track_iter(lv[l], s->st, s->tickets, s->residual, s->counts, min_count[l],
+                                       l == last_level && it == c.iters[l] - 1, st, comp);
             }
         }
         skip = &s->st->failed;

@@ -125,7 +125,7 @@ struct fb_session {
     FrameBuf fr[2];
     int next;                  // index of NextFrame in fr
     TrackState* st;
-    float* partials;
+    TrackSync* track_sync;     // k_track_loop's exchange area
     unsigned int* tickets;
     int2* residual;            // per-block photometric correspondence segments
     int* counts;               // entries per segment

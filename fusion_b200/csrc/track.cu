@@ -3,28 +3,32 @@
 // coarse-to-fine Gauss-Newton loop of Tracker::ComputeSE3
 // (Tracking/Tracking.cc:296-409), kept entirely on the device.
 //
-// One iteration is two kernels:
+// One iteration has two passes:
 //   pass A: per pixel, the ICP row (point-to-plane, 7 wide) and the RGB
 //           correspondence search; ICP products and the RGB count / sum of
-//           squared differences are reduced.  The RGB correspondence of each
-//           pixel is kept as one packed int (last-frame pixel + difference).
-//           The current frame's per-pixel inputs are staged in shared memory
-//           by bulk copies (PixelStage), two 256-pixel chunks ahead.
-//   pass B: per pixel with a correspondence, the photometric row weighted by
-//           the robust scale sigma from pass A; products reduced.  The last
-//           block to finish also solves A x = b in FP64 (LDL^T), applies the
-//           SE(3) exponential and writes the next pose for the following
-//           iteration, with the reference's failure and acceptance tests.
+//           squared differences are reduced.  The RGB correspondences go to
+//           lists, one per warp, in the order the warp met them.  The current
+//           frame's per-pixel inputs are staged in shared memory by bulk
+//           copies in 256-pixel chunks.
+//   pass B: per correspondence, the photometric row weighted by the robust
+//           scale sigma from pass A; products reduced.  Then A x = b is
+//           solved in FP64 (LDL^T) and the SE(3) exponential applied, with
+//           the reference's failure and acceptance tests.
 // Reductions are deterministic: fixed per-thread pixel sets, warp shuffles,
-// block sums in shared memory, then the blocks' partial sums are added in
-// block order in FP64 by the last block (no atomics on values).
+// block sums in shared memory, block sums added per group of kTrackCluster
+// blocks and the groups in order in FP64 (no atomics on values).
 //
-// The per-iteration kernels come in two instances of the same code: two
-// resident blocks per SM (registers for latency: a session alone) and four
-// (half the registers, some spilled: sessions sharing the GPU leave room for
-// each other).  This file is compiled without contraction of multiplies and
-// adds into FMAs, so both instances compute the same bits.
+// A session alone runs all iterations of a frame in one cooperative kernel
+// (k_track_loop).  Sessions sharing the GPU run a kernel per pass, on a
+// quarter of the blocks and with half the registers, so that several
+// sessions' passes run side by side (k_track_a_grp / k_track_b_grp).  Both
+// walk the same logical grid and add in the same order, and this file is
+// compiled without contraction of multiplies and adds into FMAs, so both
+// compute the same bits.
 #include <cooperative_groups.h>
+
+#include <algorithm>
+#include <mutex>
 
 #include "fb_async.cuh"
 #include "fb_fused.cuh"
@@ -48,10 +52,18 @@ namespace fb {
 //     zero lies between that integer and the exact sum, so it truncates to
 //     the same integer (saturation and NaN -> 0 as the double conversion);
 //   - (double)x < c for a double c that is not a float holds exactly when x
-//     is below the smallest float above c.
+//     is below the smallest float above c (1e-3; the 0.1 of the photometric
+//     distance, whose float is that smallest one).
 __device__ __forceinline__ int trunc_half_up(float f) { return __float2int_rz(__fadd_rz(f, 0.5f)); }
 constexpr float kBelow1em3 = 0.001f;   // (double)x < 1e-3  <=>  x < 0.001f
-constexpr float kBelow0p1 = 0.1f;      // (double)x < 0.1   <=>  x < 0.1f
+// Square roots compared with a constant: the correctly rounded root is
+// monotone, so fsq(x) <= 0.1f, fsq(x) < 0.1f and fsq(x) < 0.6f hold exactly
+// up to one largest x each (NaN fails both forms).
+__device__ __forceinline__ bool sqrt_le_0p1(float x) { return x <= __int_as_float(0x3c23d70b); }
+__device__ __forceinline__ bool sqrt_lt_0p1(float x) { return x <= __int_as_float(0x3c23d709); }
+__device__ __forceinline__ bool sqrt_lt_0p6(float x) { return x <= __int_as_float(0x3eb851eb); }
+// A Sobel value / 9: one reciprocal and Markstein's correction (fd_rcp).
+__device__ __forceinline__ float ninth(int d) { return fd_rcp((float)d, 9.0f, __int_as_float(0x3de38e39)); }
 __device__ __forceinline__ float below_1em6() { return __int_as_float(0x358637be); }   // (double)x < 1e-6
 
 // Photometric correspondences are packed in 32 bits: last-frame pixel
@@ -86,9 +98,9 @@ __device__ __forceinline__ bool icp_row(const TrackLevel& L, const DevPose& cur,
     f3 ncurr_g = mv(cur.R, ncurr_c);
     f3 nlast_c = xyz(L.nlast[j]);
     f3 nlast_g = mv(last.R, nlast_c);
-    float dist = norm3(sub3(vlast_g, vcurr_g));
-    float sine = norm3(cross3(ncurr_g, nlast_g));
-    if (!(sine < 0.6f && dist <= 0.1f && !isnan(ncurr_c.x) && !isnan(nlast_c.x))) return false;
+    const f3 gap = sub3(vlast_g, vcurr_g), turn = cross3(ncurr_g, nlast_g);
+    if (!(sqrt_lt_0p6(dot3(turn, turn)) && sqrt_le_0p1(dot3(gap, gap)) && !isnan(ncurr_c.x) && !isnan(nlast_c.x)))
+        return false;
     f3 nl = mv(last.Rinv, nlast_g);
     f3 vcl = mv(last.Rinv, sub3(vcurr_g, last.t));
     f3 vll = mv(last.Rinv, sub3(vlast_g, last.t));
@@ -126,15 +138,14 @@ __device__ __forceinline__ int rgb_corresp(const TrackLevel& L, const DevPose& c
     f3 vcl = mv(last.Rinv, sub3(vcurr_g, last.t));
     float pu = fa(fd(fm(L.k.fx, vcl.x), vcl.z), L.k.cx);
     float pv = fa(fd(fm(L.k.fy, vcl.y), vcl.z), L.k.cy);
-    int u = (int)floorf(__fadd_rn(pu, 0.5f));
-    int v = (int)floorf(__fadd_rn(pv, 0.5f));
+    int u = __float2int_rd(__fadd_rn(pu, 0.5f));
+    int v = __float2int_rd(__fadd_rn(pv, 0.5f));
     if (!(u >= 0 && v >= 0 && u < W && v < H)) return -1;
     float4 vlast = L.vlast[(size_t)v * L.vp + u];
     if (isnan(vlast.x)) return -1;
     float ddx = fs(vlast.x, vcurr.x), ddy = fs(vlast.y, vcurr.y), ddz = fs(vlast.z, vcurr.z),
           ddw = fs(vlast.w, vcurr.w);
-    float nd = fsq(fa(fa(fa(fm(ddx, ddx), fm(ddy, ddy)), fm(ddz, ddz)), fm(ddw, ddw)));
-    if (!(nd < kBelow0p1)) return -1;
+    if (!sqrt_lt_0p1(fa(fa(fa(fm(ddx, ddx), fm(ddy, ddy)), fm(ddz, ddz)), fm(ddw, ddw)))) return -1;
     int gl = L.glast[(size_t)v * L.gp + u];
     if (gl == 0) return -1;
     int diff = (int)L.gcurr[(size_t)y * L.gp + x] - gl;
@@ -170,30 +181,43 @@ __device__ __forceinline__ RgbIn rgb_fetch_entry(const TrackLevel& L, int2 e) {
     return in;
 }
 
-// RGBReduction::GetRow (Reduction.cu:471-508) from fetched inputs.
-__device__ __forceinline__ void rgb_row_of(const RgbIn& in, const TrackLevel& L, const DevPose& cur,
-                                           const DevPose& last, float sigma, float row[7]) {
-    const int diff = (in.packed & 511) - 255;
+// RGBReduction::GetRow (Reduction.cu:471-508) from fetched inputs, in two
+// parts: the row's six direction values, which need no weight, and the weight
+// by the robust scale.
+struct RgbDir {
+    f3 left, c;
+};
+
+__device__ __forceinline__ RgbDir rgb_dir(f3 vlast, int dx, int dy, const TrackLevel& L, const DevPose& cur,
+                                          const DevPose& last) {
+    f3 point = mv(cur.Rinv, sub3(add3(mv(last.R, vlast), last.t), cur.t));
+    float gx = ninth(dx);
+    float gy = ninth(dy);
+    float invz = __frcp_rn(point.z);
+    RgbDir d;
+    d.left.x = gx * L.k.fx * invz;
+    d.left.y = gy * L.k.fy * invz;
+    d.left.z = -(d.left.x * point.x + d.left.y * point.y) * invz;
+    d.c = cross3(point, d.left);
+    return d;
+}
+
+__device__ __forceinline__ void rgb_weighted(const RgbDir& d, int diff, float sigma, float row[7]) {
     float w = sigma + (float)abs(diff);
     w = w < kBelow1em3 ? 1.0f : __frcp_rn(w);
     if (sigma < below_1em6()) w = 1.0f;
-    f3 vlast = xyz(in.vlast);
-    f3 point = mv(cur.Rinv, sub3(add3(mv(last.R, vlast), last.t), cur.t));
-    float gx = __fdiv_rn((float)in.dx, 9.0f);
-    float gy = __fdiv_rn((float)in.dy, 9.0f);
-    float invz = __frcp_rn(point.z);
-    f3 left;
-    left.x = gx * L.k.fx * invz;
-    left.y = gy * L.k.fy * invz;
-    left.z = -(left.x * point.x + left.y * point.y) * invz;
-    f3 c = cross3(point, left);
-    row[0] = w * left.x;
-    row[1] = w * left.y;
-    row[2] = w * left.z;
-    row[3] = w * c.x;
-    row[4] = w * c.y;
-    row[5] = w * c.z;
+    row[0] = w * d.left.x;
+    row[1] = w * d.left.y;
+    row[2] = w * d.left.z;
+    row[3] = w * d.c.x;
+    row[4] = w * d.c.y;
+    row[5] = w * d.c.z;
     row[6] = -w * (float)diff;
+}
+
+__device__ __forceinline__ void rgb_row_of(const RgbIn& in, const TrackLevel& L, const DevPose& cur,
+                                           const DevPose& last, float sigma, float row[7]) {
+    rgb_weighted(rgb_dir(xyz(in.vlast), in.dx, in.dy, L, cur, last), (in.packed & 511) - 255, sigma, row);
 }
 
 // RGBReduction::GetRow of the correspondence `packed` of pixel (x, y).
@@ -303,9 +327,9 @@ __device__ __forceinline__ PixelIn staged_pixel(const PixelStage& S, int buf, in
 // pose-dependent gathers (last vertex and normal at the ICP projection, last
 // vertex and gray value at the photometric projection) issued together.
 // Needs L.rgbok.  Returns whether the ICP row is valid; *rgb = packed
-// correspondence or -1.
+// correspondence or -1, *vphoto = the last vertex at it.
 __device__ __forceinline__ bool pixel_pass_a(const TrackLevel& L, const DevPose& cur, const DevPose& last,
-                                             const PixelIn& in, float row[7], int* rgb) {
+                                             const PixelIn& in, float row[7], int* rgb, f3* vphoto = nullptr) {
     const f3 vcurr_c = xyz(in.vc);
     const bool vnan = isnan(vcurr_c.x);
     const f3 vcurr_g = add3(mv(cur.R, vcurr_c), cur.t);
@@ -324,22 +348,24 @@ __device__ __forceinline__ bool pixel_pass_a(const TrackLevel& L, const DevPose&
         const f3 vcl = mv(last.Rinv, sub3(vcurr_g, last.t));
         const float pu = fa(fd(fm(L.k.fx, vcl.x), vcl.z), L.k.cx);
         const float pv = fa(fd(fm(L.k.fy, vcl.y), vcl.z), L.k.cy);
-        ur = (int)floorf(__fadd_rn(pu, 0.5f));
-        vr = (int)floorf(__fadd_rn(pv, 0.5f));
+        ur = __float2int_rd(__fadd_rn(pu, 0.5f));
+        vr = __float2int_rd(__fadd_rn(pv, 0.5f));
         if (ur >= 0 && vr >= 0 && ur < L.W && vr < L.H) jr = vr * L.vp + ur;
     }
     const float nanf_ = qnan();
     const float4 vl4 = ju >= 0 ? L.vlast[ju] : make_float4(nanf_, nanf_, nanf_, nanf_);
     const float4 nl4 = ju >= 0 ? L.nlast[ju] : make_float4(nanf_, nanf_, nanf_, nanf_);
-    const float4 vr4 = jr >= 0 ? L.vlast[jr] : make_float4(nanf_, nanf_, nanf_, nanf_);
+    // the two projections mostly meet the same pixel: one gather then
+    float4 vr4 = jr >= 0 && jr != ju ? L.vlast[jr] : make_float4(nanf_, nanf_, nanf_, nanf_);
     const int gl = jr >= 0 ? (int)L.glast[vr * L.gp + ur] : 0;
+    if (jr >= 0 && jr == ju) vr4 = vl4;
+    if (vphoto) *vphoto = xyz(vr4);
     // photometric residual
     *rgb = -1;
     if (jr >= 0 && !isnan(vr4.x)) {
         const float ddx = fs(vr4.x, in.vc.x), ddy = fs(vr4.y, in.vc.y), ddz = fs(vr4.z, in.vc.z),
                     ddw = fs(vr4.w, in.vc.w);
-        const float nd = fsq(fa(fa(fa(fm(ddx, ddx), fm(ddy, ddy)), fm(ddz, ddz)), fm(ddw, ddw)));
-        if (nd < kBelow0p1 && gl != 0) *rgb = pack_corr(ur, vr, in.gc - gl + 255);
+        if (sqrt_lt_0p1(fa(fa(fa(fm(ddx, ddx), fm(ddy, ddy)), fm(ddz, ddz)), fm(ddw, ddw))) && gl != 0) *rgb = pack_corr(ur, vr, in.gc - gl + 255);
     }
     // ICP row (ICPReduce::getRow, Reduction.cu:252-286)
     if (ju < 0) return false;
@@ -349,9 +375,9 @@ __device__ __forceinline__ bool pixel_pass_a(const TrackLevel& L, const DevPose&
     const f3 ncurr_g = mv(cur.R, ncurr_c);
     const f3 nlast_c = xyz(nl4);
     const f3 nlast_g = mv(last.R, nlast_c);
-    const float dist = norm3(sub3(vlast_g, vcurr_g));
-    const float sine = norm3(cross3(ncurr_g, nlast_g));
-    if (!(sine < 0.6f && dist <= 0.1f && !isnan(ncurr_c.x) && !isnan(nlast_c.x))) return false;
+    const f3 gap = sub3(vlast_g, vcurr_g), turn = cross3(ncurr_g, nlast_g);
+    if (!(sqrt_lt_0p6(dot3(turn, turn)) && sqrt_le_0p1(dot3(gap, gap)) && !isnan(ncurr_c.x) && !isnan(nlast_c.x)))
+        return false;
     const f3 nl = mv(last.Rinv, nlast_g);
     const f3 vcl = mv(last.Rinv, sub3(vcurr_g, last.t));
     const f3 vll = mv(last.Rinv, sub3(vlast_g, last.t));
@@ -376,29 +402,8 @@ __device__ __forceinline__ void add_products(const float row[7], float acc[29]) 
 }
 
 // Pass B's rows of one warp segment (n entries): lane l adds the rows of
-// entries l, l + 32, ... in that order.  The next entry's loads are issued
-// before the current row is computed, so the list read and the dependent
-// gathers of two entries overlap (the clustered forms, with registers to
-// spare; the 64-register group forms add the rows one at a time,
-// add_segment_rows_seq: 2 % faster there, the same sums).
-// `a`: the fetch of entry `lane` (when lane < n), issued by the caller before
-// the robust scale is known.
+// entries l, l + 32, ... in that order.
 __device__ __forceinline__ void add_segment_rows(const TrackLevel& L, const DevPose& cur, const DevPose& last,
-                                                 float sigma, const int2* seg, int n, int lane, float acc[29],
-                                                 RgbIn a) {
-    int i = lane;
-    if (i >= n) return;
-    for (; i < n; i += 32) {
-        RgbIn b = a;
-        if (i + 32 < n) b = rgb_fetch_entry(L, seg[i + 32]);
-        float row[7];
-        rgb_row_of(a, L, cur, last, sigma, row);
-        add_products(row, acc);
-        a = b;
-    }
-}
-
-__device__ __forceinline__ void add_segment_rows_seq(const TrackLevel& L, const DevPose& cur, const DevPose& last,
                                                      float sigma, const int2* seg, int n, int lane, float acc[29]) {
     for (int i = lane; i < n; i += 32) {
         float row[7];
@@ -503,91 +508,6 @@ __device__ __forceinline__ unsigned int ticket_acq_rel(unsigned int* t) {
 
 // ----------------------------------------------------------- FP64 solver
 
-// LDL^T of the 6x6 symmetric positive definite normal matrix and the solve
-// (the effect of Eigen's ldlt().solve at Tracking.cc:388; for SPD systems the
-// factorisation needs no pivoting).  Fully unrolled so that every array stays
-// in registers.
-__device__ __forceinline__ void ldlt6(const double* A, const double* b, double* x) {
-    double L[6][6], D[6], Dinv[6], y[6];
-#pragma unroll
-    for (int k = 0; k < 6; ++k) {
-        double d = A[k * 6 + k];
-#pragma unroll
-        for (int j = 0; j < k; ++j) d -= L[k][j] * L[k][j] * D[j];
-        D[k] = d;
-        const double inv = 1.0 / d;
-        Dinv[k] = inv;
-#pragma unroll
-        for (int i = k + 1; i < 6; ++i) {
-            double t = A[i * 6 + k];
-#pragma unroll
-            for (int j = 0; j < k; ++j) t -= L[i][j] * L[k][j] * D[j];
-            L[i][k] = t * inv;
-        }
-    }
-#pragma unroll
-    for (int i = 0; i < 6; ++i) {
-        double t = b[i];
-#pragma unroll
-        for (int j = 0; j < i; ++j) t -= L[i][j] * y[j];
-        y[i] = t;
-    }
-#pragma unroll
-    for (int i = 0; i < 6; ++i) y[i] *= Dinv[i];
-#pragma unroll
-    for (int i = 5; i >= 0; --i) {
-        double t = y[i];
-#pragma unroll
-        for (int j = i + 1; j < 6; ++j) t -= L[j][i] * x[j];
-        x[i] = t;
-    }
-}
-
-// exp of the se(3) tangent (upsilon, omega) -- the Sophus::SE3d::exp of
-// Tracking.cc:389 restated from the mathematics (Rodrigues rotation, left
-// Jacobian for the translation, Taylor series near zero).
-__device__ __forceinline__ void se3_exp(const double* xi, double* T) {
-    const double* u = xi;
-    const double* w = xi + 3;
-    double th2 = w[0] * w[0] + w[1] * w[1] + w[2] * w[2];
-    double th = sqrt(th2);
-    double W[9] = {0, -w[2], w[1], w[2], 0, -w[0], -w[1], w[0], 0};
-    double W2[9];
-#pragma unroll
-    for (int i = 0; i < 3; ++i)
-#pragma unroll
-        for (int j = 0; j < 3; ++j) {
-            double s = 0;
-#pragma unroll
-            for (int k = 0; k < 3; ++k) s += W[i * 3 + k] * W[k * 3 + j];
-            W2[i * 3 + j] = s;
-        }
-    double a, b, c;
-    if (th < 1e-5) {
-        a = 1 - th2 / 6 + th2 * th2 / 120;
-        b = 0.5 - th2 / 24 + th2 * th2 / 720;
-        c = 1.0 / 6 - th2 / 120 + th2 * th2 / 5040;
-    } else {
-        double s = sin(th), co = cos(th);
-        a = s / th;
-        b = (1 - co) / th2;
-        c = (th - s) / (th2 * th);
-    }
-#pragma unroll
-    for (int i = 0; i < 3; ++i) {
-        double vi[3];
-#pragma unroll
-        for (int j = 0; j < 3; ++j) {
-            double I = (i == j) ? 1.0 : 0.0;
-            T[i * 4 + j] = I + a * W[i * 3 + j] + b * W2[i * 3 + j];
-            vi[j] = I + b * W[i * 3 + j] + c * W2[i * 3 + j];
-        }
-        T[i * 4 + 3] = vi[0] * u[0] + vi[1] * u[1] + vi[2] * u[2];
-    }
-    T[12] = T[13] = T[14] = 0;
-    T[15] = 1;
-}
-
 __device__ __forceinline__ void mat4_mul(const double* A, const double* B, double* C) {
     double T[16];
 #pragma unroll
@@ -626,25 +546,12 @@ __device__ double euler_sin_norm(const double* T) {
     return sqrt(sa * sa + sb * sb + sc * sc);
 }
 
-__device__ __forceinline__ void unpack29(const double* s, double* A, double* b) {
-    int n = 0;
-#pragma unroll
-    for (int i = 0; i < 6; ++i)
-#pragma unroll
-        for (int j = i; j < 7; ++j) {
-            double v = s[n++];
-            if (j == 6)
-                b[i] = v;
-            else
-                A[j * 6 + i] = A[i * 6 + j] = v;
-        }
-}
-
 // ------------------------------------------------------------------ kernels
 
 // Frame start: the next pose starts from the last pose (TrackFrame's
 // bootstrap fallback, Tracking.cc:156-159) and delta is the identity.
-__device__ __forceinline__ void track_begin_body(const BlockCtx&, TrackState* st) {
+__device__ __forceinline__ void track_begin_body(const BlockCtx&, TrackState* st, TrackSync* sync, unsigned step) {
+    sync->epoch += step;   // the frame's exchanges (k_track_loop) are numbered from here
     for (int i = 0; i < 16; ++i) {
         st->pose[i] = st->last_pose[i];
         st->init_pose[i] = st->last_pose[i];
@@ -656,7 +563,9 @@ __device__ __forceinline__ void track_begin_body(const BlockCtx&, TrackState* st
     st->icp_error = st->rgb_error = qnan();
     st->icp_count = st->rgb_count = 0;
 }
-__global__ void k_track_begin(TrackState* st) { track_begin_body(own_ctx(), st); }
+__global__ void k_track_begin(TrackState* st, TrackSync* sync, unsigned step) {
+    track_begin_body(own_ctx(), st, sync, step);
+}
 FB_FUSED_KERNEL(k_track_begin, track_begin_body, 32)
 
 // Fixed-order FP64 sum of nv values over nb block partials laid out as
@@ -685,29 +594,13 @@ __device__ void reduce_partials(const float* __restrict__ partials, int nb, int 
     }
 }
 
-// Capacity of the per-warp correspondence segments for n pixels: every warp
-// of the pass-A grid gets as many slots as the pixels it visits.
-size_t track_list_capacity(int n) {
+// Bytes of the per-warp correspondence segments for n pixels: every warp of
+// the pass-A grid gets as many slots as the pixels it visits, of 8 bytes, or
+// of 18 where k_track_loop keeps its lists there too.
+size_t track_list_bytes(int n) {
     const int g = track_cluster_grid(n);
     const int iters = (n + g * 256 - 1) / (g * 256);
-    return (size_t)g * iters * 256;
-}
-
-// Sum of a cluster's block sums: rank 0's first `nv` threads add value t of
-// every block of the cluster in rank order (FP64) through distributed shared
-// memory.  Every block of the cluster must call it (it holds two cluster
-// barriers: the block sums are complete before rank 0 reads, and stay alive
-// until it has read them).  Returns the sum in rank 0's threads t < nv.
-template <typename T>
-__device__ __forceinline__ double cluster_sum(cg::cluster_group& cl, T* s_vals, int nv) {
-    double v = 0;
-    cl.sync();
-    if (cl.block_rank() == 0 && (int)threadIdx.x < nv) {
-#pragma unroll
-        for (int r = 0; r < kTrackCluster; ++r) v += (double)cl.map_shared_rank(s_vals, r)[threadIdx.x];
-    }
-    cl.sync();
-    return v;
+    return (size_t)g * iters * 256 * (track_list_global(n) ? 18 : sizeof(int2));
 }
 
 // Compensated FP32 (the precision form's reduction).  two_sum is Knuth's
@@ -729,117 +622,6 @@ __device__ __forceinline__ float2 pair_add(float2 x, float2 y) {
     return make_float2(hi, __fsub_rn(lo, __fsub_rn(hi, s.x)));
 }
 
-// pass A (one cluster of kTrackCluster blocks per group): ICP rows reduced per
-// block, then per cluster into the group sums; RGB correspondences appended by
-// each warp to its own segment of `list` in pixel-visit order (ballot +
-// popc: deterministic, no block barrier in the pixel loop), with the
-// correspondence count and sum of squared differences reduced the same way
-// (integers below 2^53, exact as doubles).  L.rgbok must be set.
-template <int kMinBlocks, bool kComp>
-__global__ void __cluster_dims__(kTrackCluster, 1, 1) __launch_bounds__(256, kMinBlocks)
-    k_track_a(TrackLevel L, TrackState* st, int2* list, int* counts) {
-    const int N = L.W * L.H;
-    const int G = gridDim.x, lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    int p = blockIdx.x * 256 + threadIdx.x;
-    if (st->failed) return;   // uniform over the grid: written by an earlier kernel
-    // the pose loads are in flight while the first chunks are staged
-    const DevPose cur = st->cur, last = st->last;
-    cg::cluster_group cl = cg::this_cluster();
-    __shared__ float sm[8 * 32];
-    __shared__ long long smll[32];
-    __shared__ double s_vals[32];
-    __shared__ PixelStage stg;
-    const int iters = (N + G * 256 - 1) / (G * 256);
-    const int base = blockIdx.x * 256;
-    if (threadIdx.x == 0) {
-        mbar_init(&stg.bar[0], 1);
-        mbar_init(&stg.bar[1], 1);
-        for (int c = 0; c < 2 && c < iters && base + c * G * 256 < N; ++c) stage_chunk(stg, c, L, base + c * G * 256, N);
-    }
-    __syncthreads();
-    float acc[29];
-#pragma unroll
-    for (int k = 0; k < 29; ++k) acc[k] = 0.f;
-    long long rc = 0, rsq = 0;
-    const int gw = blockIdx.x * kTrackWarps + wid;
-    int2* seg = list + (size_t)gw * iters * 32;
-    const unsigned lt = (1u << lane) - 1u;
-    int run = 0;
-    for (int k = 0; k < iters; ++k, p += G * 256) {
-        if (base + k * G * 256 >= N) break;   // uniform: no pixel of this block's chunk k
-        const int buf = k & 1;
-        if (!take_chunk(stg, buf, (uint32_t)(k >> 1))) {
-            if (threadIdx.x == 0) atomicOr((unsigned*)&st->failed, 2u);
-            return;
-        }
-        PixelIn in;
-        if (p < N) in = staged_pixel(stg, buf, threadIdx.x);
-        __syncthreads();   // buffer `buf` is read: chunk k + 2 may overwrite it
-        if (threadIdx.x == 0 && k + 2 < iters && base + (k + 2) * G * 256 < N)
-            stage_chunk(stg, buf, L, base + (k + 2) * G * 256, N);
-        int r = -1;
-        if (p < N) {
-            float row[7];
-            if (pixel_pass_a(L, cur, last, in, row, &r)) add_products(row, acc);
-            if (r != -1) {
-                int d = (r & 511) - 255;
-                rc += 1;
-                rsq += d * d;
-            }
-        }
-        const unsigned m = __ballot_sync(0xffffffffu, r != -1);
-        if (r != -1) seg[run + __popc(m & lt)] = make_int2(in.dxy, r);
-        run += __popc(m);
-    }
-    if (lane == 0) counts[gw] = run;
-    const float bsum = block_sum29(acc, sm);
-    // block_sum_ll leaves the total in lane 0 of warp 0
-    const long long bc = __shfl_sync(0xffffffffu, block_sum_ll(rc, smll), 0);
-    const long long bs = __shfl_sync(0xffffffffu, block_sum_ll(rsq, smll), 0);
-    if constexpr (kComp) {
-        // precision form: block sums as compensated FP32 pairs, counts as integers
-        __shared__ float s_f[32];
-        __shared__ long long s_c[2];
-        if (wid == 0) s_f[lane] = lane < 29 ? bsum : 0.f;
-        if (threadIdx.x == 0) {
-            s_c[0] = bc;
-            s_c[1] = bs;
-        }
-        cl.sync();
-        if (cl.block_rank() == 0 && threadIdx.x < 31) {
-            const int g = blockIdx.x / kTrackCluster;
-            if (threadIdx.x < 29) {
-                float2 acc = make_float2(0.f, 0.f);
-#pragma unroll
-                for (int r = 0; r < kTrackCluster; ++r)
-                    acc = pair_add(acc, make_float2(cl.map_shared_rank(s_f, r)[threadIdx.x], 0.f));
-                st->grp_icp2[g][threadIdx.x] = acc;
-            } else {
-                long long t = 0;
-#pragma unroll
-                for (int r = 0; r < kTrackCluster; ++r) t += cl.map_shared_rank(s_c, r)[threadIdx.x - 29];
-                if (threadIdx.x == 29)
-                    st->grp_cnt[g] = t;
-                else
-                    st->grp_sq[g] = t;
-            }
-        }
-        cl.sync();
-        return;
-    }
-    if (wid == 0) s_vals[lane] = lane < 29 ? (double)bsum : lane == 29 ? (double)bc : lane == 30 ? (double)bs : 0.0;
-    const double v = cluster_sum(cl, s_vals, 31);
-    if (cl.block_rank() == 0 && threadIdx.x < 31) {
-        const int g = blockIdx.x / kTrackCluster;
-        if (threadIdx.x < 29)
-            st->grp_icp[g][threadIdx.x] = v;
-        else if (threadIdx.x == 29)
-            st->grp_cnt[g] = (long long)v;
-        else
-            st->grp_sq[g] = (long long)v;
-    }
-}
-
 // Staging of the tracker state for the solve of one iteration.
 struct SolveIO {
     double delta[16], last_pose[16], init_pose[16], pose[16];
@@ -849,7 +631,209 @@ struct SolveIO {
     int updated;   // delta, pose and cur hold a Gauss-Newton update
 };
 
-__device__ void solve_staged(SolveIO& io, const double* s, int min_count, int is_final);
+// The acceptance test of the last iteration (Tracking.cc:398-408), one thread.
+__device__ __noinline__ bool accept_pose(const SolveIO& io) {
+    double pinv[16], p[16];
+    mat4_rigid_inv(io.init_pose, pinv);
+    mat4_mul(pinv, io.pose, p);
+    const double tn = sqrt(p[3] * p[3] + p[7] * p[7] + p[11] * p[11]);
+    return io.icp_error < 0.0001f && euler_sin_norm(p) <= 0.1 && tn <= 0.1;
+}
+
+// Shared scratch of solve_block.
+struct SolveTmp {
+    double W[9], V[9], T[16], dinv[16];
+    double delta[16], pose[16];
+    DevPose cur;
+};
+
+// The count and error tests of one iteration (Tracking.cc:319-360), one thread.
+__device__ __forceinline__ void solve_checks(SolveIO& io, const double* s, int min_count) {
+    const float r1 = (float)s[32 + 28];
+    const float rgb_err = sqrtf((float)s[32 + 27]) / r1;
+    io.rgb_error = rgb_err;
+    io.rgb_count = r1;
+    bool fail = isnan(rgb_err) || (int)r1 < min_count;
+    if (!fail) {
+        const float q1 = (float)s[28];
+        const float icp_err = sqrtf((float)s[27]) / q1;
+        io.icp_error = icp_err;
+        io.icp_count = q1;
+        fail = isnan(icp_err) || (int)q1 < min_count;
+    }
+    io.failed = fail ? 1 : 0;
+    io.updated = fail ? 0 : 1;
+}
+
+// The Gauss-Newton step (Tracking.cc:361-394) from the FP64 sums s (ICP in
+// s[0..28], RGB in s[32..60]): tmp.delta, pose and cur from io.delta and
+// io.last_pose.
+//
+// One warp; every value is computed by the operations, in the order, of the
+// plain one-thread form (LDL^T without pivoting -- the normal matrix is
+// positive definite --, substitution, Sophus::SE3d::exp from the mathematics,
+// two 4x4 products).  It is a chain of dependent FP64 operations between two
+// iterations: one thread took 1.8 us (3.1 us where its spills met the pixel
+// passes' registers).  Row i of the factorisation is lane i's (all lanes
+// follow the divisions), the elements of the small matrices are one lane's
+// each, sine and cosine come from one sincos (the same bits as sin and cos),
+// and its three quotients from one division in three lanes.
+__device__ __forceinline__ void solve_warp(const SolveIO& io, SolveTmp& tmp, const double* s) {
+    const unsigned full = 0xffffffffu;
+    const int lane = threadIdx.x & 31;
+    __syncwarp();
+    // row `lane` of A = w RGB + ICP and of b
+    const double w = (double)1e-4f;
+    const int row = lane < 6 ? lane : 5;
+    double a[6], yb;
+#pragma unroll
+    for (int j = 0; j < 6; ++j) {
+        const int lo = min(row, j), hi = max(row, j);
+        const int k = lo * 7 - lo * (lo - 1) / 2 + hi - lo;   // the sum of row[lo] row[hi]
+        a[j] = s[32 + k] * w + s[k];
+    }
+    {
+        const int k = row * 7 - row * (row - 1) / 2 + 6 - row;
+        yb = s[32 + k] * w + s[k];
+    }
+    // (other rows' L are fetched where they are used: few live registers, as
+    // spills on this chain cost more than the shuffles)
+    double L[6], D[6], x[6], Dinv = 0;
+#pragma unroll
+    for (int k = 0; k < 6; ++k) {
+        double t = a[k];
+#pragma unroll
+        for (int j = 0; j < k; ++j) t -= L[j] * __shfl_sync(full, L[j], k) * D[j];
+        D[k] = __shfl_sync(full, t, k);
+        const double inv = 1.0 / D[k];
+        if (lane == k) Dinv = inv;
+        L[k] = t * inv;
+        const double yk = __shfl_sync(full, yb, k);
+        if (lane > k) yb -= L[k] * yk;
+    }
+    yb *= Dinv;
+#pragma unroll
+    for (int i = 5; i >= 0; --i) {
+        double t = __shfl_sync(full, yb, i);
+#pragma unroll
+        for (int j = i + 1; j < 6; ++j) t -= __shfl_sync(full, L[i], j) * x[j];
+        x[i] = t;
+    }
+    // se3_exp of (upsilon, omega) = x: Rodrigues rotation and left Jacobian,
+    // Taylor series near zero; lane 3 i + j holds element (i, j)
+    const double th2 = x[3] * x[3] + x[4] * x[4] + x[5] * x[5];
+    double ca, cb, cc;
+    const double th = sqrt(th2);
+    if (th < 1e-5) {
+        ca = 1 - th2 / 6 + th2 * th2 / 120;
+        cb = 0.5 - th2 / 24 + th2 * th2 / 720;
+        cc = 1.0 / 6 - th2 / 120 + th2 * th2 / 5040;
+    } else {
+        double sn, co;
+        sincos(th, &sn, &co);
+        const double num = lane == 0 ? sn : lane == 1 ? 1 - co : th - sn;
+        const double den = lane == 0 ? th : lane == 1 ? th2 : th2 * th;
+        const double q = num / den;
+        ca = __shfl_sync(full, q, 0);
+        cb = __shfl_sync(full, q, 1);
+        cc = __shfl_sync(full, q, 2);
+    }
+    const int i3 = lane / 3, j3 = lane - 3 * i3;
+    if (lane < 9) {
+        const int d = (j3 - i3 + 3) % 3;
+        const int c = 3 - i3 - j3;   // the axis neither index names
+        const double v = c == 0 ? x[3] : c == 1 ? x[4] : x[5];
+        tmp.W[lane] = d == 0 ? 0.0 : d == 1 ? -v : v;
+    }
+    __syncwarp();
+    if (lane < 9) {
+        double w2 = 0;
+#pragma unroll
+        for (int k = 0; k < 3; ++k) w2 += tmp.W[i3 * 3 + k] * tmp.W[k * 3 + j3];
+        const double I = i3 == j3 ? 1.0 : 0.0, wij = tmp.W[lane];
+        tmp.T[i3 * 4 + j3] = I + ca * wij + cb * w2;
+        tmp.V[lane] = I + cb * wij + cc * w2;   // the left Jacobian, for the translation
+    }
+    __syncwarp();
+    if (lane < 3)
+        tmp.T[lane * 4 + 3] = tmp.V[lane * 3] * x[0] + tmp.V[lane * 3 + 1] * x[1] + tmp.V[lane * 3 + 2] * x[2];
+    else if (lane < 7)
+        tmp.T[9 + lane] = lane == 6 ? 1.0 : 0.0;   // the last row
+    __syncwarp();
+    // delta = dT delta, pose = last delta^-1
+    const int i4 = lane >> 2, j4 = lane & 3;
+    double v = 0;
+    if (lane < 16)
+#pragma unroll
+        for (int k = 0; k < 4; ++k) v += tmp.T[i4 * 4 + k] * io.delta[k * 4 + j4];
+    if (lane < 16) tmp.delta[lane] = v;
+    __syncwarp();
+    if (lane < 16) {
+        const double* d = tmp.delta;
+        double o;
+        if (i4 == 3)
+            o = j4 == 3 ? 1.0 : 0.0;
+        else if (j4 < 3)
+            o = d[j4 * 4 + i4];
+        else
+            o = -(d[i4] * d[3] + d[4 + i4] * d[7] + d[8 + i4] * d[11]);
+        tmp.dinv[lane] = o;
+    }
+    __syncwarp();
+    if (lane < 16) {
+        v = 0;
+#pragma unroll
+        for (int k = 0; k < 4; ++k) v += io.last_pose[i4 * 4 + k] * tmp.dinv[k * 4 + j4];
+        tmp.pose[lane] = v;
+        // the float view (make_dev_pose_d)
+        float* c = (float*)&tmp.cur;
+        if (i4 < 3) {
+            if (j4 < 3) {
+                c[i4 * 3 + j4] = (float)v;
+                c[9 + j4 * 3 + i4] = (float)v;
+            } else {
+                c[18 + i4] = (float)v;
+            }
+        }
+    }
+}
+
+// The Gauss-Newton update of one iteration and, after the last one, the
+// acceptance test, on staged state by a whole block: io.delta / last_pose /
+// init_pose / icp_error in; io.pose, delta, cur, errors, counts, failed and
+// updated out (a failed count or error test leaves delta and cur as they were
+// and sets pose = last_pose; a failed acceptance test does so after the
+// update).  Ends with a block barrier.
+// As a call, for k_track_loop: inlined, its FP64 state spills the passes' registers.
+__device__ __noinline__ void solve_warp_call(const SolveIO& io, SolveTmp& tmp, const double* s) { solve_warp(io, tmp, s); }
+
+template <bool kCall>
+__device__ __forceinline__ void solve_block(SolveIO& io, SolveTmp& tmp, const double* s, int min_count, int is_final) {
+    const int t = threadIdx.x;
+    if (t < 32) {
+        if constexpr (kCall)
+            solve_warp_call(io, tmp, s);
+        else
+            solve_warp(io, tmp, s);
+    } else if (t == 32)
+        solve_checks(io, s, min_count);
+    __syncthreads();
+    const bool fail = io.failed != 0;
+    if (t < 16) {
+        io.pose[t] = fail ? io.last_pose[t] : tmp.pose[t];
+        if (!fail) io.delta[t] = tmp.delta[t];
+    } else if (t >= 32 && t < 32 + (int)(sizeof(DevPose) / 4)) {
+        if (!fail) ((float*)&io.cur)[t - 32] = ((const float*)&tmp.cur)[t - 32];
+    }
+    __syncthreads();
+    if (is_final && !fail) {
+        if (t == 0 && !accept_pose(io)) {
+            for (int i = 0; i < 16; ++i) io.pose[i] = io.last_pose[i];
+            io.failed = 1;
+        }
+        __syncthreads();
+    }
+}
 
 // The end of an iteration, in the block that finished last: the group sums
 // of both passes in group order (FP64, or compensated FP32 in the precision
@@ -912,12 +896,10 @@ __device__ __forceinline__ void finish_iteration(TrackState* st, unsigned int* t
         }
     }
     __syncthreads();
-    if (threadIdx.x == 0) {
-        *ticket = 0;
-        solve_staged(io, sums, min_count, is_final);
-    }
-    __syncthreads();
+    __shared__ SolveTmp tmp;
+    solve_block<false>(io, tmp, sums, min_count, is_final);
     // write back in parallel
+    if (threadIdx.x == 128) *ticket = 0;
     if (threadIdx.x < 16) {
         st->pose[threadIdx.x] = io.pose[threadIdx.x];
         if (io.updated) st->delta[threadIdx.x] = io.delta[threadIdx.x];
@@ -938,104 +920,18 @@ __device__ __forceinline__ void finish_iteration(TrackState* st, unsigned int* t
     }
 }
 
-// pass B (clusters as in pass A): every block derives sigma from pass A's
-// group counts (integers: the same value in every block) and builds the RGB
-// rows of its warps' segments; each cluster reduces its rows into a group
-// sum; the last cluster to finish adds the groups of both passes in group
-// order (FP64) and performs the Gauss-Newton update with one warp.
-template <int kMinBlocks, bool kComp>
-__global__ void __cluster_dims__(kTrackCluster, 1, 1) __launch_bounds__(256, kMinBlocks)
-    k_track_b(TrackLevel L, TrackState* st, unsigned int* ticket, const int2* list, const int* counts, int seg_size,
-              int min_count, int is_final) {
-    cg::cluster_group cl = cg::this_cluster();
-    __shared__ float sm[32 * 29];
-    __shared__ float s_rgb[32];
-    __shared__ double s_part[4][64];
-    __shared__ float2 s_partc[4][64];
-    __shared__ double sums[64];
-    __shared__ bool s_last;
-    __shared__ SolveIO io;
-    const int G = gridDim.x, NG = G / kTrackCluster, lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    // stage the solve's inputs early (used by the last cluster's first block)
-    if (cl.block_rank() == 0) {
-        if (threadIdx.x >= 64 && threadIdx.x < 80) {
-            const int i = threadIdx.x - 64;
-            io.delta[i] = st->delta[i];
-            io.last_pose[i] = st->last_pose[i];
-            io.init_pose[i] = st->init_pose[i];
-        }
-        if (threadIdx.x == 80) {
-            io.icp_error = st->icp_error;
-            io.icp_count = st->icp_count;
-        }
-    }
-    if (st->failed) return;
-    // the first row's inputs (list entry, then its gathers) are loaded while
-    // the robust scale is reduced: neither needs the other
-    const int gw = blockIdx.x * kTrackWarps + wid;
-    const int2* seg = list + (size_t)gw * seg_size;
-    const int nseg = counts[gw];
-    RgbIn first{};
-    if (lane < nseg) first = rgb_fetch_entry(L, seg[lane]);
-    const DevPose cur = st->cur, last = st->last;
-    // sigma = sqrt((float) sum / count) (Reduction.cu:606-608); every warp
-    // adds the group counts itself (integers: exact in any order)
-    long long c = 0, q = 0;
-    for (int g = lane; g < NG; g += 32) {
-        c += __ldcg(&st->grp_cnt[g]);
-        q += __ldcg(&st->grp_sq[g]);
-    }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        c += __shfl_xor_sync(0xffffffffu, c, o);
-        q += __shfl_xor_sync(0xffffffffu, q, o);
-    }
-    const float sigma = sqrtf((float)q / (float)(c == 0 ? 1 : c));
-    float acc[29];
-#pragma unroll
-    for (int k = 0; k < 29; ++k) acc[k] = 0.f;
-    add_segment_rows(L, cur, last, sigma, seg, nseg, lane, acc, first);
-    const float bsum = block_sum29(acc, sm);
-    if (wid == 0) s_rgb[lane] = lane < 29 ? bsum : 0.f;
-    const int grp = blockIdx.x / kTrackCluster;
-    if constexpr (kComp) {
-        cl.sync();
-        if (cl.block_rank() == 0 && threadIdx.x < 29) {
-            float2 acc = make_float2(0.f, 0.f);
-#pragma unroll
-            for (int r = 0; r < kTrackCluster; ++r)
-                acc = pair_add(acc, make_float2(cl.map_shared_rank(s_rgb, r)[threadIdx.x], 0.f));
-            st->grp_rgb2[grp][threadIdx.x] = acc;
-        }
-        cl.sync();
-        if (cl.block_rank() != 0) return;
-    } else {
-        const double v = cluster_sum(cl, s_rgb, 29);
-        if (cl.block_rank() != 0) return;
-        if (threadIdx.x < 29) st->grp_rgb[grp][threadIdx.x] = v;
-    }
-    // last cluster (its rank-0 block) to finish
-    __syncthreads();
-    if (threadIdx.x == 0) s_last = ticket_acq_rel(ticket) == (unsigned)(NG - 1);
-    __syncthreads();
-    if (!s_last) return;
-    finish_iteration<kComp>(st, ticket, NG, c, q, sigma, min_count, is_final, io, s_part, s_partc, sums);
-}
-
 // Shape of the group forms below: groups per block and resident blocks per
 // SM (4: half the registers, some spilled; 2: none spilled).
 constexpr int kGroupsPerBlock = 1;
 constexpr int kGrpMinBlocks = 4;
 
-// Group forms of k_track_a / k_track_b for sessions sharing the GPU: one
-// block per group does the work of the group's kTrackCluster clustered
-// blocks -- logical blocks b = kTrackCluster * group + r, r in rank order,
-// each with the pixels, warp segments and block sums the clustered block b
-// has in a grid of G blocks -- and adds their sums in rank order as the
-// cluster reduction does.  The results are therefore the clustered kernels'
-// bit for bit, on a grid of G / kTrackCluster blocks: a session's pass holds
-// a quarter of the block slots for longer, and other sessions' passes run
-// beside it.
+// The passes for sessions sharing the GPU: one block per group does the work
+// of the group's kTrackCluster logical blocks -- b = kTrackCluster * group + r
+// in a grid of G blocks, r in rank order -- and adds their sums in rank order.
+// A session's pass holds a quarter of the block slots for longer, and other
+// sessions' passes run beside it.  A pass leaves its group sums in the
+// tracker state; the last block of pass B to finish adds the groups and
+// solves.
 template <int kMinBlocks, bool kComp>
 __device__ __forceinline__ void track_a_grp_body(const BlockCtx& ctx, TrackLevel L, TrackState* st, int2* list,
                                                  int* counts, int G, int gpc) {
@@ -1181,7 +1077,8 @@ __device__ __forceinline__ void track_b_grp_body(const BlockCtx& ctx, TrackLevel
     }
     if (st->failed) return;
     const DevPose cur = st->cur, last = st->last;
-    // sigma as in k_track_b
+    // sigma = sqrt((float) sum / count) (Reduction.cu:606-608); every warp
+    // adds the group counts itself (integers: exact in any order)
     long long c = 0, q = 0;
     for (int g = lane; g < NG; g += 32) {
         c += __ldcg(&st->grp_cnt[g]);
@@ -1202,7 +1099,7 @@ __device__ __forceinline__ void track_b_grp_body(const BlockCtx& ctx, TrackLevel
 #pragma unroll
         for (int k = 0; k < 29; ++k) acc[k] = 0.f;
         const int gw = b * kTrackWarps + wid;
-        add_segment_rows_seq(L, cur, last, sigma, list + (size_t)gw * seg_size, counts[gw], lane, acc);
+        add_segment_rows(L, cur, last, sigma, list + (size_t)gw * seg_size, counts[gw], lane, acc);
         const float bsum = block_sum29(acc, sm);
         if (wid == 0) s_rgb[r][lane] = lane < 29 ? bsum : 0.f;
         __syncthreads();   // sm is reused by the next logical block
@@ -1256,143 +1153,508 @@ __global__ void __launch_bounds__(256, kMinBlocks)
     run_part(fp, [](const BlockCtx& c, const auto&... a) { track_b_grp_body<kMinBlocks, kComp>(c, a...); });
 }
 
-// The Gauss-Newton update of one iteration (Tracking.cc:319-394) and, after
-// the last one, the acceptance test (Tracking.cc:398-408), on staged state:
-// io.delta / last_pose / init_pose / icp_error in; io.pose, delta, cur,
-// errors, counts, failed and updated out (a failed count or error test
-// leaves delta and cur as they were and sets pose = last_pose; a failed
-// acceptance test does so after the update).  One thread; every array in
-// registers.
-__device__ void solve_staged(SolveIO& io, const double* s, int min_count, int is_final) {
-    bool fail = false;
-    {
-        float r0 = (float)s[32 + 27], r1 = (float)s[32 + 28];
-        float err = sqrtf(r0) / r1;
-        io.rgb_error = err;
-        io.rgb_count = r1;
-        if (isnan(err) || (int)r1 < min_count) fail = true;
-    }
-    if (!fail) {
-        float q0 = (float)s[27], q1 = (float)s[28];
-        float icp_err = sqrtf(q0) / q1;
-        io.icp_error = icp_err;
-        io.icp_count = q1;
-        if (isnan(icp_err) || (int)q1 < min_count) fail = true;
-    }
-    io.failed = 0;
-    io.updated = 0;
-    if (fail) {
-        for (int i = 0; i < 16; ++i) io.pose[i] = io.last_pose[i];
-        io.failed = 1;
-        return;
-    }
-    double Ar[36], br[6], Ai[36], bi[6], A[36], b[6], x[6], dT[16], dinv[16], delta[16], lastp[16], pose[16];
-    unpack29(s + 32, Ar, br);
-    unpack29(s, Ai, bi);
-    const float w = 1e-4f;
-#pragma unroll
-    for (int i = 0; i < 36; ++i) A[i] = Ar[i] * (double)w + Ai[i];
-#pragma unroll
-    for (int i = 0; i < 6; ++i) b[i] = br[i] * (double)w + bi[i];
-    ldlt6(A, b, x);
-    se3_exp(x, dT);
-#pragma unroll
-    for (int i = 0; i < 16; ++i) {
-        delta[i] = io.delta[i];
-        lastp[i] = io.last_pose[i];
-    }
-    mat4_mul(dT, delta, delta);
-    mat4_rigid_inv(delta, dinv);
-    mat4_mul(lastp, dinv, pose);
-#pragma unroll
-    for (int i = 0; i < 16; ++i) {
-        io.delta[i] = delta[i];
-        io.pose[i] = pose[i];
-    }
-    io.cur = make_dev_pose_d(pose);
-    io.updated = 1;
-    if (is_final) {
-        double pinv[16], p[16], init[16];
-#pragma unroll
-        for (int i = 0; i < 16; ++i) init[i] = io.init_pose[i];
-        mat4_rigid_inv(init, pinv);
-        mat4_mul(pinv, pose, p);
-        double tn = sqrt(p[3] * p[3] + p[7] * p[7] + p[11] * p[11]);
-        if (!(io.icp_error < 0.0001f && euler_sin_norm(p) <= 0.1 && tn <= 0.1)) {
-            for (int i = 0; i < 16; ++i) io.pose[i] = io.last_pose[i];
-            io.failed = 1;
-        }
-    }
+// ------------------------------------------- the whole loop in one launch
+//
+// A session alone runs all its Gauss-Newton iterations in this one kernel: a
+// cooperative grid of clusters, resident together, whose blocks hand each
+// other their results through global memory instead of ending.  What bounds
+// it is the chain of an iteration.  As two launches per iteration (clusters
+// of the same shape: two launches, two state loads, two staging waits, four
+// cluster barriers, a ticket) an iteration took 13 us on 160x120 pixels, 18
+// on 320x240 and 26 on 640x480; here 8.7, 11.8 and 19 (a frame's 18
+// iterations: 234 -> 154 us at 160x120, 393 -> 299 us at 640x480).  Per
+// iteration:
+//   - every block waits for the pose (8 slots), runs pass A over its pixels,
+//     publishes its correspondence count and squared differences, reduces and
+//     publishes its ICP sums while the other blocks' counts arrive;
+//   - every block adds all counts (integers: exact), hence sigma, and runs
+//     pass B from its correspondence list in shared memory (the gathered last
+//     vertex is kept there by pass A) and publishes its RGB sums;
+//   - the four blocks of cluster 0 each add one of the four group ranges of
+//     both passes, block 0 adds the ranges, solves and publishes the pose.
+// Pixels, lists, block sums, and the order in which they are added are those
+// of the group kernels' logical grid of G blocks: the same bits.
+//
+// The exchanged values travel in 16-byte slots {3 words, epoch} stored and
+// loaded as one 128-bit access each, so a slot that holds the expected epoch
+// holds its data: no fences, tickets or second round trips.  A slot is
+// rewritten only after everyone who needs its last value has published
+// something that the rewriting waits for.  Every wait is bounded; a wait that
+// gives up fails the frame (failed bit 1) and its block leaves.
+// The blocks must be resident together, hence the cooperative launch and the
+// size rule of launch_track_loop.
+constexpr int kLoopPolls = 1 << 18;
+constexpr int kLoopRows = 80;                       // blocks of one group range, at most
+constexpr int kLoopMaxBuf = 12;
+constexpr int kLoopScratch = kLoopRows / kTrackCluster * 32 * 8 + kLoopRows * 30 * 4;   // cluster 0's sums (14720)
+constexpr int kLoopListBytes = 256 * (16 + 2);      // correspondence list of one chunk
+
+// One 256-pixel chunk of the current frame (as PixelStage).
+struct LoopStage {
+    float4 v[256];
+    float4 n[256];
+    int16_t dx[256];
+    int16_t dy[256];
+    uint8_t ok[256];
+    uint8_t g[256];
+};
+
+struct LoopArgs {
+    TrackLevel L[3];
+    int iters[3], min_count[3], G[3];
+    int nbuf;      // chunk buffers
+    int chunks;    // chunks of a block, at most (the list's capacity)
+    unsigned char* list;   // the lists in global memory (kGlobalList)
+};
+
+__device__ __forceinline__ void slot_put(TrackSlot* p, uint32_t x, uint32_t y, uint32_t z, uint32_t e) {
+    asm volatile(
+        "{\n"
+        ".reg .b64 a, b;\n"
+        ".reg .b128 t;\n"
+        "mov.b64 a, {%1, %2};\n"
+        "mov.b64 b, {%3, %4};\n"
+        "mov.b128 t, {a, b};\n"
+        "st.relaxed.gpu.global.b128 [%0], t;\n"
+        "}\n" ::"l"(p), "r"(x), "r"(y), "r"(z), "r"(e)
+        : "memory");
 }
 
-// The Gauss-Newton update of one iteration (Tracking.cc:319-394) and, after
-// the last one, the acceptance test (Tracking.cc:398-408).  One thread; the
-// normal equations are in FP64, every array in registers.
-// The Gauss-Newton update of one iteration (Tracking.cc:319-394) and, after
-// the last one, the acceptance test (Tracking.cc:398-408), from the FP64 sums
-// s (ICP in s[0..28], RGB in s[32..60]).  One thread; every array in
-// registers.
-__device__ __forceinline__ void solve_step(TrackState* st, const double* s, int min_count, int is_final) {
-    bool fail = false;
-    {
-        float r0 = (float)s[32 + 27], r1 = (float)s[32 + 28];
-        float err = sqrtf(r0) / r1;
-        st->rgb_error = err;
-        st->rgb_count = r1;
-        if (isnan(err) || (int)r1 < min_count) fail = true;
+__device__ __forceinline__ uint4 slot_get(const TrackSlot* p) {
+    uint4 v;
+    asm volatile(
+        "{\n"
+        ".reg .b64 a, b;\n"
+        ".reg .b128 t;\n"
+        "ld.relaxed.gpu.global.b128 t, [%4];\n"
+        "mov.b128 {a, b}, t;\n"
+        "mov.b64 {%0, %1}, a;\n"
+        "mov.b64 {%2, %3}, b;\n"
+        "}\n"
+        : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
+        : "l"(p)
+        : "memory");
+    return v;
+}
+
+// Waits until the slot holds exchange e; false after kLoopPolls loads.
+__device__ __forceinline__ bool slot_wait(const TrackSlot* p, uint32_t e, uint4& v) {
+    for (int i = 0; i < kLoopPolls; ++i) {
+        v = slot_get(p);
+        if (v.w == e) return true;
     }
-    float icp_err = st->icp_error;
-    if (!fail) {
-        float q0 = (float)s[27], q1 = (float)s[28];
-        icp_err = sqrtf(q0) / q1;
-        st->icp_error = icp_err;
-        st->icp_count = q1;
-        if (isnan(icp_err) || (int)q1 < min_count) fail = true;
-    }
-    if (fail) {
-        for (int i = 0; i < 16; ++i) st->pose[i] = st->last_pose[i];
-        __threadfence();
-        st->failed = 1;
-        return;
-    }
-    double Ar[36], br[6], Ai[36], bi[6], A[36], b[6], x[6], dT[16], dinv[16], delta[16], lastp[16], pose[16];
-    unpack29(s + 32, Ar, br);
-    unpack29(s, Ai, bi);
-    const float w = 1e-4f;
+    return false;
+}
+
+// The 29 block sums (lane l of warp 0 holds value l) into ten slots.
+__device__ __forceinline__ void publish_sums(TrackSlot* slots, float r, int lane, uint32_t e) {
+    const int k = lane < 10 ? 3 * lane : 0;
+    const float x = __shfl_sync(0xffffffffu, r, k), y = __shfl_sync(0xffffffffu, r, k + 1),
+                z = __shfl_sync(0xffffffffu, r, k + 2);
+    if (lane < 10) slot_put(slots + lane, __float_as_uint(x), __float_as_uint(y), __float_as_uint(z), e);
+}
+
+// One lane: copy the chunk of pixels [start, min(start + 256, N)) into buf.
+__device__ __forceinline__ void loop_fill(LoopStage& S, uint64_t* bar, const TrackLevel& L, int start, int N) {
+    const int cnt = min(256, N - start);
+    const uint32_t b16 = (uint32_t)cnt * 16u, b1 = ((uint32_t)cnt + 15u) & ~15u;
+    const uint32_t b2 = ((uint32_t)cnt * 2u + 15u) & ~15u;
+    mbar_arrive_expect_tx(bar, 2u * b16 + 2u * b2 + 2u * b1);
+    bulk_copy_g2s(S.v, L.vcurr + start, b16, bar);
+    bulk_copy_g2s(S.n, L.ncurr + start, b16, bar);
+    bulk_copy_g2s(S.dx, L.dx + start, b2, bar);
+    bulk_copy_g2s(S.dy, L.dy + start, b2, bar);
+    bulk_copy_g2s(S.ok, L.rgbok + start, b1, bar);
+    bulk_copy_g2s(S.g, L.gcurr + start, b1, bar);
+}
+
+// The sums of ng groups (kTrackCluster blocks each, from `src`: ten slots of
+// one pass per block) in rank order, as FP64 (or compensated pairs) in
+// ((double*)scratch)[group * 32 + value].  Whole block; false in a thread
+// whose wait gave up.
+template <bool kComp>
+__device__ __forceinline__ bool range_sums(unsigned char* scratch, const TrackSlot* src, int ng, uint32_t e) {
+    constexpr int kRowsAtOnce = 25;   // 25 x 10 slots by 250 threads
+    const int t = threadIdx.x, nb = ng * kTrackCluster;
+    float* const S = (float*)(scratch + kLoopRows / kTrackCluster * 32 * 8);
+    bool ok = true;
+    if (t < kRowsAtOnce * 10) {
+        const int col = t % 10, row = t / 10;
+        src += col;
+        uint4 v[(kLoopRows + kRowsAtOnce - 1) / kRowsAtOnce];
 #pragma unroll
-    for (int i = 0; i < 36; ++i) A[i] = Ar[i] * (double)w + Ai[i];
+        for (int j = 0; j < (kLoopRows + kRowsAtOnce - 1) / kRowsAtOnce; ++j)
+            if (row + kRowsAtOnce * j < nb) v[j] = slot_get(src + (size_t)(row + kRowsAtOnce * j) * kSumSlots);
 #pragma unroll
-    for (int i = 0; i < 6; ++i) b[i] = br[i] * (double)w + bi[i];
-    ldlt6(A, b, x);
-    se3_exp(x, dT);
-#pragma unroll
-    for (int i = 0; i < 16; ++i) {
-        delta[i] = st->delta[i];
-        lastp[i] = st->last_pose[i];
-    }
-    mat4_mul(dT, delta, delta);
-    mat4_rigid_inv(delta, dinv);
-    mat4_mul(lastp, dinv, pose);
-#pragma unroll
-    for (int i = 0; i < 16; ++i) {
-        st->delta[i] = delta[i];
-        st->pose[i] = pose[i];
-    }
-    st->cur = make_dev_pose_d(pose);
-    if (is_final) {
-        double pinv[16], p[16], init[16];
-#pragma unroll
-        for (int i = 0; i < 16; ++i) init[i] = st->init_pose[i];
-        mat4_rigid_inv(init, pinv);
-        mat4_mul(pinv, pose, p);
-        double tn = sqrt(p[3] * p[3] + p[7] * p[7] + p[11] * p[11]);
-        if (!(icp_err < 0.0001f && euler_sin_norm(p) <= 0.1 && tn <= 0.1)) {
-            for (int i = 0; i < 16; ++i) st->pose[i] = st->last_pose[i];
-            __threadfence();
-            st->failed = 1;
+        for (int j = 0; j < (kLoopRows + kRowsAtOnce - 1) / kRowsAtOnce; ++j) {
+            const int r = row + kRowsAtOnce * j;
+            if (r < nb) {
+                if (v[j].w != e) ok &= slot_wait(src + (size_t)r * kSumSlots, e, v[j]);
+                float* o = S + r * 30 + 3 * col;
+                o[0] = __uint_as_float(v[j].x);
+                o[1] = __uint_as_float(v[j].y);
+                o[2] = __uint_as_float(v[j].z);
+            }
         }
     }
-    __threadfence();
+    __syncthreads();
+    const int val = t & 31;
+    if (val < 29)
+        for (int g = t >> 5; g < ng; g += kTrackWarps) {
+            const float* x = S + kTrackCluster * g * 30 + val;
+            if constexpr (kComp) {
+                float2 v = make_float2(0.f, 0.f);
+#pragma unroll
+                for (int r = 0; r < kTrackCluster; ++r) v = pair_add(v, make_float2(x[30 * r], 0.f));
+                ((float2*)scratch)[g * 32 + val] = v;
+            } else {
+                double v = 0;
+#pragma unroll
+                for (int r = 0; r < kTrackCluster; ++r) v += (double)x[30 * r];
+                ((double*)scratch)[g * 32 + val] = v;
+            }
+        }
+    __syncthreads();
+    return ok;
+}
+
+template <bool kComp, bool kGlobalList>
+__global__ void __cluster_dims__(kTrackCluster, 1, 1) __launch_bounds__(256, 2)
+    k_track_loop(const __grid_constant__ LoopArgs A, TrackState* st, TrackSync* sync) {
+    extern __shared__ __align__(128) unsigned char dyn[];
+    __shared__ uint64_t bar[kLoopMaxBuf];
+    __shared__ DevPose s_cur, s_last;
+    __shared__ float sm[2][8 * 32];
+    __shared__ uint32_t s_cnt[8], s_sq[8], s_tc[8];
+    __shared__ unsigned long long s_tq[8];
+    __shared__ double s_part[4][64];
+    __shared__ double sums[64];
+    __shared__ SolveIO io;
+    __shared__ SolveTmp tmp;
+    __shared__ int s_failed, s_bad;
+    const int t = threadIdx.x, lane = t & 31, wid = t >> 5, b = blockIdx.x;
+    LoopStage* const stage = (LoopStage*)dyn;
+    // this block's correspondence list: A.chunks * 256 entries of 16 bytes,
+    // then of 2, a segment per warp
+    unsigned char* const scratch = dyn + (size_t)A.nbuf * sizeof(LoopStage);
+    unsigned char* const list = kGlobalList ? A.list + (size_t)b * A.chunks * kLoopListBytes : scratch;
+    float4* const seg = (float4*)list + wid * A.chunks * 32;
+    int16_t* const segd = (int16_t*)(list + (size_t)A.chunks * 256 * 16) + wid * A.chunks * 32;
+    cg::cluster_group cl = cg::this_cluster();
+    const unsigned base = sync->epoch, total = (unsigned)(A.iters[0] + A.iters[1] + A.iters[2]);
+    if (t == 224)
+        for (int i = 0; i < A.nbuf; ++i) mbar_init(&bar[i], 1);
+    if (t == 0) s_failed = s_bad = 0;
+    if (t < (int)(sizeof(DevPose) / 4)) {
+        ((float*)&s_cur)[t] = ((const float*)&st->cur)[t];
+        ((float*)&s_last)[t] = ((const float*)&st->last)[t];
+        if (b == 0) ((float*)&io.cur)[t] = ((const float*)&st->cur)[t];
+    }
+    if (b == 0) {
+        if (t >= 64 && t < 80) {
+            io.delta[t - 64] = st->delta[t - 64];
+            io.last_pose[t - 64] = st->last_pose[t - 64];
+            io.init_pose[t - 64] = st->init_pose[t - 64];
+        }
+        if (t == 80) {
+            io.icp_error = st->icp_error;
+            io.icp_count = st->icp_count;
+        }
+    }
+    __syncthreads();
+    // chunks of this block at level l; copies of the first nbuf of them
+    // (issued by one lane; every thread keeps the buffers' wait parities and
+    // which of them have a copy in flight)
+    auto chunks_of = [&](int l) {
+        const int N = A.L[l].W * A.L[l].H, S = A.G[l] * 256;
+        return b * 256 < N ? (N - b * 256 + S - 1) / S : 0;
+    };
+    uint32_t parity = 0, flight = 0;
+    auto prefetch = [&](int l) {
+        const int n = min(A.nbuf, chunks_of(l));
+        if (t == 224) {
+            fence_proxy_async_smem();
+            for (int k = 0; k < n; ++k)
+                loop_fill(stage[k], &bar[k], A.L[l], b * 256 + k * A.G[l] * 256, A.L[l].W * A.L[l].H);
+        }
+        flight |= (1u << n) - 1u;
+    };
+    unsigned e = base;
+    bool fetched = false, alive = true;
+    int bad = 0;
+    const unsigned lt = (1u << lane) - 1u;
+    for (int l = 2; l >= 0 && alive; --l) {
+        const int iters = A.iters[l], G = A.G[l];
+        if (iters == 0) continue;
+        if (b >= G) {   // no pixels here at this level
+            e += iters;
+            continue;
+        }
+        if (!fetched) prefetch(l);
+        fetched = true;
+        int finer = l - 1;
+        while (finer >= 0 && A.iters[finer] == 0) --finer;
+        const TrackLevel& L = A.L[l];
+        const int N = L.W * L.H, cb = chunks_of(l);
+        const bool resident = cb <= A.nbuf;
+        int f = 0;   // chunk fills taken at this level
+        for (int it = 0; it < iters; ++it) {
+            if (e != base && b != 0) {
+                if (wid == 0) {
+                    // a frame that failed at a coarser level, where this block
+                    // had no pixels, says so under an earlier number
+                    uint4 v;
+                    bool got = false;
+                    for (int i = 0; i < kLoopPolls && !got; ++i) {
+                        v = slot_get(&sync->pose[b % kPoseCopies][lane & 7]);
+                        const bool lost = (lane & 7) == 7 && v.x != 0 && v.w - base - 1u < total;
+                        if (__any_sync(0xffffffffu, lost)) {
+                            if (lane == 0) s_failed = 1;
+                            got = true;
+                            v.w = base;   // no pose
+                        } else {
+                            got = __all_sync(0xffffffffu, v.w == e);
+                        }
+                    }
+                    if (!got) {
+                        if (lane == 0) {
+                            atomicOr((unsigned*)&st->failed, 2u);
+                            s_failed = 2;
+                        }
+                    } else if (lane < 7 && v.w == e) {
+                        uint32_t* c = (uint32_t*)&s_cur + 3 * lane;
+                        c[0] = v.x;
+                        c[1] = v.y;
+                        c[2] = v.z;
+                    }
+                }
+            }
+            __syncthreads();   // (block 0 wrote its pose itself)
+            if (s_failed) {
+                alive = false;
+                break;
+            }
+            const DevPose &cur = s_cur, &last = s_last;
+            float acc[29];
+#pragma unroll
+            for (int k = 0; k < 29; ++k) acc[k] = 0.f;
+            // pass A
+            uint32_t rc = 0, rsq = 0;
+            int run = 0;
+            for (int k = 0; k < cb; ++k) {
+                int buf = k;
+                if (!resident) buf = f % A.nbuf;
+                if (!resident || it == 0) {
+                    if (!mbar_wait(&bar[buf], (parity >> buf) & 1u)) bad = 1;
+                    parity ^= 1u << buf;
+                    flight &= ~(1u << buf);
+                }
+                const int p = b * 256 + k * G * 256 + t;
+                PixelIn in;
+                if (p < N) {
+                    const LoopStage& S = stage[buf];
+                    in.vc = S.v[t];
+                    const float4 n = S.n[t];
+                    in.nc = make_float3(n.x, n.y, n.z);
+                    in.ok = S.ok[t];
+                    in.gc = S.g[t];
+                    in.dxy = (int)(uint16_t)S.dx[t] | ((int)S.dy[t] << 16);
+                }
+                if (!resident) {
+                    __syncthreads();   // the buffer is read: it may be filled again
+                    if (f + A.nbuf < iters * cb) {
+                        if (t == 224) {
+                            fence_proxy_async_smem();
+                            loop_fill(stage[buf], &bar[buf], L, b * 256 + (f + A.nbuf) % cb * G * 256, N);
+                        }
+                        flight |= 1u << buf;
+                    }
+                    ++f;
+                }
+                int r = -1;
+                f3 vl;
+                if (p < N) {
+                    float row[7];
+                    if (pixel_pass_a(L, cur, last, in, row, &r, &vl)) add_products(row, acc);
+                }
+                const int d = (r & 511) - 255;
+                if (r != -1) {
+                    rc += 1;
+                    rsq += (uint32_t)(d * d);
+                }
+                const unsigned m = __ballot_sync(0xffffffffu, r != -1);
+                if (r != -1) {
+                    const int o = run + __popc(m & lt);
+                    seg[o] = make_float4(vl.x, vl.y, vl.z, __int_as_float(in.dxy));
+                    segd[o] = (int16_t)d;
+                }
+                run += __popc(m);
+            }
+            rc = __reduce_add_sync(0xffffffffu, rc);
+            rsq = __reduce_add_sync(0xffffffffu, rsq);
+            if (lane == 0) {
+                s_cnt[wid] = rc;
+                s_sq[wid] = rsq;
+            }
+            __syncthreads();
+            if (t == 0) {
+                uint32_t c = 0, q = 0;
+#pragma unroll
+                for (int w = 0; w < kTrackWarps; ++w) {
+                    c += s_cnt[w];
+                    q += s_sq[w];
+                }
+                slot_put(&sync->count[b], c, q, 0, e + 1);
+            }
+            if (it == iters - 1 && finer >= 0) prefetch(finer);   // its copies land during the rest of this iteration
+            float bsum = block_sum29(acc, sm[0]);
+            if (wid == 0) publish_sums(sync->sums[b], bsum, lane, e + 1);
+            __syncwarp();   // the list is read by other lanes than wrote it
+            // the first photometric row up to its weight, while the counts arrive
+            RgbDir d0{};
+            int diff0 = 0;
+            if (lane < run) {
+                const float4 v = seg[lane];
+                const int dxy = __float_as_int(v.w);
+                d0 = rgb_dir(xyz(v), (int)(int16_t)(dxy & 0xffff), dxy >> 16, L, cur, last);
+                diff0 = segd[lane];
+            }
+            // sigma = sqrt((float) sum / count) (Reduction.cu:606-608)
+            uint32_t tc = 0, tq = 0;   // at most three blocks' sums per thread: below 2^32
+            for (int j = t; j < G; j += 256) {
+                uint4 v;
+                if (!slot_wait(&sync->count[j], e + 1, v)) bad = 1;
+                tc += v.x;
+                tq += v.y;
+            }
+            tc = __reduce_add_sync(0xffffffffu, tc);
+            const uint32_t qlo = __reduce_add_sync(0xffffffffu, tq & 0xffffu);
+            const uint32_t qhi = __reduce_add_sync(0xffffffffu, tq >> 16);
+            if (lane == 0) {
+                s_tc[wid] = tc;
+                s_tq[wid] = ((unsigned long long)qhi << 16) + qlo;
+            }
+            bad = __syncthreads_or(bad);
+            long long C = 0, Q = 0;
+#pragma unroll
+            for (int w = 0; w < kTrackWarps; ++w) {
+                C += s_tc[w];
+                Q += (long long)s_tq[w];
+            }
+            if (bad && b >= kTrackCluster) {
+                if (t == 0) atomicOr((unsigned*)&st->failed, 2u);
+                alive = false;
+                break;
+            }
+            const float sigma = sqrtf((float)Q / (float)(C == 0 ? 1 : C));
+            // pass B
+#pragma unroll
+            for (int k = 0; k < 29; ++k) acc[k] = 0.f;
+            if (lane < run) {
+                float row[7];
+                rgb_weighted(d0, diff0, sigma, row);
+                add_products(row, acc);
+            }
+            for (int i = lane + 32; i < run; i += 32) {
+                const float4 v = seg[i];
+                const int dxy = __float_as_int(v.w);
+                float row[7];
+                rgb_weighted(rgb_dir(xyz(v), (int)(int16_t)(dxy & 0xffff), dxy >> 16, L, cur, last), segd[i], sigma, row);
+                add_products(row, acc);
+            }
+            bsum = block_sum29(acc, sm[1]);
+            ++e;
+            if (wid == 0) publish_sums(sync->sums[b] + 10, bsum, lane, e);
+            const bool is_final = finer < 0 && it == iters - 1;
+            if (b >= kTrackCluster) {
+                if (is_final) alive = false;
+                continue;
+            }
+            // cluster 0: block r adds group range r of both passes (the
+            // ranges, and the orders inside, of finish_iteration); its list
+            // space is free (block_sum29's barrier) and takes the sums.  The
+            // ICP sums have arrived and are added while the last RGB sums come.
+            const int NG = G / kTrackCluster, per = (NG + 3) / 4, g0 = b * per;
+            const int ng = max(0, min(NG, g0 + per) - g0);
+            for (int pass = 0; pass < 2; ++pass) {
+                bad |= !range_sums<kComp>(scratch, &sync->sums[g0 * kTrackCluster][10 * pass], ng, e);
+                if (t < 32) {
+                    double* dst = (double*)cl.map_shared_rank(&s_part[0][0], 0) + b * 64 + 32 * pass + t;
+                    if constexpr (kComp) {
+                        float2 v = make_float2(0.f, 0.f);
+                        if (t < 29)
+                            for (int g = 0; g < ng; ++g) v = pair_add(v, ((const float2*)scratch)[g * 32 + t]);
+                        *(float2*)dst = v;
+                    } else {
+                        double v = 0;
+                        if (t < 29)
+#pragma unroll 4
+                            for (int g = 0; g < ng; ++g) v += ((const double*)scratch)[g * 32 + t];
+                        *dst = v;
+                    }
+                }
+                __syncthreads();   // the scratch is read
+            }
+            bad = __syncthreads_or(bad);
+            if (t == 0 && bad) *cl.map_shared_rank(&s_bad, 0) = 1;
+            cl.sync();
+            if (b != 0) {
+                if (is_final) alive = false;
+                continue;
+            }
+            if (t < 64) {
+                if constexpr (kComp) {
+                    const float2 v = pair_add(pair_add(pair_add(*(float2*)&s_part[0][t], *(float2*)&s_part[1][t]),
+                                                       *(float2*)&s_part[2][t]),
+                                              *(float2*)&s_part[3][t]);
+                    sums[t] = (double)v.x + (double)v.y;
+                } else {
+                    sums[t] = ((s_part[0][t] + s_part[1][t]) + s_part[2][t]) + s_part[3][t];
+                }
+            }
+            __syncthreads();
+            solve_block<true>(io, tmp, sums, A.min_count[l], is_final ? 1 : 0);
+            const int failed = s_bad ? 3 : io.failed;
+            if (!is_final && t < 8 * kPoseCopies) {
+                const int k = t & 7;
+                const uint32_t* c = (const uint32_t*)&io.cur + 3 * k;
+                if (k < 7)
+                    slot_put(&sync->pose[t >> 3][k], c[0], c[1], c[2], e);
+                else
+                    slot_put(&sync->pose[t >> 3][7], (uint32_t)failed, 0, 0, e);
+            }
+            if (t >= 64 && t < 64 + (int)(sizeof(DevPose) / 4)) ((float*)&s_cur)[t - 64] = ((const float*)&io.cur)[t - 64];
+            if (is_final || failed) {
+                if (t < 16) {
+                    st->pose[t] = io.pose[t];
+                    st->delta[t] = io.delta[t];
+                } else if (t >= 32 && t < 32 + (int)(sizeof(DevPose) / 4)) {
+                    ((float*)&st->cur)[t - 32] = ((const float*)&io.cur)[t - 32];
+                } else if (t >= 64 && t < 93) {
+                    st->icp_sums[t - 64] = sums[t - 64];
+                    st->rgb_sums[t - 64] = sums[32 + t - 64];
+                } else if (t == 96) {
+                    st->icp_error = io.icp_error;
+                    st->icp_count = io.icp_count;
+                    st->rgb_error = io.rgb_error;
+                    st->rgb_count = io.rgb_count;
+                    st->rgb_cnt = C;
+                    st->rgb_sq = Q;
+                    st->sigma = sigma;
+                    st->failed = failed;
+                }
+                alive = false;
+                break;
+            }
+        }
+    }
+    // copies still in flight (a frame that failed before a level it had
+    // begun to stage) land before the block leaves
+    while (flight) {
+        const int i = __ffs((int)flight) - 1;
+        mbar_wait(&bar[i], (parity >> i) & 1u);
+        flight &= flight - 1u;
+    }
 }
 
 // Single-step entry points (the reference's ICPStep / RGBStep): reduce the
@@ -1498,15 +1760,64 @@ int track_grid(int n) {
     return g < cap ? g : cap;
 }
 
-int launch_track_begin(TrackState* st, cudaStream_t s) {
-    fb_launch(k_track_begin, (const void*)k_track_begin_fused, 1, 1, 0, s, st);
+int launch_track_begin(TrackState* st, TrackSync* sync, const int iters[3], cudaStream_t s) {
+    const unsigned step = (unsigned)(iters[0] + iters[1] + iters[2]) + 1u;
+    fb_launch(k_track_begin, (const void*)k_track_begin_fused, 1, 1, 0, s, st, sync, step);
     return 1;
 }
 
-// Grid of the clustered per-iteration kernels: track_grid rounded up to whole
-// clusters, at most as many clusters as can be resident at once (a cluster
-// needs all its blocks on one GPC, so fewer than 2 x SMs / kTrackCluster may
-// fit), so that every launch runs in a single wave.
+// Chunks that a block of k_track_loop has at a level stay in shared memory
+// for all of its iterations where they fit; a block with more than
+// kLoopSmemChunks of them streams them through kLoopRing buffers every
+// iteration, and keeps its list in global memory: both leave the L1 cache to
+// the gathers (1280x960, 17 chunks: with the lists in shared memory 30 KB of
+// L1 were left to 16 warps, and a level-0 iteration took 82 us instead of 65).
+constexpr int kLoopSmemChunks = 6;
+constexpr int kLoopRing = 3;
+constexpr int kLoopMost = kLoopSmemChunks * ((int)sizeof(LoopStage) + kLoopListBytes);
+static_assert(kLoopSmemChunks <= kLoopMaxBuf && kLoopMost >= kLoopSmemChunks * (int)sizeof(LoopStage) + kLoopScratch,
+              "the list holds the scratch");
+
+static const void* loop_kernel(bool compensated, bool global_list) {
+    return compensated ? (global_list ? (const void*)k_track_loop<true, true> : (const void*)k_track_loop<true, false>)
+                       : (global_list ? (const void*)k_track_loop<false, true>
+                                      : (const void*)k_track_loop<false, false>);
+}
+
+// Clusters of k_track_loop resident at once on the current device with the
+// most shared memory a launch takes (so the answer holds for every launch);
+// -1 where it cannot run.
+static int loop_clusters(bool compensated, bool global_list) {
+    static std::mutex lock;
+    static int resident[64][4] = {};
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) {
+        cudaGetLastError();
+        return -1;
+    }
+    std::lock_guard<std::mutex> guard(lock);
+    int& r = resident[dev][(compensated ? 2 : 0) + (global_list ? 1 : 0)];
+    if (!r) {
+        const void* k = loop_kernel(compensated, global_list);
+        r = -1;
+        int coop = 0, n = 0;
+        cudaLaunchConfig_t q = {};
+        q.gridDim = dim3(kTrackMaxBlocks);
+        q.blockDim = dim3(256);
+        q.dynamicSmemBytes = kLoopMost;
+        if (cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev) == cudaSuccess && coop &&
+            cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, kLoopMost) == cudaSuccess &&
+            cudaOccupancyMaxActiveClusters(&n, k, &q) == cudaSuccess && n > 0)
+            r = n;
+        cudaGetLastError();
+    }
+    return r;
+}
+
+// The logical grid of the tracking passes: track_grid rounded up to whole
+// groups, at most as many as k_track_loop has clusters resident at once (a
+// cluster needs all its blocks on one GPC, so fewer than 2 x SMs /
+// kTrackCluster may fit).
 int track_cluster_grid(int n) {
     static int cap = 0;
     if (!cap) {
@@ -1514,15 +1825,8 @@ int track_cluster_grid(int n) {
         cudaGetDevice(&dev);
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
         int c = sms > 0 ? 2 * sms / kTrackCluster : kTrackMaxGroups;
-        cudaLaunchConfig_t cfg = {};
-        cfg.gridDim = dim3(c * kTrackCluster);
-        cfg.blockDim = dim3(256);
-        int ca = 0, cb = 0;
-        // the register-rich instances (two blocks per SM) bound the grid of both
-        if (cudaOccupancyMaxActiveClusters(&ca, (void*)k_track_a<2, false>, &cfg) == cudaSuccess && ca > 0 && ca < c)
-            c = ca;
-        if (cudaOccupancyMaxActiveClusters(&cb, (void*)k_track_b<2, false>, &cfg) == cudaSuccess && cb > 0 && cb < c)
-            c = cb;
+        const int r = loop_clusters(false, false);
+        if (r > 0 && r < c) c = r;
         cudaGetLastError();
         if (c > kTrackMaxGroups) c = kTrackMaxGroups;
         cap = c * kTrackCluster;
@@ -1533,36 +1837,72 @@ int track_cluster_grid(int n) {
 }
 
 int launch_track_iter(const TrackLevel& L, TrackState* st, unsigned int* tickets, int2* residual, int* counts,
-                      int min_count, bool is_final, cudaStream_t s, bool shared_gpu, bool compensated) {
+                      int min_count, bool is_final, cudaStream_t s, bool compensated) {
     const int n = L.W * L.H;
     const int g = track_cluster_grid(n);
     const int seg = (n + g * 256 - 1) / (g * 256) * 32;
     const int fin = is_final ? 1 : 0;
-    // sessions sharing the GPU: the group forms, kGroupsPerBlock groups per
-    // block, the same results; fused launches (a recorder) take the group
-    // forms too, since clusters do not span the parts of a fused grid
-    if (launch_recorder()) shared_gpu = true;
     const int ng = g / kTrackCluster, gpc = kGroupsPerBlock, gb = (ng + gpc - 1) / gpc;
     if (compensated) {
-        if (shared_gpu) {
-            fb_launch(k_track_a_grp<kGrpMinBlocks, true>, (const void*)k_track_a_grp_fused<kGrpMinBlocks, true>, gb,
-                      256, 0, s, L, st, residual, counts, g, gpc);
-            fb_launch(k_track_b_grp<kGrpMinBlocks, true>, (const void*)k_track_b_grp_fused<kGrpMinBlocks, true>, gb,
-                      256, 0, s, L, st, tickets + 1, residual, counts, seg, min_count, fin, ng, gpc);
-        } else {
-            k_track_a<2, true><<<g, 256, 0, s>>>(L, st, residual, counts);
-            k_track_b<2, true><<<g, 256, 0, s>>>(L, st, tickets + 1, residual, counts, seg, min_count, fin);
-        }
-    } else if (shared_gpu) {
+        fb_launch(k_track_a_grp<kGrpMinBlocks, true>, (const void*)k_track_a_grp_fused<kGrpMinBlocks, true>, gb, 256,
+                  0, s, L, st, residual, counts, g, gpc);
+        fb_launch(k_track_b_grp<kGrpMinBlocks, true>, (const void*)k_track_b_grp_fused<kGrpMinBlocks, true>, gb, 256,
+                  0, s, L, st, tickets + 1, residual, counts, seg, min_count, fin, ng, gpc);
+    } else {
         fb_launch(k_track_a_grp<kGrpMinBlocks, false>, (const void*)k_track_a_grp_fused<kGrpMinBlocks, false>, gb, 256,
                   0, s, L, st, residual, counts, g, gpc);
         fb_launch(k_track_b_grp<kGrpMinBlocks, false>, (const void*)k_track_b_grp_fused<kGrpMinBlocks, false>, gb, 256,
                   0, s, L, st, tickets + 1, residual, counts, seg, min_count, fin, ng, gpc);
-    } else {
-        k_track_a<2, false><<<g, 256, 0, s>>>(L, st, residual, counts);
-        k_track_b<2, false><<<g, 256, 0, s>>>(L, st, tickets + 1, residual, counts, seg, min_count, fin);
     }
     return 2;
+}
+
+// Whether k_track_loop keeps its lists for n pixels in global memory.
+bool track_list_global(int n) {
+    const int g = track_cluster_grid(n);
+    return (n + g * 256 - 1) / (g * 256) > kLoopSmemChunks;
+}
+
+// k_track_loop's launch for these levels, when its grid is resident at once.
+int launch_track_loop(const TrackLevel lv[3], const int iters[3], const int min_count[3], TrackState* st,
+                      TrackSync* sync, void* list, cudaStream_t s, bool compensated) {
+    if (launch_recorder()) return 0;
+    LoopArgs A{};
+    int grid = 0, chunks = 0;
+    bool global = false;
+    for (int l = 0; l < 3; ++l) {
+        A.L[l] = lv[l];
+        A.iters[l] = iters[l];
+        A.min_count[l] = min_count[l];
+        const int n = lv[l].W * lv[l].H;
+        A.G[l] = n > 0 ? track_cluster_grid(n) : 0;
+        if (iters[l] <= 0) continue;
+        if (n <= 0 || !lv[l].rgbok) return 0;
+        grid = std::max(grid, A.G[l]);
+        chunks = std::max(chunks, (n + A.G[l] * 256 - 1) / (A.G[l] * 256));
+        global = global || track_list_global(n);
+    }
+    const int per = (grid / kTrackCluster + 3) / 4;
+    if (grid == 0 || per * kTrackCluster > kLoopRows) return 0;
+    A.chunks = chunks;
+    A.nbuf = global ? kLoopRing : chunks;
+    A.list = (unsigned char*)list;
+    const int fixed = global ? kLoopScratch : std::max(chunks * kLoopListBytes, kLoopScratch);
+    if (grid / kTrackCluster > loop_clusters(compensated, global)) return 0;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(256);
+    cfg.dynamicSmemBytes = (size_t)A.nbuf * sizeof(LoopStage) + fixed;
+    cfg.stream = s;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeCooperative;
+    at[0].val.cooperative = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    void* args[] = {&A, &st, &sync};
+    if (cudaLaunchKernelExC(&cfg, loop_kernel(compensated, global), args) == cudaSuccess) return 1;
+    cudaGetLastError();
+    return 0;
 }
 
 int launch_step_icp(const TrackLevel& L, const DevPose& cur, const DevPose& last, float* partials,
