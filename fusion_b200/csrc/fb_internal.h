@@ -366,10 +366,11 @@ int launch_match2(const float* q, int nq, const float* t, int nt, int2* idx, flo
 bool pose_estimate(const double* src, const double* ref, int n, int iterations, bool check_angle, uint64_t seed,
                    double T[16], uint8_t* outlier);
 
-// Marching-cubes mesh of the map over its n_blocks allocated blocks: *total =
-// triangles found; the first min(total, cap) written to V / N (float3 per
-// vertex) and C (uchar3) when all three are given.  Synchronous on st.
-int launch_mesh(const MapView& m, int n_blocks, float* V, float* N, uint8_t* C, unsigned long long cap,
+// Marching-cubes mesh of the map: *total = triangles found; the first
+// min(total, cap) written to V / N (float3 per vertex) and C (uchar3) when all
+// three are given.  scratch: mesh_scratch_bytes(NS).  Synchronous on st.
+size_t mesh_scratch_bytes(int n_blocks);
+int launch_mesh(const MapView& m, void* scratch, float* V, float* N, uint8_t* C, unsigned long long cap,
                 unsigned long long* total, cudaStream_t st);
 
 }  // namespace fb

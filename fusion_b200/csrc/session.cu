@@ -289,7 +289,8 @@ bool carve_session(fb_session* s, const fb_config* cfg) {
          dalloc(s, &s->tickets, 4) &&
          dalloc(s, (char**)&s->residual, track_list_bytes(s->W[0] * s->H[0])) &&
          dalloc(s, &s->counts, (size_t)kTrackMaxBlocks * kTrackWarps) &&
-         dalloc(s, &s->scratch_pose, 1) && dalloc(s, &s->d_out, 1);
+         dalloc(s, &s->scratch_pose, 1) && dalloc(s, &s->d_out, 1) &&
+         dalloc(s, &s->mesh_scratch, mesh_scratch_bytes(cfg->num_blocks));
     MapView& m = s->map;
     if (ok) {
         m.NB = cfg->num_buckets;

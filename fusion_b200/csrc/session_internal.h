@@ -8,6 +8,7 @@
 
 #include <cstdio>
 #include <map>
+#include <mutex>
 #include <tuple>
 #include <vector>
 
@@ -132,6 +133,8 @@ struct fb_session {
     MapView map;
     MapCounters* ctr;
     DevPose* scratch_pose;
+    char* mesh_scratch;        // triangle counts and offsets of the pool's blocks (launch_mesh)
+    std::mutex mesh_lock;      // held while a mesh uses it
     FrameOut* d_out;
     FrameOut* h_out;           // pinned
     FrameOut* h_out_dev;       // h_out's device address (cudaHostGetDevicePointer), null if none

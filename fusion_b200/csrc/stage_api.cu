@@ -419,12 +419,13 @@ int fb_mesh_scene(fb_session* s, float* vertex, float* normal, uint8_t* color, u
     const bool any = vertex || normal || color;
     if (any && !(vertex && normal && color)) return FB_EINVAL;
     cudaStream_t st = stream ? as_stream(stream) : s->stream;
-    MapCounters c;
-    FB_CUDA(cudaMemcpyAsync(&c, s->ctr, sizeof c, cudaMemcpyDeviceToHost, st));
-    FB_CUDA(cudaStreamSynchronize(st));
     unsigned long long total = 0;
-    const int rc = launch_mesh(s->map, c.n_alloc, vertex, normal, color, any ? max_triangles : 0, &total, st);
-    if (rc != FB_OK) return rc;
+    {
+        // one mesh at a time uses the session's scratch
+        std::lock_guard<std::mutex> guard(s->mesh_lock);
+        const int rc = launch_mesh(s->map, s->mesh_scratch, vertex, normal, color, any ? max_triangles : 0, &total, st);
+        if (rc != FB_OK) return rc;
+    }
     s->launches += any ? 3 : 2;
     *no_triangles = total;
     return FB_OK;
