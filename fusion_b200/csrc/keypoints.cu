@@ -20,6 +20,8 @@
 // Everything is deterministic: box sums are integer, candidates are ranked
 // by (response, sample index) with a total order, and every reduction has a
 // fixed order.
+#include <cooperative_groups.h>
+
 #include <algorithm>
 #include <cmath>
 #include <cstdio>
@@ -27,7 +29,10 @@
 #include <mutex>
 
 #include "../../include/fusion_b200.h"
+#include "fb_async.cuh"
 #include "fb_internal.h"
+
+namespace cg = cooperative_groups;
 
 namespace fb {
 
@@ -459,87 +464,211 @@ __global__ void __launch_bounds__(1024) k_backproject(const float4* __restrict__
 // ----------------------------------------------------------------- matching
 
 // Two nearest train descriptors of each query by L2 distance (BFMatcher
-// knnMatch with k = 2).  One CTA of 256 threads per 32 queries: train tiles
-// of 64 descriptors in shared memory, 8 threads per query each taking every
-// 8th train of the tile, best two merged in a fixed order.  Distances are
-// square roots of the sums of squares in descriptor order; ties go to the
-// lower train index.
-__global__ void __launch_bounds__(256) k_match2(const float* __restrict__ Q, int nq, const float* __restrict__ T,
-                                                int nt, int2* __restrict__ idx, float2* __restrict__ dist) {
-    __shared__ float sq[32][kKeyDesc + 1];
-    __shared__ float st[64][kKeyDesc + 1];
-    const int q0 = blockIdx.x * 32;
-    for (int t = threadIdx.x; t < 32 * kKeyDesc; t += 256) {
-        const int r = t / kKeyDesc, c = t % kKeyDesc;
-        sq[r][c] = (q0 + r < nq) ? Q[(size_t)(q0 + r) * kKeyDesc + c] : 0.f;
+// knnMatch with k = 2).  Distances are square roots of the sums of squares in
+// descriptor order (one FMA chain per pair); the two nearest are the smallest
+// by (distance, train index).
+//
+// FP32 arithmetic bounds it (128 operations per pair; descriptors are read
+// once per 32 queries).  A thread holds kTQ queries x 4 trains; the queries
+// are staged negated and interleaved, so a read gives pairs of them for
+// two-lane operations (f32x2: half the instructions; (t - q)^2 has the bits
+// of (q - t)^2).  A warp's lanes share their queries (broadcast reads) and
+// own consecutive trains (rows of 68 floats: no bank conflicts).  The trains are dealt to the CTAs of
+// a cluster, tile by tile, and their best pairs merged through distributed
+// shared memory, so few queries still fill the chip.  900 queries x 20 000
+// trains: 140 us (1728 us with one CTA per 32 queries and two shared loads per
+// two operations); the FMA pipes' floor is 64 us, a fifth of the SMs get no
+// cluster, and the rest issue in three cycles of four.
+constexpr int kMatchTrains = 4;                       // trains per thread and step
+constexpr int kMatchRow = kKeyDesc + 4;               // floats per staged row
+
+struct Best2 {
+    float d1, d2;
+    int i1, i2;
+};
+
+// a < b in (distance, index) order; index -1 (none) comes last.
+__device__ __forceinline__ bool nearer(float a, int ia, float b, int ib) {
+    return a < b || (a == b && ia >= 0 && (ib < 0 || ia < ib));
+}
+
+__device__ __forceinline__ Best2 merge2(const Best2& a, const Best2& b) {
+    Best2 r;
+    if (nearer(a.d1, a.i1, b.d1, b.i1)) {
+        r.d1 = a.d1;
+        r.i1 = a.i1;
+        const bool own = nearer(a.d2, a.i2, b.d1, b.i1);
+        r.d2 = own ? a.d2 : b.d1;
+        r.i2 = own ? a.i2 : b.i1;
+    } else {
+        r.d1 = b.d1;
+        r.i1 = b.i1;
+        const bool own = nearer(a.d1, a.i1, b.d2, b.i2);
+        r.d2 = own ? a.d1 : b.d2;
+        r.i2 = own ? a.i1 : b.i2;
     }
-    const int qi = threadIdx.x >> 3, part = threadIdx.x & 7;
-    float b1 = INFINITY, b2 = INFINITY;
-    int i1 = -1, i2 = -1;
-    for (int t0 = 0; t0 < nt; t0 += 64) {
-        __syncthreads();
-        for (int t = threadIdx.x; t < 64 * kKeyDesc; t += 256) {
+    return r;
+}
+
+// Rows [r0, r0 + rows) of D (n of them, kKeyDesc floats each) into staged
+// rows by cp.async, zeros beyond n; 16 bytes at a time where D allows it.
+__device__ __forceinline__ void stage_rows(float* dst, const float* __restrict__ D, int r0, int rows, int n) {
+    if (((uintptr_t)D & 15) == 0) {
+        for (int t = threadIdx.x; t < rows * (kKeyDesc / 4); t += blockDim.x) {
+            const int r = t / (kKeyDesc / 4), c = t % (kKeyDesc / 4);
+            const bool in = r0 + r < n;
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem_addr(dst + r * kMatchRow + 4 * c)),
+                         "l"(D + (in ? (size_t)(r0 + r) * kKeyDesc + 4 * c : 0)), "r"(in ? 16 : 0)
+                         : "memory");
+        }
+    } else {
+        for (int t = threadIdx.x; t < rows * kKeyDesc; t += blockDim.x) {
             const int r = t / kKeyDesc, c = t % kKeyDesc;
-            st[r][c] = (t0 + r < nt) ? T[(size_t)(t0 + r) * kKeyDesc + c] : 0.f;
+            const bool in = r0 + r < n;
+            asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(smem_addr(dst + r * kMatchRow + c)),
+                         "l"(D + (in ? (size_t)(r0 + r) * kKeyDesc + c : 0)), "r"(in ? 4 : 0)
+                         : "memory");
+        }
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+}
+
+__device__ __forceinline__ unsigned long long twice(float v) {
+    unsigned long long r;
+    asm("mov.b64 %0, {%1, %1};" : "=l"(r) : "f"(v));
+    return r;
+}
+
+// acc + (t - q)^2 of two queries; nq = the negated queries.
+__device__ __forceinline__ void add_square(unsigned long long& acc, unsigned long long t, unsigned long long nq) {
+    asm("{\n"
+        ".reg .b64 d;\n"
+        "add.rn.f32x2 d, %1, %2;\n"
+        "fma.rn.f32x2 %0, d, d, %0;\n"
+        "}\n"
+        : "+l"(acc)
+        : "l"(t), "l"(nq));
+}
+
+// kTQ queries per thread; kQG x kParts warps = query groups x parts of the
+// train tile.  Queries per CTA kQG * kTQ, trains per tile 128 * kParts.
+template <int kTQ, int kQG, int kParts>
+__global__ void __launch_bounds__(32 * kQG * kParts) k_match2(const float* __restrict__ Q, int nq, const float* __restrict__ T,
+                                                int nt, int2* __restrict__ idx, float2* __restrict__ dist) {
+    constexpr int kQueries = kQG * kTQ, kTile = 32 * kMatchTrains * kParts;
+    extern __shared__ __align__(16) float dyn_match[];
+    float* const sq = dyn_match;                                  // [value][query], negated
+    float* const st = dyn_match + kKeyDesc * kQueries;            // two tiles
+    __shared__ Best2 s_best[kQG * kParts][kTQ];
+    __shared__ Best2 s_cta[kQueries];
+    cg::cluster_group cl = cg::this_cluster();
+    const int rank = (int)cl.block_rank(), ranks = (int)cl.num_blocks();
+    const int q0 = ((int)blockIdx.x / ranks) * kQueries;
+    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31, qg = w % kQG, part = w / kQG;
+    const int tiles = (nt + kTile - 1) / kTile;
+    Best2 best[kTQ];
+#pragma unroll
+    for (int a = 0; a < kTQ; ++a) best[a] = Best2{INFINITY, INFINITY, -1, -1};
+    for (int t = threadIdx.x; t < kKeyDesc * kQueries; t += blockDim.x) {
+        const int r = t % kQueries, c = t / kQueries;
+        sq[t] = q0 + r < nq ? -Q[(size_t)(q0 + r) * kKeyDesc + c] : 0.f;
+    }
+    if (rank < tiles) stage_rows(st, T, rank * kTile, kTile, nt);
+    int buf = 0;
+    for (int tile = rank; tile < tiles; tile += ranks, buf ^= 1) {
+        if (tile + ranks < tiles) {
+            stage_rows(st + (buf ^ 1) * kTile * kMatchRow, T, (tile + ranks) * kTile, kTile, nt);
+            asm volatile("cp.async.wait_group 1;" ::: "memory");
+        } else {
+            asm volatile("cp.async.wait_group 0;" ::: "memory");
         }
         __syncthreads();
-        for (int r = part; r < 64 && t0 + r < nt; r += 8) {
-            float acc = 0.f;
-#pragma unroll 16
-            for (int c = 0; c < kKeyDesc; ++c) {
-                const float d = sq[qi][c] - st[r][c];
-                acc = fmaf(d, d, acc);
-            }
-            const int ti = t0 + r;
-            if (acc < b1) {
-                b2 = b1;
-                i2 = i1;
-                b1 = acc;
-                i1 = ti;
-            } else if (acc < b2) {
-                b2 = acc;
-                i2 = ti;
-            }
-        }
-    }
-    // merge the 8 partial results of each query (xor tree: fixed order)
-    auto less = [](float a, int ia, float b, int ib) { return a < b || (a == b && ia >= 0 && (ib < 0 || ia < ib)); };
+        const float* const qp = sq + qg * kTQ;
+        const float* const tp = st + (buf * kTile + part * 32 * kMatchTrains + lane) * kMatchRow;
+        unsigned long long acc2[kTQ / 2][kMatchTrains] = {};
+#pragma unroll 4
+        for (int c = 0; c < kKeyDesc; c += 4) {
+            float4 t[kMatchTrains];
 #pragma unroll
-    for (int off = 1; off < 8; off <<= 1) {
-        const float ob1 = __shfl_xor_sync(0xffffffffu, b1, off), ob2 = __shfl_xor_sync(0xffffffffu, b2, off);
-        const int oi1 = __shfl_xor_sync(0xffffffffu, i1, off), oi2 = __shfl_xor_sync(0xffffffffu, i2, off);
-        float c1, c2;
-        int j1, j2;
-        if (less(b1, i1, ob1, oi1)) {
-            c1 = b1;
-            j1 = i1;
-            if (less(b2, i2, ob1, oi1)) {
-                c2 = b2;
-                j2 = i2;
-            } else {
-                c2 = ob1;
-                j2 = oi1;
-            }
-        } else {
-            c1 = ob1;
-            j1 = oi1;
-            if (less(b1, i1, ob2, oi2)) {
-                c2 = b1;
-                j2 = i1;
-            } else {
-                c2 = ob2;
-                j2 = oi2;
+            for (int b = 0; b < kMatchTrains; ++b)
+                t[b] = *reinterpret_cast<const float4*>(tp + 32 * b * kMatchRow + c);
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                unsigned long long q[kTQ / 2];
+                if constexpr (kTQ == 4) {
+                    const ulonglong2 v = *reinterpret_cast<const ulonglong2*>(qp + (c + e) * kQueries);
+                    q[0] = v.x;
+                    q[kTQ / 2 - 1] = v.y;
+                } else {
+                    q[0] = *reinterpret_cast<const unsigned long long*>(qp + (c + e) * kQueries);
+                }
+#pragma unroll
+                for (int b = 0; b < kMatchTrains; ++b) {
+                    const unsigned long long tt = twice(e == 0 ? t[b].x : e == 1 ? t[b].y : e == 2 ? t[b].z : t[b].w);
+#pragma unroll
+                    for (int a = 0; a < kTQ / 2; ++a) add_square(acc2[a][b], tt, q[a]);
+                }
             }
         }
-        b1 = c1;
-        i1 = j1;
-        b2 = c2;
-        i2 = j2;
+        float acc[kTQ][kMatchTrains];
+#pragma unroll
+        for (int a = 0; a < kTQ / 2; ++a)
+#pragma unroll
+            for (int b = 0; b < kMatchTrains; ++b)
+                asm("mov.b64 {%0, %1}, %2;" : "=f"(acc[2 * a][b]), "=f"(acc[2 * a + 1][b]) : "l"(acc2[a][b]));
+        // a lane's trains come in ascending order: a tie keeps the earlier
+        const int t0 = tile * kTile + part * 32 * kMatchTrains + lane;
+#pragma unroll
+        for (int b = 0; b < kMatchTrains; ++b) {
+            const int ti = t0 + 32 * b;
+            if (ti >= nt) break;
+#pragma unroll
+            for (int a = 0; a < kTQ; ++a) {
+                const float v = acc[a][b];
+                if (v < best[a].d2) {
+                    const bool first = v < best[a].d1;
+                    best[a].d2 = first ? best[a].d1 : v;
+                    best[a].i2 = first ? best[a].i1 : ti;
+                    if (first) {
+                        best[a].d1 = v;
+                        best[a].i1 = ti;
+                    }
+                }
+            }
+        }
+        __syncthreads();   // the tile's buffer is read
     }
-    if (part == 0 && q0 + qi < nq) {
-        idx[q0 + qi] = make_int2(i1, i2);
-        dist[q0 + qi] = make_float2(sqrtf(b1), sqrtf(b2));
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    __syncwarp();
+#pragma unroll
+    for (int a = 0; a < kTQ; ++a) {
+#pragma unroll
+        for (int off = 1; off < 32; off <<= 1) {
+            Best2 o;
+            o.d1 = __shfl_xor_sync(0xffffffffu, best[a].d1, off);
+            o.d2 = __shfl_xor_sync(0xffffffffu, best[a].d2, off);
+            o.i1 = __shfl_xor_sync(0xffffffffu, best[a].i1, off);
+            o.i2 = __shfl_xor_sync(0xffffffffu, best[a].i2, off);
+            best[a] = merge2(best[a], o);
+        }
+        if (lane == 0) s_best[w][a] = best[a];
     }
+    __syncthreads();
+    if (threadIdx.x < kQueries) {
+        const int g = threadIdx.x / kTQ, a = threadIdx.x % kTQ;
+        Best2 r = s_best[g][a];
+#pragma unroll
+        for (int p = 1; p < kParts; ++p) r = merge2(r, s_best[g + p * kQG][a]);
+        s_cta[threadIdx.x] = r;
+    }
+    cl.sync();
+    if (rank == 0 && threadIdx.x < kQueries && q0 + (int)threadIdx.x < nq) {
+        Best2 r = s_cta[threadIdx.x];
+        for (int p = 1; p < ranks; ++p) r = merge2(r, cl.map_shared_rank(s_cta, p)[threadIdx.x]);
+        idx[q0 + threadIdx.x] = make_int2(r.i1, r.i2);
+        dist[q0 + threadIdx.x] = make_float2(sqrtf(r.d1), sqrtf(r.d2));
+    }
+    cl.sync();   // the other blocks' results are read
 }
 
 // ------------------------------------------------------------------ launch
@@ -632,10 +761,63 @@ int launch_backproject(const KeyScratch& ks, int n, const float* depth, int dp, 
     return cudaGetLastError() == cudaSuccess ? FB_OK : FB_ECUDA;
 }
 
+// Shapes: 32 queries x 256 trains by 512 threads (one CTA per SM), and 8
+// queries x 256 trains by 256 threads for fewer queries than fill the chip so.
+// The cluster size is the one whose waves of resident clusters take the
+// fewest tiles (clusters of 5 leave SMs of a GPC unused, and so on: the
+// runtime knows how many of a size are resident).
 int launch_match2(const float* q, int nq, const float* t, int nt, int2* idx, float2* dist, cudaStream_t st) {
     if (nq <= 0) return FB_OK;
-    k_match2<<<(nq + 31) / 32, 256, 0, st>>>(q, nq, t, nt, idx, dist);
-    return cudaGetLastError() == cudaSuccess ? FB_OK : FB_ECUDA;
+    constexpr int kTile = 256;
+    int dev = 0, sms = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64 ||
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
+        return FB_ECUDA;
+    const int tiles = (nt + kTile - 1) / kTile;
+    const bool wide = (nq + 31) / 32 * std::min(8, std::max(tiles, 1)) >= sms;
+    const int queries = wide ? 32 : 8, threads = wide ? 512 : 256, groups = (nq + queries - 1) / queries;
+    const size_t smem = ((size_t)queries * kKeyDesc + 2 * kTile * kMatchRow) * sizeof(float);
+    const void* k = wide ? (const void*)k_match2<4, 8, 2> : (const void*)k_match2<2, 4, 2>;
+    cudaLaunchConfig_t cfg = {};
+    cfg.blockDim = dim3(threads);
+    cfg.dynamicSmemBytes = smem;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    int ranks = 1;
+    {
+        static std::mutex lock;
+        static int resident[64][2][9] = {};   // clusters of each size, by device and shape
+        std::lock_guard<std::mutex> guard(lock);
+        int* r = resident[dev][wide];
+        if (!r[0]) {
+            if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
+                return FB_ECUDA;
+            for (int c = 1; c <= 8; ++c) {
+                at[0].val.clusterDim.x = (unsigned)c;
+                cfg.gridDim = dim3((unsigned)c);
+                if (cudaOccupancyMaxActiveClusters(&r[c], k, &cfg) != cudaSuccess) r[c] = 0;
+            }
+            cudaGetLastError();
+            r[0] = 1;
+        }
+        long long best = -1;
+        for (int c = 1; c <= 8 && (c == 1 || c <= tiles); ++c) {
+            if (r[c] <= 0) continue;
+            const long long cost = (long long)((groups + r[c] - 1) / r[c]) * ((tiles + c - 1) / c);
+            if (best < 0 || cost < best) {
+                best = cost;
+                ranks = c;
+            }
+        }
+    }
+    at[0].val.clusterDim.x = (unsigned)ranks;
+    cfg.gridDim = dim3((unsigned)(groups * ranks));
+    cfg.stream = st;
+    void* args[] = {&q, &nq, &t, &nt, &idx, &dist};
+    return cudaLaunchKernelExC(&cfg, k, args) == cudaSuccess ? FB_OK : FB_ECUDA;
 }
 
 // ------------------------------------------------------------- pose solver
