@@ -215,20 +215,31 @@ struct MapCounters {
     int excess_total;      // new blocks going to the excess list this frame
     unsigned int err;      // ErrFlag bits, sticky
     int seq_path;          // last allocation used the sequential path
-    // snapshot taken before insertion (read by the insert kernel only)
-    int snap_M, snap_hc, snap_ep, snap_na;
-    int fast;              // the parallel insertion path applies
+    int unused[5];         // (a snapshot holds this struct: its layout stays)
     unsigned int ray_next; // tile counter of the queued raycast (zeroed with the z ranges)
-    unsigned int scan_ticket; // chunk-scan blocks done this frame (the last one resets it)
+    unsigned int unused2;
 };
 
-struct NewBlock {
-    short x, y, z, pad;
+struct __align__(16) NewBlock {
+    short x, y, z;
+    short he;              // its bucket's head slot is empty
     uint32_t bucket;
     int setslot;           // slot in the request set (cleared after insertion)
-    int j;                 // arrival index inside the bucket
-    int rank;              // canonical rank: order by (bucket, x, y, z)
-    int pad2;
+    int next;              // the bin's block requested before (AllocBins), -1: none
+    int fills;             // he, and the first of its bucket to be requested: one per such bucket
+    int pad[2];
+};
+
+// One frame's new blocks by bins of consecutive buckets (bucket >> bin_shift):
+// requests count and chain them, and an inserted block finds its canonical
+// rank from the scanned counts and its bin's chain.  Zero counts and empty
+// chains between frames.
+constexpr int kAllocBins = 4096;
+struct AllocBins {
+    unsigned long long cnt[kAllocBins];   // blocks | blocks with `fills` << 32
+    int head[kAllocBins];                 // the bin's newest request, -1: none
+    unsigned ticket;                      // insertion blocks done (the last one resets it)
+    unsigned pad[3];
 };
 
 // Geometry of the map (runtime form of DeviceMap's constants).
@@ -254,13 +265,10 @@ struct MapView {
     int reqcap;
     NewBlock* newblk;           // this frame's new blocks (newcap)
     int newcap;
-    int* order;                 // canonical order -> newblk index (newcap)
-    int* arrival;               // bucket segment -> newblk index (newcap)
+    int* order;                 // canonical order -> newblk index (newcap; the sequential path's)
     int* bucket_cnt;            // NB, zero between frames
-    int* bucket_start;          // NB
-    int* bucket_x;              // NB: excess start << 1 | head-was-empty
-    int* chunk_sums;            // 2 * nchunks
-    int nchunks;
+    AllocBins* bins;
+    int bin_shift;
     float* zmin;                // z-range image, zc x zr
     float* zmax;
     int zc, zr;
@@ -285,17 +293,24 @@ inline int raycast_tiles(int W, int H, int bx, int by) {
 }
 inline int raycast_tile_cap(int W, int H) { return W * H / 32 + W + H + 1; }
 
-constexpr int kScanChunk = 4096;
 constexpr int kMinNewBlocks = 1 << 16;
 
 int launch_map_reset(const MapView& m, cudaStream_t s);
 // pose: device pointer; skip: device flag (nonzero: do nothing), may be null
+// zinit: also clears the z-range images and counters (for launch_view).
 int launch_allocate(const MapView& m, const float* raw, int rp, int W, int H, const Intr& k, const DevPose* pose,
-                     const int* skip, cudaStream_t s);
+                     const int* skip, cudaStream_t s, bool zinit = false);
 // after_allocate: launched right after launch_allocate, whose last kernel
 // already zeroed the visible-block and rendering-rectangle counters.
 int launch_visibility(const MapView& m, int W, int H, const Intr& k, const DevPose* pose, const int* skip,
                        cudaStream_t s, bool after_allocate = false);
+// Visibility and z ranges of a fused frame in one launch, right after
+// launch_allocate(zinit): the visible blocks are projected where they are
+// found.  The integration then clears the dense block index (clear_grid) and
+// launch_grid_fill fills it.
+int launch_view(const MapView& m, int W, int H, const Intr& k, const DevPose* pose, const int* skip, cudaStream_t s,
+                int rc_tiles);
+int launch_grid_fill(const MapView& m, const int* skip, cudaStream_t s);
 // The visible entries (at most `capacity`) in the reference's 32-byte
 // HashEntry layout at dst; the table, voxels and counters in the reference's
 // layouts (the reference form's voxels are the reference's already: the
@@ -311,7 +326,7 @@ int launch_fuse_records(const MapView& m, const float* raw, int rp, const uint8_
 // ctas_per_sm: the grid (CTAs per SM, each taking every grid-th visible
 // block); 0: the form's default.  Results do not depend on it.
 int launch_integrate(const MapView& m, int W, int H, const Intr& k, const DevPose* pose, const int* skip,
-                     cudaStream_t s, int ctas_per_sm = 0);
+                     cudaStream_t s, int ctas_per_sm = 0, bool clear_grid = false);
 // rc_tiles: tiles of the raycast that follows (raycast_tiles), whose block
 // order this pass prepares from the last raycast's costs; 0: leave it as it is.
 int launch_zrange(const MapView& m, const Intr& k, const DevPose* pose, const int* skip, cudaStream_t s,

@@ -12,21 +12,19 @@
 //              (Fusion::CreateBlocks, FuseMap.cu:80-111); blocks that are not in
 //              the map go into a per-frame open-addressing request set (CAS on
 //              64-bit keys); the first insert of a key appends it to the list
-//              of new blocks.
-//   scan / place / rank : a counting sort of the new blocks by bucket
-//              (per-bucket counters taken by the requests, a two-level scan
-//              over all buckets whose top level runs in the last chunk block
-//              to finish), then the rank of each block inside its bucket by
-//              coordinates.
-//   insert   : (also the counters after the frame and the clearing of the
-//              per-bucket counters) each new block computes from its rank alone where the
-//              sequential insertion would put it: free-stack position, head
-//              slot or excess slot, and its chain link; the one block per
-//              bucket that extends an existing chain links the old tail.  If
-//              the pool or the excess list would run out, or an earlier
-//              exhaustion left empty entries inside chains, a single thread
-//              performs the same insertions one by one with the reference's
-//              exact CreateBlock rules instead.
+//              of new blocks, counts it in its bin of consecutive buckets and
+//              chains it there.
+//   insert   : each new block finds its canonical rank -- its bin's start plus
+//              the blocks of the bin's chain before it -- and computes from
+//              it alone where the sequential insertion would put it:
+//              free-stack position, head slot or excess slot, and its chain
+//              link; the one block per bucket that extends an existing chain
+//              links the old tail.  The last block to finish writes the
+//              counters after the frame and clears the bins.  If the pool or
+//              the excess list would run out, or an earlier exhaustion left
+//              empty entries inside chains, a single thread of that last
+//              block performs the same insertions one by one with the
+//              reference's exact CreateBlock rules instead.
 // Visibility walks the list of allocated entries rather than every slot of
 // the table (CheckVisibleBlockKernel, FuseMap.cu:113-138, scans all of them).
 // Integration processes one visible block per CTA iteration: 256 threads, two
@@ -37,20 +35,21 @@
 
 #include "fb_fused.cuh"
 #include "fb_internal.h"
+#include "fb_view.cuh"
 
 namespace fb {
 
-// FindEntry (DeviceMap.cu:122-135): slot of the live entry for a block, or -1.
-__device__ __forceinline__ int find_slot(const MapView& m, int x, int y, int z) {
-    int b = (int)bucket_of_m(x, y, z, (uint32_t)m.NB, m.nb_mask);
+// Whether block (x, y, z) has a live entry (FindEntry, DeviceMap.cu:122-135);
+// its bucket b, and he = the bucket's head slot is empty.
+__device__ __forceinline__ bool find_entry(const MapView& m, int x, int y, int z, uint32_t b, bool& he) {
     HEntry e = m.entries[b];
-    if (e.ptr != -1 && e.x == x && e.y == y && e.z == z) return b;
+    he = e.ptr == -1;
+    if (!he && e.x == x && e.y == y && e.z == z) return true;
     for (int guard = 0; e.offset > 0 && e.offset <= m.NE && guard <= m.NE; ++guard) {
-        int s = m.NB + e.offset - 1;
-        e = m.entries[s];
-        if (e.x == x && e.y == y && e.z == z && e.ptr != -1) return s;
+        e = m.entries[m.NB + e.offset - 1];
+        if (e.x == x && e.y == y && e.z == z && e.ptr != -1) return true;
     }
-    return -1;
+    return false;
 }
 
 __device__ __forceinline__ unsigned long long block_key(int x, int y, int z) {
@@ -73,7 +72,9 @@ __device__ __forceinline__ void request_block(const MapView& m, int x, int y, in
         atomicOr(&m.ctr->err, kErrCoordRange);
         return;
     }
-    if (find_slot(m, x, y, z) >= 0) return;
+    const uint32_t bucket = bucket_of_m(x, y, z, (uint32_t)m.NB, m.nb_mask);
+    bool he;
+    if (find_entry(m, x, y, z, bucket, he)) return;
     const unsigned long long key = block_key(x, y, z);
     uint32_t h = mix64(key) & (uint32_t)(m.reqcap - 1);
     for (int probe = 0; probe < 64; ++probe) {
@@ -85,14 +86,16 @@ __device__ __forceinline__ void request_block(const MapView& m, int x, int y, in
                 nb.x = (short)x;
                 nb.y = (short)y;
                 nb.z = (short)z;
-                nb.pad = 0;
-                nb.bucket = bucket_of_m(x, y, z, (uint32_t)m.NB, m.nb_mask);
+                nb.he = he ? 1 : 0;
+                nb.bucket = bucket;
                 nb.setslot = (int)h;
-                // arrival order inside the bucket (any order: the rank
-                // below orders the bucket by coordinates)
-                nb.j = atomicAdd(&m.bucket_cnt[nb.bucket], 1);
-                nb.rank = 0;
-                nb.pad2 = 0;
+                // one block of a bucket with an empty head fills it: which of
+                // them is counted for it does not matter
+                nb.fills = atomicAdd(&m.bucket_cnt[bucket], 1) == 0 && he ? 1 : 0;
+                const uint32_t bin = bucket >> m.bin_shift;
+                atomicAdd(&m.bins->cnt[bin], 1ull | (unsigned long long)nb.fills << 32);
+                nb.next = atomicExch(&m.bins->head[bin], idx);
+                nb.pad[0] = nb.pad[1] = 0;
                 m.newblk[idx] = nb;
             } else {
                 atomicOr(&m.ctr->err, kErrNewListFull);
@@ -107,13 +110,8 @@ __device__ __forceinline__ void request_block(const MapView& m, int x, int y, in
 }
 
 // Fusion::CreateBlocks (FuseMap.cu:80-111) for one pixel of the raw depth map.
-__device__ __forceinline__ void alloc_requests_body(const BlockCtx& ctx, MapView m, const float* __restrict__ raw,
-                                                    int rp, int W, int H, Intr k, const DevPose* __restrict__ posep,
-                                                    const int* __restrict__ skip) {
-    if (skip && *skip) return;
-    const int x = ctx.bx * blockDim.x + threadIdx.x;
-    const int y = ctx.by * blockDim.y + threadIdx.y;
-    if (x >= W || y >= H) return;
+__device__ __forceinline__ void request_pixel(const MapView& m, const float* __restrict__ raw, int rp, int x, int y,
+                                              const Intr& k, const DevPose* __restrict__ posep) {
     const float z = raw[(size_t)y * rp + x];
     const float dmin = m.g.depth_min, dmax = m.g.depth_max;
     if (isnan(z) || z < dmin || z > dmax) return;
@@ -147,206 +145,41 @@ __device__ __forceinline__ void alloc_requests_body(const BlockCtx& ctx, MapView
     }
 }
 
+// The last of n blocks to come here (true in every thread of it): what the
+// blocks wrote before is visible to it.  It resets the ticket.
+__device__ __forceinline__ bool last_to_finish(unsigned* ticket, unsigned n) {
+    __shared__ bool s_last;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        __threadfence();
+        s_last = atomicAdd(ticket, 1u) == n - 1u;
+        if (s_last) *ticket = 0;
+        __threadfence();
+    }
+    __syncthreads();
+    return s_last;
+}
+
+__device__ __forceinline__ void alloc_requests_body(const BlockCtx& ctx, MapView m, const float* __restrict__ raw,
+                                                    int rp, int W, int H, Intr k, const DevPose* __restrict__ posep,
+                                                    const int* __restrict__ skip) {
+    if (skip && *skip) return;   // the whole grid
+    const int x = ctx.bx * blockDim.x + threadIdx.x;
+    const int y = ctx.by * blockDim.y + threadIdx.y;
+    if (x < W && y < H) request_pixel(m, raw, rp, x, y, k, posep);
+}
+
 __global__ void __launch_bounds__(256) k_alloc_requests(MapView m, const float* __restrict__ raw, int rp, int W,
                                   int H, Intr k, const DevPose* __restrict__ posep, const int* __restrict__ skip) {
     alloc_requests_body(own_ctx(), m, raw, rp, W, H, k, posep, skip);
 }
 FB_FUSED_KERNEL(k_alloc_requests, alloc_requests_body, 256)
 
-__device__ __forceinline__ void scan_top_body(MapView m);
-
-// Per chunk of kScanChunk buckets: number of new blocks, and of those that go
-// to the excess list (all but the first when the bucket's head slot is empty).
-// The last block to finish then scans the chunk sums (scan_top_body).
-__device__ __forceinline__ void scan_chunks_body(const BlockCtx& ctx, MapView m) {
-    __shared__ int s_c[256], s_x[256];
-    __shared__ bool s_last;
-    const int base = ctx.bx * kScanChunk;
-    const bool any = m.ctr->n_req > 0;
-    int c = 0, xs = 0;
-    for (int q = threadIdx.x; any && q < kScanChunk; q += 256) {
-        int b = base + q;
-        if (b >= m.NB) break;
-        int n = m.bucket_cnt[b];
-        if (n) {
-            int he = m.entries[b].ptr == -1 ? 1 : 0;
-            c += n;
-            xs += n - he;
-        }
-    }
-    s_c[threadIdx.x] = c;
-    s_x[threadIdx.x] = xs;
-    __syncthreads();
-    for (int o = 128; o > 0; o >>= 1) {
-        if (threadIdx.x < o) {
-            s_c[threadIdx.x] += s_c[threadIdx.x + o];
-            s_x[threadIdx.x] += s_x[threadIdx.x + o];
-        }
-        __syncthreads();
-    }
-    if (threadIdx.x == 0) {
-        m.chunk_sums[2 * ctx.bx] = s_c[0];
-        m.chunk_sums[2 * ctx.bx + 1] = s_x[0];
-        __threadfence();
-        s_last = atomicAdd(&m.ctr->scan_ticket, 1u) == (unsigned)ctx.gx - 1u;
-    }
-    __syncthreads();
-    if (!s_last) return;
-    __threadfence();
-    if (threadIdx.x == 0) m.ctr->scan_ticket = 0;
-    scan_top_body(m);
-}
-
-__global__ void __launch_bounds__(256) k_scan_chunks(MapView m) {
-    scan_chunks_body(own_ctx(), m);
-}
-FB_FUSED_KERNEL(k_scan_chunks, scan_chunks_body, 256)
-
-// Exclusive scan over the chunk sums (the 256 threads of the last chunk
-// block, chunks in order); snapshot of the counters and choice of the
-// parallel or sequential insertion path.
-__device__ __forceinline__ void scan_top_body(MapView m) {
-    MapCounters* c = m.ctr;
-    const int M = min(c->n_req, m.newcap);
-    __shared__ int s_a[256], s_e[256];
-    __shared__ int s_base_a, s_base_e;
-    if (threadIdx.x == 0) {
-        s_base_a = 0;
-        s_base_e = 0;
-    }
-    __syncthreads();
-    if (M > 0) {
-        for (int c0 = 0; c0 < m.nchunks; c0 += 256) {
-            const int i = c0 + threadIdx.x;
-            const int a = i < m.nchunks ? __ldcg(&m.chunk_sums[2 * i]) : 0;
-            const int e = i < m.nchunks ? __ldcg(&m.chunk_sums[2 * i + 1]) : 0;
-            s_a[threadIdx.x] = a;
-            s_e[threadIdx.x] = e;
-            __syncthreads();
-            for (int o = 1; o < 256; o <<= 1) {   // inclusive Hillis-Steele scan
-                int ta = threadIdx.x >= o ? s_a[threadIdx.x - o] : 0;
-                int te = threadIdx.x >= o ? s_e[threadIdx.x - o] : 0;
-                __syncthreads();
-                s_a[threadIdx.x] += ta;
-                s_e[threadIdx.x] += te;
-                __syncthreads();
-            }
-            if (i < m.nchunks) {
-                m.chunk_sums[2 * i] = s_base_a + s_a[threadIdx.x] - a;
-                m.chunk_sums[2 * i + 1] = s_base_e + s_e[threadIdx.x] - e;
-            }
-            __syncthreads();
-            if (threadIdx.x == 0) {
-                s_base_a += s_a[255];
-                s_base_e += s_e[255];
-            }
-            __syncthreads();
-        }
-    }
-    if (threadIdx.x == 0) {
-        const int total_x = s_base_e;
-        c->excess_total = total_x;
-        c->snap_M = M;
-        c->snap_hc = c->heap_counter;
-        c->snap_ep = c->entry_ptr;
-        c->snap_na = c->n_alloc;
-        // the parallel path reproduces sequential insertion only while the
-        // free stack and the excess list suffice and no chain holds an empty
-        // entry left by an earlier exhaustion
-        c->fast = (M <= c->heap_counter + 1) && (c->entry_ptr - 1 + total_x <= m.NE) && !c->holes;
-    }
-}
-
-
-// Per chunk: exclusive scan of the per-bucket counts into segment starts and
-// excess starts.
-__device__ __forceinline__ void scan_apply_body(const BlockCtx& ctx, MapView m) {
-    if (m.ctr->snap_M == 0) return;
-    __shared__ int s_c[256], s_x[256];
-    constexpr int per = kScanChunk / 256;
-    const int base = ctx.bx * kScanChunk + threadIdx.x * per;
-    int cnt[per], he[per];
-    int c = 0, xs = 0;
-#pragma unroll
-    for (int q = 0; q < per; ++q) {
-        int b = base + q;
-        cnt[q] = 0;
-        he[q] = 0;
-        if (b < m.NB) {
-            cnt[q] = m.bucket_cnt[b];
-            if (cnt[q]) he[q] = m.entries[b].ptr == -1 ? 1 : 0;
-        }
-        c += cnt[q];
-        xs += cnt[q] - he[q];
-    }
-    s_c[threadIdx.x] = c;
-    s_x[threadIdx.x] = xs;
-    __syncthreads();
-    // Hillis-Steele inclusive scan over 256 thread totals
-    for (int o = 1; o < 256; o <<= 1) {
-        int ac = threadIdx.x >= o ? s_c[threadIdx.x - o] : 0;
-        int ax = threadIdx.x >= o ? s_x[threadIdx.x - o] : 0;
-        __syncthreads();
-        s_c[threadIdx.x] += ac;
-        s_x[threadIdx.x] += ax;
-        __syncthreads();
-    }
-    int run_c = m.chunk_sums[2 * ctx.bx] + s_c[threadIdx.x] - c;
-    int run_x = m.chunk_sums[2 * ctx.bx + 1] + s_x[threadIdx.x] - xs;
-#pragma unroll
-    for (int q = 0; q < per; ++q) {
-        int b = base + q;
-        if (cnt[q]) {
-            m.bucket_start[b] = run_c;
-            m.bucket_x[b] = (run_x << 1) | he[q];
-        }
-        run_c += cnt[q];
-        run_x += cnt[q] - he[q];
-    }
-}
-
-__global__ void __launch_bounds__(256) k_scan_apply(MapView m) {
-    scan_apply_body(own_ctx(), m);
-}
-FB_FUSED_KERNEL(k_scan_apply, scan_apply_body, 256)
-
-__device__ __forceinline__ void alloc_place_body(const BlockCtx& ctx, MapView m) {
-    const int M = m.ctr->snap_M;
-    for (int i = ctx.bx * blockDim.x + threadIdx.x; i < M; i += ctx.gx * blockDim.x) {
-        const NewBlock& nb = m.newblk[i];
-        m.arrival[m.bucket_start[nb.bucket] + nb.j] = i;
-    }
-}
-
-__global__ void __launch_bounds__(256) k_alloc_place(MapView m) {
-    alloc_place_body(own_ctx(), m);
-}
-FB_FUSED_KERNEL(k_alloc_place, alloc_place_body, 256)
-
 __device__ __forceinline__ bool coord_less(const NewBlock& a, const NewBlock& b) {
     if (a.x != b.x) return a.x < b.x;
     if (a.y != b.y) return a.y < b.y;
     return a.z < b.z;
 }
-
-__device__ __forceinline__ void alloc_rank_body(const BlockCtx& ctx, MapView m) {
-    const int M = m.ctr->snap_M;
-    for (int p = ctx.bx * blockDim.x + threadIdx.x; p < M; p += ctx.gx * blockDim.x) {
-        const int i = m.arrival[p];
-        const NewBlock me = m.newblk[i];
-        const int s = m.bucket_start[me.bucket], n = m.bucket_cnt[me.bucket];
-        int r = 0;
-        for (int q = s; q < s + n; ++q)
-            if (coord_less(m.newblk[m.arrival[q]], me)) ++r;
-        m.newblk[i].rank = s + r;
-        m.order[s + r] = i;
-    }
-}
-
-__global__ void __launch_bounds__(256) k_alloc_rank(MapView m) {
-    alloc_rank_body(own_ctx(), m);
-}
-FB_FUSED_KERNEL(k_alloc_rank, alloc_rank_body, 256)
 
 // CreateBlock (DeviceMap.cu:23-62) without lock contention, one block at a
 // time, for the sequential path.  Returns the slot written or -1.
@@ -395,80 +228,146 @@ __device__ int create_block_seq(const MapView& m, int x, int y, int z, int& hc, 
     return -1;
 }
 
-// The insertion (parallel or sequential path), the clearing of the per-bucket
-// counters for the next frame, and the map counters after this frame: every
-// thread reads only the snapshot, so the first thread can write the counters
-// at once.
-__device__ __forceinline__ void alloc_insert_body(const BlockCtx& ctx, MapView m) {
+// Starts of the bins (blocks, blocks with `fills`) in shared memory: an
+// exclusive scan of their counts by 256 threads, each a run of consecutive
+// bins.  Returns all of them.
+__device__ __forceinline__ int2 scan_bins(const MapView& m, int2* start) {
+    constexpr int kEach = kAllocBins / 256;
+    __shared__ int2 s_warp[8];
+    const int t = threadIdx.x;
+    const ulonglong2* src = reinterpret_cast<const ulonglong2*>(m.bins->cnt + t * kEach);
+    int2 v[kEach];
+    int2 sum = make_int2(0, 0);
+#pragma unroll
+    for (int q = 0; q < kEach / 2; ++q) {
+        const ulonglong2 c = src[q];
+        v[2 * q] = make_int2((int)(uint32_t)c.x, (int)(c.x >> 32));
+        v[2 * q + 1] = make_int2((int)(uint32_t)c.y, (int)(c.y >> 32));
+    }
+#pragma unroll
+    for (int q = 0; q < kEach; ++q) {
+        sum.x += v[q].x;
+        sum.y += v[q].y;
+    }
+    int2 run = sum;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int ux = __shfl_up_sync(0xffffffffu, run.x, o), uy = __shfl_up_sync(0xffffffffu, run.y, o);
+        if ((t & 31) >= o) {
+            run.x += ux;
+            run.y += uy;
+        }
+    }
+    if ((t & 31) == 31) s_warp[t >> 5] = run;
+    __syncthreads();
+    run.x -= sum.x;
+    run.y -= sum.y;
+    int2 all = make_int2(0, 0);
+#pragma unroll
+    for (int w = 0; w < 8; ++w) {
+        if (w < (t >> 5)) {
+            run.x += s_warp[w].x;
+            run.y += s_warp[w].y;
+        }
+        all.x += s_warp[w].x;
+        all.y += s_warp[w].y;
+    }
+#pragma unroll
+    for (int q = 0; q < kEach; ++q) {
+        start[t * kEach + q] = run;
+        run.x += v[q].x;
+        run.y += v[q].y;
+    }
+    __syncthreads();
+    return all;
+}
+
+// Where the sequential insertion in canonical order puts a new block, from
+// its bin: rank = its place in the order, among = its place in its bucket,
+// xbefore = blocks of the buckets before that go to the excess list, more =
+// another of its bucket follows.
+struct NewPlace {
+    int rank, among, xbefore;
+    bool more;
+};
+
+__device__ __forceinline__ NewPlace place_of(const MapView& m, const int2* starts, const NewBlock& nb, int M) {
+    const uint32_t bin = nb.bucket >> m.bin_shift;
+    const int2 start = starts[bin];
+    int less = 0, fills = 0, among = 0, same = 0;
+    int q = m.bins->head[bin];
+    for (int guard = 0; q >= 0 && guard < M; ++guard) {
+        const NewBlock o = m.newblk[q];
+        q = o.next;
+        if (o.bucket < nb.bucket) {
+            ++less;
+            fills += o.fills;
+        } else if (o.bucket == nb.bucket) {
+            ++same;
+            among += coord_less(o, nb) ? 1 : 0;
+        }
+    }
+    NewPlace p;
+    p.rank = start.x + less + among;
+    p.among = among;
+    p.xbefore = start.x + less - (start.y + fills);
+    p.more = among + 1 < same;
+    return p;
+}
+
+// The insertion (parallel or sequential path), the clearing of the request
+// set, of the per-bucket counters and, in the block that finishes last, of the
+// bins for the next frame, and the map counters after this frame (written
+// there too, when every block has read them).  zinit: the z-range images and
+// counters of the pass that follows are cleared as well.
+// It is bound by latency (counters, bins, chain, free stack, entry): 9 us at
+// 640x480.  With the request kernel it replaces a counting sort over all
+// buckets in five launches: 38 -> 20 us a frame at 640x480 with 2^20 buckets
+// (19 us of it the two scans of the buckets), 22 -> 13 us at 160x120 with 2^18.
+__device__ __forceinline__ void alloc_insert_body(const BlockCtx& ctx, MapView m, int zinit) {
     MapCounters* c = m.ctr;
-    const int M = c->snap_M;
-    const bool fast = c->fast;
+    const int M = min(c->n_req, m.newcap);
     const int gtid = ctx.bx * blockDim.x + threadIdx.x, gstride = ctx.gx * blockDim.x;
-    if (gtid == 0) {
-        if (M > 0 && fast) {
-            c->heap_counter = c->snap_hc - M;
-            c->entry_ptr = c->snap_ep + c->excess_total;
-            c->n_alloc = c->snap_na + M;
-            c->seq_path = 0;
-        }
-        c->n_new = M;
-        c->n_req = 0;
-        c->n_visible = 0;
-        c->n_tiles = 0;
+    const int hc0 = c->heap_counter, ep0 = c->entry_ptr, na0 = c->n_alloc, holes0 = c->holes;
+    if (zinit) zrange_clear(m, gtid, gstride);
+    __shared__ int2 starts[kAllocBins];
+    bool fast = true;
+    if (ctx.bx * (int)blockDim.x < M) {   // the block has new blocks to insert
+        const int2 all = scan_bins(m, starts);
+        // blocks that do not fill a head slot go to the excess list
+        const int excess = all.x - all.y;
+        if (threadIdx.x == 0) c->excess_total = excess;   // the same from every block
+        // the parallel path reproduces sequential insertion only while the
+        // free stack and the excess list suffice and no chain holds an empty
+        // entry left by an earlier exhaustion
+        fast = M <= hc0 + 1 && ep0 - 1 + excess <= m.NE && !holes0;
     }
-    if (M == 0) return;
-    const int hc0 = c->snap_hc, ep0 = c->snap_ep, na0 = c->snap_na;
-    if (!fast) {
-        if (gtid == 0) {
-            int hc = hc0, ep = ep0, holes = c->holes, na = na0;
-            for (int R = 0; R < M; ++R) {
-                const NewBlock nb = m.newblk[m.order[R]];
-                int slot = create_block_seq(m, nb.x, nb.y, nb.z, hc, ep, holes);
-                if (slot >= 0 && m.entries[slot].ptr != -1) m.alloc_list[na++] = slot;
-            }
-            unsigned err = kErrSequentialInsert;
-            if (hc < -1) err |= kErrHeapExhausted;
-            if (ep - 1 > m.NE) err |= kErrExcessFull;
-            atomicOr(&c->err, err);
-            c->heap_counter = hc;
-            c->entry_ptr = ep;
-            c->holes = holes;
-            c->n_alloc = na;
-            c->seq_path = 1;
-        }
-        for (int R = gtid; R < M; R += gstride) {
-            const NewBlock& nb = m.newblk[m.order[R]];
-            m.reqset[nb.setslot] = 0ull;
-            m.bucket_cnt[nb.bucket] = 0;
-        }
-        return;
-    }
-    for (int R = gtid; R < M; R += gstride) {
-        const int i = m.order[R];
+    for (int i = gtid; i < M; i += gstride) {
         const NewBlock nb = m.newblk[i];
+        const NewPlace p = place_of(m, starts, nb, M);
         const int b = (int)nb.bucket;
-        const int s = m.bucket_start[b], bx = m.bucket_x[b];
-        const int he = bx & 1, xs = bx >> 1;
-        const int r = R - s;
-        // the bucket's blocks are consecutive in canonical order: another
-        // follows this one exactly when the next block has the same bucket
-        const bool more = R + 1 < M && (int)m.newblk[m.order[R + 1]].bucket == b;
+        m.reqset[nb.setslot] = 0ull;
+        m.bucket_cnt[b] = 0;
+        if (!fast) {
+            m.order[p.rank] = i;
+            continue;
+        }
         HEntry e;
         e.x = nb.x;
         e.y = nb.y;
         e.z = nb.z;
         e.pad = 0;
-        e.ptr = m.heap[hc0 - R];
+        e.ptr = m.heap[hc0 - p.rank];
         int slot;
-        if (he && r == 0) {
+        if (nb.he && p.among == 0) {
             slot = b;
-            e.offset = more ? ep0 + xs : 0;
+            e.offset = p.more ? ep0 + p.xbefore : 0;
         } else {
-            const int q = r - he;                 // rank among this bucket's excess blocks
-            const int off = ep0 + xs + q;
+            const int q = p.among - nb.he;        // rank among this bucket's excess blocks
+            const int off = ep0 + p.xbefore + q;
             slot = m.NB + off - 1;
-            e.offset = more ? off + 1 : 0;
-            if (q == 0 && !he) {
+            e.offset = p.more ? off + 1 : 0;
+            if (q == 0 && !nb.he) {
                 // link the tail of the existing chain (CreateBlock's e->offset = offset)
                 int t = b;
                 for (int guard = 0; m.entries[t].offset > 0 && m.entries[t].offset <= m.NE && guard <= m.NE;
@@ -478,54 +377,51 @@ __device__ __forceinline__ void alloc_insert_body(const BlockCtx& ctx, MapView m
             }
         }
         m.entries[slot] = e;
-        m.alloc_list[na0 + R] = slot;
-        m.reqset[nb.setslot] = 0ull;
-        m.bucket_cnt[b] = 0;
+        m.alloc_list[na0 + p.rank] = slot;
     }
+    if (!last_to_finish(&m.bins->ticket, (unsigned)(ctx.gx * ctx.gy))) return;
+    if (M > 0)
+        for (int i = threadIdx.x; i < kAllocBins; i += blockDim.x) {
+            m.bins->cnt[i] = 0;
+            m.bins->head[i] = -1;
+        }
+    if (threadIdx.x != 0) return;
+    const int excess = M > 0 ? __ldcg(&c->excess_total) : 0;
+    if (M > 0 && M <= hc0 + 1 && ep0 - 1 + excess <= m.NE && !holes0) {
+        c->heap_counter = hc0 - M;
+        c->entry_ptr = ep0 + excess;
+        c->n_alloc = na0 + M;
+        c->seq_path = 0;
+    } else if (M > 0) {
+        int hc = hc0, ep = ep0, holes = holes0, na = na0;
+        for (int R = 0; R < M; ++R) {
+            const NewBlock nb = m.newblk[__ldcg(&m.order[R])];
+            int slot = create_block_seq(m, nb.x, nb.y, nb.z, hc, ep, holes);
+            if (slot >= 0 && m.entries[slot].ptr != -1) m.alloc_list[na++] = slot;
+        }
+        unsigned err = kErrSequentialInsert;
+        if (hc < -1) err |= kErrHeapExhausted;
+        if (ep - 1 > m.NE) err |= kErrExcessFull;
+        atomicOr(&c->err, err);
+        c->heap_counter = hc;
+        c->entry_ptr = ep;
+        c->holes = holes;
+        c->n_alloc = na;
+        c->seq_path = 1;
+    }
+    c->n_new = M;
+    c->n_req = 0;
+    c->n_visible = 0;
+    c->n_tiles = 0;
 }
 
-__global__ void __launch_bounds__(256) k_alloc_insert(MapView m) {
-    alloc_insert_body(own_ctx(), m);
+__global__ void __launch_bounds__(256) k_alloc_insert(MapView m, int zinit) {
+    alloc_insert_body(own_ctx(), m, zinit);
 }
 FB_FUSED_KERNEL(k_alloc_insert, alloc_insert_body, 256)
 
 
 // ---------------------------------------------------------------- visibility
-
-// Fusion::CheckVertexVisibility / CheckBlockVisibility (FuseMap.cu:36-78);
-// the eight corners are reached by the reference's sequence of float adds.
-__device__ __forceinline__ bool vertex_visible(f3 p, const DevPose& P, const Intr& k, int W, int H,
-                                               const MapGeom& g) {
-    p = mv(P.Rinv, sub3(p, P.t));
-    if (p.z < 1e-3f) return false;
-    float u = fa(fd(fm(k.fx, p.x), p.z), k.cx), v = fa(fd(fm(k.fy, p.y), p.z), k.cy);
-    return u >= 0 && v >= 0 && u < (float)W && v < (float)H && p.z >= g.depth_min && p.z <= g.depth_max;
-}
-
-__device__ bool block_visible(int bx, int by, int bz, const DevPose& P, const Intr& k, int W, int H,
-                              const MapGeom& g) {
-    const float s = g.block_width;
-    f3 c = mk3(fm((float)bx, s), fm((float)by, s), fm((float)bz, s));
-    if (vertex_visible(c, P, k, W, H, g)) return true;
-    c.z = fa(c.z, s);
-    if (vertex_visible(c, P, k, W, H, g)) return true;
-    c.y = fa(c.y, s);
-    if (vertex_visible(c, P, k, W, H, g)) return true;
-    c.x = fa(c.x, s);
-    if (vertex_visible(c, P, k, W, H, g)) return true;
-    c.z = fs(c.z, s);
-    if (vertex_visible(c, P, k, W, H, g)) return true;
-    c.y = fs(c.y, s);
-    if (vertex_visible(c, P, k, W, H, g)) return true;
-    c.x = fs(c.x, s);
-    c.y = fa(c.y, s);
-    if (vertex_visible(c, P, k, W, H, g)) return true;
-    c.x = fa(c.x, s);
-    c.y = fs(c.y, s);
-    c.z = fa(c.z, s);
-    if (vertex_visible(c, P, k, W, H, g)) return true;
-    return false;
-}
 
 __device__ __forceinline__ void reset_visible_body(const BlockCtx& ctx, MapCounters* c) {
     c->n_visible = 0;
@@ -542,7 +438,6 @@ __device__ __forceinline__ void visibility_body(const BlockCtx& ctx, MapView m, 
     if (skip && *skip) return;
     const DevPose P = *posep;
     const int n = m.ctr->n_alloc;
-    const int lane = threadIdx.x & 31;
     const int nIter = (n + ctx.gx * blockDim.x - 1) / (ctx.gx * blockDim.x);
     for (int it = 0; it < nIter; ++it) {
         const int i = (it * ctx.gx + ctx.bx) * blockDim.x + threadIdx.x;
@@ -554,22 +449,7 @@ __device__ __forceinline__ void visibility_body(const BlockCtx& ctx, MapView m, 
             e = m.entries[slot];
             vis = block_visible(e.x, e.y, e.z, P, k, W, H, m.g);
         }
-        // warp-aggregated append
-        unsigned mask = __ballot_sync(0xffffffffu, vis);
-        if (mask) {
-            int base = 0;
-            if (lane == 0) base = atomicAdd(&m.ctr->n_visible, __popc(mask));
-            base = __shfl_sync(0xffffffffu, base, 0);
-            if (vis) {
-                int o = base + __popc(mask & ((1u << lane) - 1));
-                if (o < m.NS) {
-                    m.visible[o] = slot;
-                    m.vis_blocks[o] = e;   // read by integration and z ranges without a second gather
-                } else {
-                    atomicOr(&m.ctr->err, kErrVisibleFull);
-                }
-            }
-        }
+        append_visible(m, vis, slot, e);
     }
 }
 
@@ -663,8 +543,10 @@ __device__ __forceinline__ bool integrate_voxel(Voxel& vox, int vx, int vy, int 
 }
 
 __device__ __forceinline__ void integrate_body(const BlockCtx& ctx, MapView m, int W, int H, Intr k,
-                                               const DevPose* __restrict__ posep, const int* __restrict__ skip) {
+                                               const DevPose* __restrict__ posep, const int* __restrict__ skip,
+                                               int clear_grid) {
     if (skip && *skip) return;
+    if (clear_grid) grid_clear(m, ctx.bx * blockDim.x + threadIdx.x, ctx.gx * blockDim.x);
     __shared__ float s_div255[256];
     s_div255[threadIdx.x] = fd((float)threadIdx.x, 255.f);   // blockDim.x == 256
     __syncthreads();
@@ -704,8 +586,8 @@ __device__ __forceinline__ void integrate_body(const BlockCtx& ctx, MapView m, i
 }
 
 __global__ void __launch_bounds__(256) k_integrate(MapView m, int W, int H, Intr k, const DevPose* __restrict__ posep,
-                                  const int* __restrict__ skip) {
-    integrate_body(own_ctx(), m, W, H, k, posep, skip);
+                                  const int* __restrict__ skip, int clear_grid) {
+    integrate_body(own_ctx(), m, W, H, k, posep, skip, clear_grid);
 }
 FB_FUSED_KERNEL(k_integrate, integrate_body, 256)
 
@@ -738,8 +620,9 @@ __device__ __forceinline__ float byte_as_magic(uint32_t word, uint32_t sel) {
 
 __device__ __forceinline__ void integrate_compact_body(const BlockCtx& ctx, MapView m, int W, int H, Intr k,
                                                        const DevPose* __restrict__ posep,
-                                                       const int* __restrict__ skip) {
+                                                       const int* __restrict__ skip, int clear_grid) {
     if (skip && *skip) return;
+    if (clear_grid) grid_clear(m, ctx.bx * blockDim.x + threadIdx.x, ctx.gx * blockDim.x);
     const DevPose P = *posep;
     const int n = min(m.ctr->n_visible, m.NS);
     const int t = threadIdx.x, l = t & 31, wq = t >> 5;
@@ -841,8 +724,9 @@ __device__ __forceinline__ void integrate_compact_body(const BlockCtx& ctx, MapV
 }
 
 __global__ void __launch_bounds__(128, 7) k_integrate_compact(MapView m, int W, int H, Intr k,
-                                  const DevPose* __restrict__ posep, const int* __restrict__ skip) {
-    integrate_compact_body(own_ctx(), m, W, H, k, posep, skip);
+                                  const DevPose* __restrict__ posep, const int* __restrict__ skip,
+                                  int clear_grid) {
+    integrate_compact_body(own_ctx(), m, W, H, k, posep, skip, clear_grid);
 }
 FB_FUSED_KERNEL(k_integrate_compact, integrate_compact_body, 128, 7)
 
@@ -928,7 +812,12 @@ __global__ void k_map_reset(MapView m) {
     }
     for (size_t i = tid; i < (size_t)m.NB; i += stride) m.bucket_cnt[i] = 0;
     for (size_t i = tid; i < (size_t)m.reqcap; i += stride) m.reqset[i] = 0ull;
+    for (size_t i = tid; i < (size_t)kAllocBins; i += stride) {
+        m.bins->cnt[i] = 0;
+        m.bins->head[i] = -1;
+    }
     if (tid == 0) {
+        m.bins->ticket = 0;
         MapCounters* c = m.ctr;
         c->heap_counter = m.NS - 1;
         c->entry_ptr = 1;
@@ -941,9 +830,7 @@ __global__ void k_map_reset(MapView m) {
         c->excess_total = 0;
         c->err = 0;
         c->seq_path = 0;
-        c->snap_M = 0;
         c->ray_next = 0;
-        c->scan_ticket = 0;
     }
 }
 
@@ -965,16 +852,11 @@ int launch_map_reset(const MapView& m, cudaStream_t s) { k_map_reset<<<sm_count(
 }
 
 int launch_allocate(const MapView& m, const float* raw, int rp, int W, int H, const Intr& k, const DevPose* pose,
-                     const int* skip, cudaStream_t s) {
+                     const int* skip, cudaStream_t s, bool zinit) {
     dim3 b(32, 8), g((W + 31) / 32, (H + 7) / 8);
     fb_launch(k_alloc_requests, (const void*)k_alloc_requests_fused, g, b, 0, s, m, raw, rp, W, H, k, pose, skip);
-    const int gs = sm_count() * 4;
-    fb_launch(k_scan_chunks, (const void*)k_scan_chunks_fused, m.nchunks, 256, 0, s, m);
-    fb_launch(k_scan_apply, (const void*)k_scan_apply_fused, m.nchunks, 256, 0, s, m);
-    fb_launch(k_alloc_place, (const void*)k_alloc_place_fused, gs, 256, 0, s, m);
-    fb_launch(k_alloc_rank, (const void*)k_alloc_rank_fused, gs, 256, 0, s, m);
-    fb_launch(k_alloc_insert, (const void*)k_alloc_insert_fused, gs, 256, 0, s, m);
-    return 6;
+    fb_launch(k_alloc_insert, (const void*)k_alloc_insert_fused, sm_count() * 2, 256, 0, s, m, zinit ? 1 : 0);
+    return 2;
 }
 
 int launch_visibility(const MapView& m, int W, int H, const Intr& k, const DevPose* pose, const int* skip,
@@ -1007,12 +889,14 @@ int launch_fuse_records(const MapView& m, const float* raw, int rp, const uint8_
 }
 
 int launch_integrate(const MapView& m, int W, int H, const Intr& k, const DevPose* pose, const int* skip,
-                     cudaStream_t s, int ctas_per_sm) {
+                     cudaStream_t s, int ctas_per_sm, bool clear_grid) {
+    const int clear = clear_grid ? 1 : 0;
     const int ctas = sm_count() * (ctas_per_sm ? ctas_per_sm : m.cvox ? 7 : 8);
     if (m.cvox)
-        fb_launch(k_integrate_compact, (const void*)k_integrate_compact_fused, ctas, 128, 0, s, m, W, H, k, pose, skip);
+        fb_launch(k_integrate_compact, (const void*)k_integrate_compact_fused, ctas, 128, 0, s, m, W, H, k, pose,
+                  skip, clear);
     else
-        fb_launch(k_integrate, (const void*)k_integrate_fused, ctas, 256, 0, s, m, W, H, k, pose, skip);
+        fb_launch(k_integrate, (const void*)k_integrate_fused, ctas, 256, 0, s, m, W, H, k, pose, skip, clear);
     return 1;
 }
 

@@ -18,24 +18,13 @@
 
 #include "fb_fused.cuh"
 #include "fb_internal.h"
+#include "fb_view.cuh"
 
 namespace fb {
 
 __device__ __forceinline__ void zrange_init_body(const BlockCtx& ctx, MapView m, const int* __restrict__ skip) {
     if (skip && *skip) return;
-    if (ctx.bx == 0 && threadIdx.x < 3) {
-        m.ctr->bmin[threadIdx.x] = 0x7fffffff;
-        m.ctr->bmax[threadIdx.x] = -0x7fffffff;
-    }
-    if (ctx.bx == 0 && threadIdx.x == 0) {
-        m.ctr->ray_next = 0;
-        m.ctr->n_tiles = 0;   // counted again by each z-range pass
-    }
-    const int n = m.zc * m.zr;
-    for (int i = ctx.bx * blockDim.x + threadIdx.x; i < n; i += ctx.gx * blockDim.x) {
-        m.zmin[i] = 100.f;   // CreateRenderingBlocks uploads 100 (RenderScene.cu:245-251)
-        m.zmax[i] = 0.f;     // and clears zRangeY (RenderScene.cu:244)
-    }
+    zrange_clear(m, ctx.bx * blockDim.x + threadIdx.x, ctx.gx * blockDim.x);
 }
 
 __global__ void __launch_bounds__(256) k_zrange_init(MapView m, const int* __restrict__ skip) {
@@ -68,7 +57,17 @@ __device__ __forceinline__ void order_tiles(const MapView& m, int n) {
     hist[t] = 0;
     hist[t + 256] = 0;
     __syncthreads();
-    for (int i = t; i < n; i += 256) atomicAdd(&hist[cost_bucket(m.rc_cost[i])], 1);
+    // eight costs are loaded before any is counted: one tile at a time, this
+    // block was the z ranges' last to end (9600 tiles: 18 us)
+    constexpr int kAhead = 8;
+    for (int i0 = 0; i0 < n; i0 += 256 * kAhead) {
+        uint32_t c[kAhead];
+#pragma unroll
+        for (int q = 0; q < kAhead; ++q) c[q] = i0 + q * 256 + t < n ? m.rc_cost[i0 + q * 256 + t] : 0;
+#pragma unroll
+        for (int q = 0; q < kAhead; ++q)
+            if (i0 + q * 256 + t < n) atomicAdd(&hist[cost_bucket(c[q])], 1);
+    }
     __syncthreads();
     // bucket starts in descending bucket order: thread t owns buckets 511 - 2t
     // and 510 - 2t (a block-wide exclusive scan of their counts)
@@ -87,16 +86,23 @@ __device__ __forceinline__ void order_tiles(const MapView& m, int n) {
     hist[511 - 2 * t] = excl;   // every thread has read its two counts above
     hist[510 - 2 * t] = excl + h0;
     __syncthreads();
-    for (int i = t; i < n; i += 256) {
-        const int slot = atomicAdd(&hist[cost_bucket(m.rc_cost[i])], 1);
-        m.rc_order[1 + slot] = i;
-        m.rc_cost[i] = 0;
+    for (int i0 = 0; i0 < n; i0 += 256 * kAhead) {
+        uint32_t c[kAhead];
+#pragma unroll
+        for (int q = 0; q < kAhead; ++q) c[q] = i0 + q * 256 + t < n ? m.rc_cost[i0 + q * 256 + t] : 0;
+#pragma unroll
+        for (int q = 0; q < kAhead; ++q) {
+            const int i = i0 + q * 256 + t;
+            if (i < n) {
+                m.rc_order[1 + atomicAdd(&hist[cost_bucket(c[q])], 1)] = i;
+                m.rc_cost[i] = 0;
+            }
+        }
     }
     if (t == 0) m.rc_order[0] = n;
 }
 
-// Projection::projectBlock (RenderScene.cu:54-104) + the first tile's fill
-// (fillBlocks, RenderScene.cu:156-179).  With ord_n > 0 the grid's last block
+// The visible blocks' z ranges and the box they span.  With ord_n > 0 the grid's last block
 // prepares the next raycast's block order instead (order_tiles), beside the
 // projection.
 __device__ __forceinline__ void zrange_body(const BlockCtx& ctx, MapView m, Intr k, const DevPose* __restrict__ posep,
@@ -109,68 +115,27 @@ __device__ __forceinline__ void zrange_body(const BlockCtx& ctx, MapView m, Intr
     const int gx = ord_n > 0 ? ctx.gx - 1 : ctx.gx;
     const DevPose P = *posep;
     const int n = min(m.ctr->n_visible, m.NS);
-    const int zc = m.zc, zr = m.zr;
-    // box of the visible blocks (warp-reduced, then one atomic per warp)
-    {
-        int lo[3] = {0x7fffffff, 0x7fffffff, 0x7fffffff}, hi[3] = {-0x7fffffff, -0x7fffffff, -0x7fffffff};
-        for (int i = ctx.bx * blockDim.x + threadIdx.x; i < n; i += gx * blockDim.x) {
-            const HEntry e = m.vis_blocks[i];
-            lo[0] = min(lo[0], (int)e.x);
-            lo[1] = min(lo[1], (int)e.y);
-            lo[2] = min(lo[2], (int)e.z);
-            hi[0] = max(hi[0], (int)e.x);
-            hi[1] = max(hi[1], (int)e.y);
-            hi[2] = max(hi[2], (int)e.z);
-        }
-#pragma unroll
-        for (int a = 0; a < 3; ++a) {
-            lo[a] = __reduce_min_sync(0xffffffffu, lo[a]);
-            hi[a] = __reduce_max_sync(0xffffffffu, hi[a]);
-        }
-        if ((threadIdx.x & 31) == 0 && lo[0] <= hi[0]) {
-#pragma unroll
-            for (int a = 0; a < 3; ++a) {
-                atomicMin(&m.ctr->bmin[a], lo[a]);
-                atomicMax(&m.ctr->bmax[a], hi[a]);
+    __shared__ ZRects s_r;
+    int lo[3] = {0x7fffffff, 0x7fffffff, 0x7fffffff}, hi[3] = {-0x7fffffff, -0x7fffffff, -0x7fffffff};
+    for (int i0 = ctx.bx * kViewBatch; i0 < n; i0 += gx * kViewBatch) {
+        if (threadIdx.x == 0) s_r.n = 0;
+        __syncthreads();
+        if (threadIdx.x < kViewBatch) {
+            const int i = i0 + threadIdx.x;
+            bool has = false;
+            ZRect r;
+            if (i < n) {
+                const HEntry e = m.vis_blocks[i];
+                grow_box(lo, hi, e);
+                has = project_block(m, e, P, k, r);
             }
+            add_rect(m, s_r, has, r);
         }
+        __syncthreads();
+        fill_rects(m, s_r);
+        __syncthreads();
     }
-    for (int i = ctx.bx * blockDim.x + threadIdx.x; i < n; i += gx * blockDim.x) {
-        const HEntry e = m.vis_blocks[i];
-        int ulx = zc, uly = zr, lrx = -1, lry = -1;
-        float zx = m.g.depth_max, zy = m.g.depth_min;
-        for (int c = 0; c < 8; ++c) {
-            const int tx = e.x + ((c & 1) ? 1 : 0), ty = e.y + ((c & 2) ? 1 : 0), tz = e.z + ((c & 4) ? 1 : 0);
-            f3 p = mk3(fm((float)(tx * 8), m.g.voxel_size), fm((float)(ty * 8), m.g.voxel_size),
-                       fm((float)(tz * 8), m.g.voxel_size));
-            p = mv(P.Rinv, sub3(p, P.t));
-            if ((double)p.z < 2e-1) continue;
-            const float qx = fd(fa(fd(fm(k.fx, p.x), p.z), k.cx), 8.0f);
-            const float qy = fd(fa(fd(fm(k.fy, p.y), p.z), k.cy), 8.0f);
-            // upperLeft / lowerRight are short2 (DeviceMap.h:11-18)
-            if ((float)ulx > floorf(qx)) ulx = (short)(int)floorf(qx);
-            if ((float)lrx < ceilf(qx)) lrx = (short)(int)ceilf(qx);
-            if ((float)uly > floorf(qy)) uly = (short)(int)floorf(qy);
-            if ((float)lry < ceilf(qy)) lry = (short)(int)ceilf(qy);
-            if (zx > p.z) zx = p.z;
-            if (zy < p.z) zy = p.z;
-        }
-        if (ulx < 0) ulx = 0;
-        if (uly < 0) uly = 0;
-        if (lrx >= zc) lrx = zc - 1;
-        if (lry >= zr) lry = zr - 1;
-        if (ulx > lrx || uly > lry) continue;
-        if (zx < m.g.depth_min) zx = m.g.depth_min;
-        if (zy < m.g.depth_min) continue;
-        atomicAdd(&m.ctr->n_tiles, 1);
-        const int ex = min(ulx + 15, lrx), ey = min(uly + 15, lry);
-        const int bzx = __float_as_int(zx), bzy = __float_as_int(zy);
-        for (int y = uly; y <= ey; ++y)
-            for (int x = ulx; x <= ex; ++x) {
-                atomicMin((int*)&m.zmin[y * zc + x], bzx);
-                atomicMax((int*)&m.zmax[y * zc + x], bzy);
-            }
-    }
+    widen_box(m, lo, hi);
 }
 
 __global__ void __launch_bounds__(256) k_zrange(MapView m, Intr k, const DevPose* __restrict__ posep,
@@ -178,6 +143,58 @@ __global__ void __launch_bounds__(256) k_zrange(MapView m, Intr k, const DevPose
     zrange_body(own_ctx(), m, k, posep, skip, ord_n);
 }
 FB_FUSED_KERNEL(k_zrange, zrange_body, 256)
+
+// Visibility (k_visibility) and z ranges (k_zrange) of a fused frame in one
+// pass over the allocated blocks: a block found visible is appended, widens
+// the box and is projected by the thread that found it.  The z-range images
+// and counters were cleared with the allocation.  With the clearing of the
+// index in the integration, this takes the place of four launches: 17 -> 8 us
+// at 640x480, 28 -> 12 at 1280x960, 14 -> 7.5 at 160x120.
+__device__ __forceinline__ void view_body(const BlockCtx& ctx, MapView m, int W, int H, Intr k,
+                                          const DevPose* __restrict__ posep, const int* __restrict__ skip, int ord_n) {
+    if (skip && *skip) return;
+    if (ord_n > 0 && ctx.bx == ctx.gx - 1) {
+        order_tiles(m, ord_n);
+        return;
+    }
+    const int gx = ord_n > 0 ? ctx.gx - 1 : ctx.gx;
+    const DevPose P = *posep;
+    const int n = m.ctr->n_alloc;
+    __shared__ ZRects s_r;
+    int lo[3] = {0x7fffffff, 0x7fffffff, 0x7fffffff}, hi[3] = {-0x7fffffff, -0x7fffffff, -0x7fffffff};
+    for (int i0 = ctx.bx * kViewBatch; i0 < n; i0 += gx * kViewBatch) {
+        if (threadIdx.x == 0) s_r.n = 0;
+        __syncthreads();
+        if (threadIdx.x < kViewBatch) {
+            const int i = i0 + threadIdx.x;
+            bool vis = false, has = false;
+            int slot = -1;
+            HEntry e;
+            ZRect r;
+            if (i < n) {
+                slot = m.alloc_list[i];
+                e = m.entries[slot];
+                vis = block_visible(e.x, e.y, e.z, P, k, W, H, m.g);
+            }
+            append_visible(m, vis, slot, e);
+            if (vis) {
+                grow_box(lo, hi, e);
+                has = project_block(m, e, P, k, r);
+            }
+            add_rect(m, s_r, has, r);
+        }
+        __syncthreads();
+        fill_rects(m, s_r);
+        __syncthreads();
+    }
+    widen_box(m, lo, hi);
+}
+
+__global__ void __launch_bounds__(256) k_view(MapView m, int W, int H, Intr k, const DevPose* __restrict__ posep,
+                                              const int* __restrict__ skip, int ord_n) {
+    view_body(own_ctx(), m, W, H, k, posep, skip, ord_n);
+}
+FB_FUSED_KERNEL(k_view, view_body, 256)
 
 // Dense block index for the raycast: every allocated block inside the box of
 // this frame's visible blocks (one block of margin) gets its pool index in
@@ -187,40 +204,9 @@ FB_FUSED_KERNEL(k_zrange, zrange_body, 256)
 // lookup returns the same block: a ray's samples turn one indexed load instead
 // of a bucket probe and chain walk, which also keeps a warp's lanes together.
 //
-// The box from the z-range pass's bounds (every block of the clearing kernel
-// derives it; block 0 publishes it for the fill and the raycast).
-struct GridBox {
-    int o[3], n[3];
-    bool on;
-};
-
-__device__ __forceinline__ GridBox grid_box(const MapView& m) {
-    const MapCounters* c = m.ctr;
-    GridBox b;
-    long long vol = 1;
-    for (int a = 0; a < 3; ++a) {
-        b.o[a] = c->bmin[a] - 1;
-        b.n[a] = c->bmax[a] - c->bmin[a] + 3;
-        if (b.n[a] < 1) b.n[a] = 0;
-        vol *= b.n[a];
-    }
-    b.on = c->bmin[0] <= c->bmax[0] && vol > 0 && vol <= m.grid_cap;
-    return b;
-}
-
 __device__ __forceinline__ void grid_clear_body(const BlockCtx& ctx, MapView m, const int* __restrict__ skip) {
     if (skip && *skip) return;
-    const GridBox gb = grid_box(m);
-    if (ctx.bx == 0 && threadIdx.x < 3) {
-        m.ctr->g_o[threadIdx.x] = gb.o[threadIdx.x];
-        m.ctr->g_n[threadIdx.x] = gb.on ? gb.n[threadIdx.x] : 0;
-        if (threadIdx.x == 0) m.ctr->g_on = gb.on ? 1 : 0;
-    }
-    if (!gb.on) return;
-    const int vol = gb.n[0] * gb.n[1] * gb.n[2];
-    int4* g4 = (int4*)m.grid;
-    const int4 none = make_int4(-1, -1, -1, -1);
-    for (int i = ctx.bx * blockDim.x + threadIdx.x; i < (vol + 3) / 4; i += ctx.gx * blockDim.x) g4[i] = none;
+    grid_clear(m, ctx.bx * blockDim.x + threadIdx.x, ctx.gx * blockDim.x);
 }
 
 __global__ void __launch_bounds__(256) k_grid_clear(MapView m, const int* __restrict__ skip) {
@@ -705,8 +691,20 @@ int launch_zrange(const MapView& m, const Intr& k, const DevPose* pose, const in
     fb_launch(k_zrange, (const void*)k_zrange_fused, sm_count_rc() * 2 + (ord_n > 0 ? 1 : 0), 256, 0, s, m, k, pose,
               skip, ord_n);
     fb_launch(k_grid_clear, (const void*)k_grid_clear_fused, sm_count_rc() * 4, 256, 0, s, m, skip);
+    return 3 + launch_grid_fill(m, skip, s);
+}
+
+int launch_view(const MapView& m, int W, int H, const Intr& k, const DevPose* pose, const int* skip, cudaStream_t s,
+                int rc_tiles) {
+    const int ord_n = m.rc_order ? rc_tiles : 0;
+    fb_launch(k_view, (const void*)k_view_fused, sm_count_rc() * 4 + (ord_n > 0 ? 1 : 0), 256, 0, s, m, W, H, k, pose,
+              skip, ord_n);
+    return 1;
+}
+
+int launch_grid_fill(const MapView& m, const int* skip, cudaStream_t s) {
     fb_launch(k_grid_fill, (const void*)k_grid_fill_fused, sm_count_rc() * 4, 256, 0, s, m, skip);
-    return 4;
+    return 1;
 }
 
 int launch_raycast(const MapView& m, float4* vmap, float4* nmap, int p, int W, int H, const Intr& k,

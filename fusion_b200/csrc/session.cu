@@ -302,7 +302,8 @@ bool carve_session(fb_session* s, const fb_config* cfg) {
         // all of them and the exhaustion is handled by the exact sequential path
         m.newcap = m.NS > kMinNewBlocks ? m.NS : kMinNewBlocks;
         m.reqcap = (int)next_pow2((size_t)2 * m.newcap);
-        m.nchunks = (m.NB + kScanChunk - 1) / kScanChunk;
+        m.bin_shift = 0;
+        while (((m.NB - 1) >> m.bin_shift) >= kAllocBins) ++m.bin_shift;
         // dense raycast index: 16 cells per pool block, 64 K to 4 M cells
         {
             const size_t cap = (size_t)16 * m.NS;
@@ -318,9 +319,8 @@ bool carve_session(fb_session* s, const fb_config* cfg) {
              dalloc(s, &m.ctr, 1) && dalloc(s, &m.alloc_list, m.NS) &&
              dalloc(s, &m.visible, m.NS) && dalloc(s, &m.vis_blocks, m.NS) && dalloc(s, &m.reqset, m.reqcap) &&
              dalloc(s, &m.newblk, m.newcap) &&
-             dalloc(s, &m.order, m.newcap) && dalloc(s, &m.arrival, m.newcap) &&
-             dalloc(s, &m.bucket_cnt, m.NB) && dalloc(s, &m.bucket_start, m.NB) && dalloc(s, &m.bucket_x, m.NB) &&
-             dalloc(s, &m.chunk_sums, 2 * (size_t)m.nchunks) && dalloc(s, &m.zmin, (size_t)m.zc * m.zr) &&
+             dalloc(s, &m.order, m.newcap) && dalloc(s, &m.bucket_cnt, m.NB) && dalloc(s, &m.bins, 1) &&
+             dalloc(s, &m.zmin, (size_t)m.zc * m.zr) &&
              dalloc(s, &m.grid, (size_t)m.grid_cap) &&
              dalloc(s, &m.zmax, (size_t)m.zc * m.zr) && dalloc(s, &m.frec, (size_t)64 * m.zc * m.zr) &&
              dalloc(s, &m.fcol, (size_t)64 * m.zc * m.zr) && dalloc(s, &m.rc_cost, (size_t)m.rc_cap) &&
@@ -460,18 +460,21 @@ int issue_frame(fb_session* s, bool track, bool fuse, bool render, bool init, un
         *ran |= 1u << 2;
     }
     const DevPose* pose = &s->st->cur;
+    const int tiles = raycast_tiles(s->W[0], s->H[0], s->rc_bx, s->rc_by);
     mark(3);
     if (fuse) {
         // Mapping::FuseColor(LastFrame) after the swap (Mapping.cc:76-90):
         // raw depth, colour and level-0 normals of the frame just tracked
         launch_slot(kSlotAllocate);
-        n += launch_allocate(s->map, N.raw, s->W[0], s->W[0], s->H[0], s->K[0], pose, skip, st);
+        n += launch_allocate(s->map, N.raw, s->W[0], s->W[0], s->H[0], s->K[0], pose, skip, st, render);
         mark(4);
         launch_slot(kSlotVisibility);
-        n += launch_visibility(s->map, s->W[0], s->H[0], s->K[0], pose, skip, st, true);
+        // a rendered frame's z ranges and dense block index are made on the way
+        n += render ? launch_view(s->map, s->W[0], s->H[0], s->K[0], pose, skip, st, tiles)
+                    : launch_visibility(s->map, s->W[0], s->H[0], s->K[0], pose, skip, st, true);
         mark(5);
         launch_slot(kSlotIntegrate);
-        n += launch_integrate(s->map, s->W[0], s->H[0], s->K[0], pose, skip, st, s->integ_cps);
+        n += launch_integrate(s->map, s->W[0], s->H[0], s->K[0], pose, skip, st, s->integ_cps, render);
         *ran |= 7u << 3;
     } else {
         mark(4);
@@ -487,7 +490,7 @@ int issue_frame(fb_session* s, bool track, bool fuse, bool render, bool init, un
         }
         // Mapping::RayTrace (Mapping.cc:92-109) into the frame's level-0 maps
         launch_slot(kSlotZRange);
-        n += launch_zrange(s->map, s->K[0], pose, skip, st, raycast_tiles(s->W[0], s->H[0], s->rc_bx, s->rc_by));
+        n += fuse ? launch_grid_fill(s->map, skip, st) : launch_zrange(s->map, s->K[0], pose, skip, st, tiles);
         mark(7);
         launch_slot(kSlotRaycast);
         n += launch_raycast(s->map, N.vmap[0], N.nmap[0], s->W[0], s->W[0], s->H[0], s->K[0], pose, skip, st,

@@ -256,7 +256,7 @@ int fb_fuse_map_color(fb_session* s, const fb_image* depth, const fb_image* rgb,
     k_set_pose<<<1, 1, 0, st>>>(s->scratch_pose, pose_from(Rview, RviewInv, tview));
     const Intr k = intr_from(K);
     launch_allocate(s->map, (const float*)depth->data, (int)(depth->pitch / 4), W, H, k, s->scratch_pose, nullptr, st);
-    launch_visibility(s->map, W, H, k, s->scratch_pose, nullptr, st);
+    launch_visibility(s->map, W, H, k, s->scratch_pose, nullptr, st, true);
     launch_fuse_records(s->map, (const float*)depth->data, (int)(depth->pitch / 4), (const uint8_t*)rgb->data,
                         (int)rgb->pitch, (const float4*)nmap->data, (int)(nmap->pitch / 16), W, H, st);
     launch_integrate(s->map, W, H, k, s->scratch_pose, nullptr, st);

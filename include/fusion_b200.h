@@ -150,7 +150,9 @@ FB_API int fb_stage_frame(fb_session* s, const uint16_t* depth, size_t depth_pit
  * accumulates device milliseconds per stage: 0 resize of the last frame's
  * maps (its kernels run inside the pyramid's launches, so its own time is
  * only the events'), 1 pyramid and resize, 2 tracking, 3 block allocation,
- * 4 visibility, 5 integration, 6 z ranges, 7 raycast.  Switching it on
+ * 4 visibility (of a fused frame: and z ranges, which one kernel makes), 5
+ * integration (and the clearing of the raycast's block index), 6 z ranges (of
+ * a fused frame: the filling of that index), 7 raycast.  Switching it on
  * resets the sums. */
 FB_API int fb_session_set_profiling(fb_session* s, int on);
 FB_API int fb_session_stage_times(fb_session* s, double* ms, uint64_t* calls, int n);
