@@ -39,17 +39,28 @@ __device__ __forceinline__ void level0_body(const BlockCtx& ctx, const uint16_t*
     if (!filt) return;
     const int tx = min(x + 3, W - 1), ty = min(y + 3, H - 1);
     float sum1 = 0.f, sum2 = 0.f;
-    for (int cy = max(y - 2, 0); cy < ty; ++cy) {
-        const uint16_t* row = depth + (size_t)cy * dpitch;
-        for (int cx = max(x - 2, 0); cx < tx; ++cx) {
-            float val = fm((float)row[cx], inv);
-            float space2 = (float)((x - cx) * (x - cx) + (y - cy) * (y - cy));
-            float dz = fs(center, val);
-            float color2 = fm(dz, dz);
-            float weight = expf(-fa(fm(space2, sigSpace), fm(color2, sigRange)));
-            sum1 = fa(sum1, fm(val, weight));
-            sum2 = fa(sum2, weight);
-        }
+    auto tap = [&](uint16_t d, int dx, int dy) {
+        const float val = fm((float)d, inv);
+        const float space = fm((float)(dx * dx + dy * dy), sigSpace);
+        const float dz = fs(center, val);
+        // -(space + 2 dz^2): doubling is exact, so one FMA rounds it as the
+        // sum; the centre tap's argument is -0, its weight 1
+        const float weight = dx == 0 && dy == 0 ? 1.0f : expf(__fmaf_rn(fm(dz, dz), -sigRange, -space));
+        sum1 = fa(sum1, fm(val, weight));
+        sum2 = fa(sum2, weight);
+    };
+    if (x >= 2 && y >= 2 && x + 3 < W && y + 3 < H) {
+        // the whole window: its 25 loads together, constant distances
+        // (1283x721: 30 us with clipped loops, 23 so; bound by instruction
+        // issue, 24 exponentials per pixel)
+        uint16_t d[25];
+#pragma unroll
+        for (int q = 0; q < 25; ++q) d[q] = depth[(size_t)(y - 2 + q / 5) * dpitch + x - 2 + q % 5];
+#pragma unroll
+        for (int q = 0; q < 25; ++q) tap(d[q], 2 - q % 5, 2 - q / 5);
+    } else {
+        for (int cy = max(y - 2, 0); cy < ty; ++cy)
+            for (int cx = max(x - 2, 0); cx < tx; ++cx) tap(depth[(size_t)cy * dpitch + cx], x - cx, y - cy);
     }
     float fin = fd(sum1, sum2);
     filt[(size_t)y * fpitch + x] = fin < cutoff ? fin : qnan();
@@ -69,6 +80,32 @@ FB_FUSED_KERNEL(k_level0, level0_body, 256)
 template <class T>
 __device__ __forceinline__ T pyr_pixel(const T* __restrict__ src, int spitch, int SW, int SH, int x, int y) {
     const int tx = min(2 * x + 3, SW - 1), ty = min(2 * y + 3, SH - 1);
+    if (x >= 1 && y >= 1 && 2 * x + 3 < SW && 2 * y + 3 < SH) {
+        // the whole window: its 25 loads together, constant weights
+        constexpr int g[5] = {1, 4, 6, 4, 1};
+        T v[25];
+#pragma unroll
+        for (int q = 0; q < 25; ++q) v[q] = src[(size_t)(2 * y - 2 + q / 5) * spitch + 2 * x - 2 + q % 5];
+        if constexpr (sizeof(T) == 1) {
+            // sums below 2^16: integers give the float sum, and its quotient
+            // by 256 truncates to the high byte
+            int sum = 0;
+#pragma unroll
+            for (int q = 0; q < 25; ++q) sum += (int)v[q] * (g[q / 5] * g[q % 5]);
+            return (T)(sum >> 8);
+        } else {
+            float sum = 0.f;
+            int count = 0;
+#pragma unroll
+            for (int q = 0; q < 25; ++q) {
+                const int k = g[q / 5] * g[q % 5];
+                const bool ok = !isnan(v[q]);
+                sum = ok ? fa(sum, fm(v[q], (float)k)) : sum;
+                count += ok ? k : 0;
+            }
+            return (T)fd(sum, (float)count);
+        }
+    }
     float sum = 0.f;
     int count = 0;
     for (int cy = max(0, 2 * y - 2); cy < ty; ++cy)
@@ -169,33 +206,40 @@ __device__ __forceinline__ void maps_body(const BlockCtx& ctx, const float* __re
     }
     if (dxo) {
         // kernel index runs 8 -> 0 over the clipped window; integer sums are
-        // exact, as the reference's float sums of small integers are
-        const int sx[9] = {1, 0, -1, 2, 0, -2, 1, 0, -1};
-        const int sy[9] = {1, 2, 1, 0, 0, 0, -1, -2, -1};
-        int gx = 0, gy = 0, idx = 8;
-        for (int j = max(y - 1, 0); j <= min(y + 1, H - 1); ++j)
-            for (int i = max(x - 1, 0); i <= min(x + 1, W - 1); ++i) {
-                int v = gray[(size_t)j * gp + i];
-                gx += v * sx[idx];
-                gy += v * sy[idx];
-                --idx;
-            }
+        // exact, as the reference's float sums of small integers are.  rgbok:
+        // the pose-independent part of RGBReduction::FindCorresp
+        // (Tracking/Reduction.cu:413-425): 5-pixel border, gray > 0 over the
+        // window y-2..y+1, x-2..x+1, nonzero gradient
+        int gx = 0, gy = 0;
+        bool ok = x >= 5 && x < W - 5 && y >= 5 && y < H - 5;
+        if (x >= 2 && y >= 2 && x + 1 < W && y + 1 < H) {
+            // both windows inside the image: one set of 16 loads
+            int v[4][4];
+#pragma unroll
+            for (int j = 0; j < 4; ++j)
+#pragma unroll
+                for (int i = 0; i < 4; ++i) v[j][i] = gray[(size_t)(y - 2 + j) * gp + x - 2 + i];
+            gx = (v[1][3] + 2 * v[2][3] + v[3][3]) - (v[1][1] + 2 * v[2][1] + v[3][1]);
+            gy = (v[3][1] + 2 * v[3][2] + v[3][3]) - (v[1][1] + 2 * v[1][2] + v[1][3]);
+#pragma unroll
+            for (int j = 0; j < 4; ++j)
+#pragma unroll
+                for (int i = 0; i < 4; ++i) ok = ok && v[j][i] != 0;
+        } else {
+            const int sx[9] = {1, 0, -1, 2, 0, -2, 1, 0, -1};
+            const int sy[9] = {1, 2, 1, 0, 0, 0, -1, -2, -1};
+            int idx = 8;
+            for (int j = max(y - 1, 0); j <= min(y + 1, H - 1); ++j)
+                for (int i = max(x - 1, 0); i <= min(x + 1, W - 1); ++i) {
+                    int v = gray[(size_t)j * gp + i];
+                    gx += v * sx[idx];
+                    gy += v * sy[idx];
+                    --idx;
+                }
+        }
         dxo[(size_t)y * sp + x] = (int16_t)gx;
         dyo[(size_t)y * sp + x] = (int16_t)gy;
-        if (rgbok) {
-            // the pose-independent part of RGBReduction::FindCorresp
-            // (Tracking/Reduction.cu:413-425): 5-pixel border, gray > 0 over
-            // the window y-2..y+1, x-2..x+1, nonzero gradient
-            bool ok = x >= 5 && x < W - 5 && y >= 5 && y < H - 5 && ((int16_t)gx != 0 || (int16_t)gy != 0);
-            if (ok)
-                for (int u = y - 2; u < y + 2 && ok; ++u)
-                    for (int v = x - 2; v < x + 2; ++v)
-                        if (gray[(size_t)u * gp + v] == 0) {
-                            ok = false;
-                            break;
-                        }
-            rgbok[(size_t)y * sp + x] = ok ? 1 : 0;
-        }
+        if (rgbok) rgbok[(size_t)y * sp + x] = ok && ((int16_t)gx != 0 || (int16_t)gy != 0) ? 1 : 0;
     }
 }
 
