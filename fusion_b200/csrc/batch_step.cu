@@ -144,12 +144,10 @@ int build_fused(fb_batch* b, fb_session* const* ss, int n, const FramePlan* plan
         launch_recorder() = &r;
         unsigned ran = 0;
         const int issued = issue_frame(s, plans[i].track, plans[i].fuse, plans[i].render, plans[i].init, &ran);
-        launch_slot(kSlotOut);
-        launch_result_out(s, b->origin);
         launch_recorder() = nullptr;
         s->profile = prof;
         // every kernel of the frame went through the recorder, in slot order
-        if ((int)r.recs.size() != issued + 1) {
+        if ((int)r.recs.size() != issued) {
             fb_set_error_text("fused batch step: a frame kernel was not recorded");
             return FB_ECUDA;
         }
@@ -334,7 +332,8 @@ int issue_step(fb_batch* b, fb_session* const* ss, int n, const FramePlan* plans
             *kernels += issue_frame(s, plans[i].track, plans[i].fuse, plans[i].render, plans[i].init, &ran);
             s->stream = keep;
         }
-        FB_CUDA(cudaMemcpyAsync(s->h_out, s->d_out, sizeof(FrameOut), cudaMemcpyDeviceToHost, st));
+        const int rc = fetch_result(s, st);
+        if (rc) return rc;
     }
     for (int k = 0; k < used; ++k) {
         FB_CUDA(cudaEventRecord(b->done[k], b->slots[k]));

@@ -162,7 +162,6 @@ enum FusedStage : int {
     kSlotZRange,
     kSlotRaycast,
     kSlotCommit,
-    kSlotOut,
 };
 
 // Tags the launches that follow (no-op without a recorder).

@@ -77,6 +77,26 @@ struct TrackSync {
     TrackSlot pose[kPoseCopies][8];              // 21 floats of a DevPose, then {failed, -, -}
 };
 
+// Exchange numbers a frame takes (launch_track_begin's step).
+inline unsigned track_exchanges(const int iters[3]) { return (unsigned)(iters[0] + iters[1] + iters[2]) + 1u; }
+
+// Frame start: the next pose starts from the last pose (TrackFrame's
+// bootstrap fallback, Tracking.cc:156-159) and delta is the identity.
+// One thread.
+__device__ __forceinline__ void track_begin(TrackState* st, TrackSync* sync, unsigned step) {
+    sync->epoch += step;   // the frame's exchanges (k_track_loop) are numbered from here
+    for (int i = 0; i < 16; ++i) {
+        st->pose[i] = st->last_pose[i];
+        st->init_pose[i] = st->last_pose[i];
+        st->delta[i] = (i % 5 == 0) ? 1.0 : 0.0;
+    }
+    st->cur = make_dev_pose_d(st->pose);
+    st->last = make_dev_pose_d(st->last_pose);
+    st->failed = 0;
+    st->icp_error = st->rgb_error = qnan();
+    st->icp_count = st->rgb_count = 0;
+}
+
 int track_grid(int n);
 int track_cluster_grid(int n);   // the passes' logical grid: track_grid in whole groups
 int launch_track_begin(TrackState* st, TrackSync* sync, const int iters[3], cudaStream_t s);
@@ -183,6 +203,10 @@ struct PreLaunch {
     PyrArgs py;
     MapsArgs mp;
     int gx[4], gy[4];
+    // one more block sets the tracker's start (launch_track_begin); null: none
+    TrackState* begin;
+    TrackSync* sync;
+    unsigned step;
 };
 // Role setters (same arguments as the launchers above) and the launch.
 void pre_level0(PreLaunch& P, const uint16_t* depth, int dpitch, const uint8_t* rgb, int rgbpitch, int W, int H,
@@ -195,6 +219,7 @@ void pre_pyrdown(PreLaunch& P, const float* sd, int sdp, const uint8_t* sg, int 
 void pre_maps(PreLaunch& P, const float* depth, int dp, const uint8_t* gray, int gp, int W, int H, const Intr& k,
               float cutoff, float4* vmap, int vp, float4* nmap, int np, int16_t* dx, int16_t* dy, int sp,
               uint8_t* rgbok, const FuseRecDst* fr);
+void pre_track_begin(PreLaunch& P, TrackState* st, TrackSync* sync, const int iters[3]);
 int launch_pre(const PreLaunch& P, cudaStream_t st);
 
 // ----------------------------------------------------------------------- map

@@ -360,7 +360,8 @@ int grab_with_keys(fb_session* s, fb_frame_result* out) {
         rc = check_launch();
     }
     if (rc) return rc;
-    FB_CUDA(cudaMemcpyAsync(s->h_out, s->d_out, sizeof(FrameOut), cudaMemcpyDeviceToHost, s->stream));
+    rc = fetch_result(s, s->stream);
+    if (rc) return rc;
     FB_CUDA(cudaStreamSynchronize(s->stream));
     if (relocalised) {
         // case -1 of Tracker::Track: lastState = 0, SwapFrame

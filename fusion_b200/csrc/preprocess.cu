@@ -320,6 +320,7 @@ __device__ __forceinline__ void pre_body(const BlockCtx& ctx, const PreLaunch& P
         }
         b -= n;
     }
+    if (P.begin && threadIdx.x == 0 && threadIdx.y == 0) track_begin(P.begin, P.sync, P.step);   // the block beyond the roles
 }
 
 __global__ void __launch_bounds__(256) k_pre(PreLaunch P) { pre_body(own_ctx(), P); }
@@ -362,8 +363,14 @@ void pre_maps(PreLaunch& P, const float* depth, int dp, const uint8_t* gray, int
     set_role(P, 3, W, H);
 }
 
+void pre_track_begin(PreLaunch& P, TrackState* st, TrackSync* sync, const int iters[3]) {
+    P.begin = st;
+    P.sync = sync;
+    P.step = track_exchanges(iters);
+}
+
 int launch_pre(const PreLaunch& P, cudaStream_t st) {
-    int blocks = 0;
+    int blocks = P.begin ? 1 : 0;
     for (int r = 0; r < 4; ++r) blocks += P.gx[r] * P.gy[r];
     if (blocks == 0) return 0;
     fb_launch(k_pre, (const void*)k_pre_fused, blocks, dim3(32, 8), 0, st, P);

@@ -65,43 +65,40 @@ __device__ __forceinline__ void init_poses_body(const BlockCtx&, TrackState* st)
 __global__ void k_init_poses(TrackState* st) { init_poses_body(own_ctx(), st); }
 FB_FUSED_KERNEL(k_init_poses, init_poses_body, 32)
 
-// After the frame: a tracked frame becomes the last frame (SwapFrame).
+// After the frame: a tracked frame becomes the last frame (SwapFrame), and the
+// frame's result goes to `out` -- the session's pinned host memory where the
+// device can write it (a copy of the 184 bytes after the kernel took 3 us and
+// a gap of 6), else device memory.  64 threads.
 __device__ __forceinline__ void commit_body(const BlockCtx&, TrackState* st, MapCounters* c, FrameOut* out,
                                             int tracked_path) {
-    if (tracked_path && !st->failed) {
-        for (int i = 0; i < 16; ++i) st->last_pose[i] = st->pose[i];
-        st->last = st->cur;
+    const int t = threadIdx.x;
+    if (t < 16) {
+        const double v = st->pose[t];
+        out->pose[t] = v;
+        if (tracked_path && !st->failed) st->last_pose[t] = v;
+    } else if (t < 16 + (int)(sizeof(DevPose) / 4)) {
+        if (tracked_path && !st->failed) ((float*)&st->last)[t - 16] = ((const float*)&st->cur)[t - 16];
+    } else if (t == 40) {
+        out->failed = st->failed;
+        out->icp_error = st->icp_error;
+        out->icp_count = st->icp_count;
+        out->rgb_error = st->rgb_error;
+        out->rgb_count = st->rgb_count;
+    } else if (t == 41) {
+        out->n_alloc = c->n_alloc;
+        out->n_visible = c->n_visible;
+        out->n_new = c->n_new;
+        out->n_tiles = c->n_tiles;
+        out->err = c->err;
+        out->heap_counter = c->heap_counter;
+        out->entry_ptr = c->entry_ptr;
+        out->seq_path = c->seq_path;
     }
-    for (int i = 0; i < 16; ++i) out->pose[i] = st->pose[i];
-    out->failed = st->failed;
-    out->icp_error = st->icp_error;
-    out->icp_count = st->icp_count;
-    out->rgb_error = st->rgb_error;
-    out->rgb_count = st->rgb_count;
-    out->n_alloc = c->n_alloc;
-    out->n_visible = c->n_visible;
-    out->n_new = c->n_new;
-    out->n_tiles = c->n_tiles;
-    out->err = c->err;
-    out->heap_counter = c->heap_counter;
-    out->entry_ptr = c->entry_ptr;
-    out->seq_path = c->seq_path;
 }
 __global__ void k_commit(TrackState* st, MapCounters* c, FrameOut* out, int tracked_path) {
     commit_body(own_ctx(), st, c, out, tracked_path);
 }
-FB_FUSED_KERNEL(k_commit, commit_body, 32)
-
-// The frame result into the caller's pinned host memory (device-accessible
-// through unified addressing): the fused batch step reads every session's
-// result this way instead of one copy per session.
-__device__ __forceinline__ void result_out_body(const BlockCtx&, const FrameOut* d, FrameOut* h) {
-    static_assert(sizeof(FrameOut) % 4 == 0, "FrameOut is copied in words");
-    const int n = (int)(sizeof(FrameOut) / 4);
-    for (int i = threadIdx.x; i < n; i += blockDim.x) ((int*)h)[i] = ((const int*)d)[i];
-}
-__global__ void k_result_out(const FrameOut* d, FrameOut* h) { result_out_body(own_ctx(), d, h); }
-FB_FUSED_KERNEL(k_result_out, result_out_body, 64)
+FB_FUSED_KERNEL(k_commit, commit_body, 64)
 
 
 // Export of the hash table in the reference's field order, ptr as voxel index.
@@ -369,6 +366,8 @@ int issue_frame(fb_session* s, bool track, bool fuse, bool render, bool init, un
     const fb_config& c = s->cfg;
     int n = 0;
     *ran = 0;
+    // a whole frame's preprocessing also sets the tracker's start
+    const bool begin = part == 0 && track && !init;
     auto mark = [&](int k) {
         if (s->profile) cudaEventRecord(s->ev[k], st);
     };
@@ -402,6 +401,7 @@ int issue_frame(fb_session* s, bool track, bool fuse, bool render, bool init, un
             pre_level0(P, N.depth_in, s->W[0], N.rgb, 3 * s->W[0], s->W[0], s->H[0], c.depth_scale, c.depth_cutoff,
                        N.raw, s->W[0], N.depth[0], s->W[0], N.gray[0], s->W[0]);
             resize(P, 1);
+            if (begin) pre_track_begin(P, s->st, s->track_sync, c.iters);
             n += launch_pre(P, st);
         }
         {
@@ -434,7 +434,7 @@ int issue_frame(fb_session* s, bool track, bool fuse, bool render, bool init, un
     } else if (track) {
         // Tracker::ComputeSE3 (Tracking.cc:296-409)
         static const int min_count[3] = {2000, 1000, 100};   // MIN_ICP_COUNT, Tracking.h:102
-        n += launch_track_begin(s->st, s->track_sync, c.iters, st);
+        if (!begin) n += launch_track_begin(s->st, s->track_sync, c.iters, st);
         if (start) {
             Pose16 T;
             std::memcpy(T.m, start, sizeof T.m);
@@ -570,12 +570,14 @@ LaunchRecorder*& launch_recorder() {
     return r;
 }
 
-void launch_result_out(fb_session* s, cudaStream_t st) {
-    fb_launch(k_result_out, (const void*)k_result_out_fused, 1, 64, 0, st, s->d_out, s->h_out_dev);
+void launch_commit(fb_session* s, int tracked_path, cudaStream_t st) {
+    fb_launch(k_commit, (const void*)k_commit_fused, 1, 64, 0, st, s->st, s->ctr, s->h_out_dev ? s->h_out_dev : s->d_out,
+              tracked_path);
 }
 
-void launch_commit(fb_session* s, int tracked_path, cudaStream_t st) {
-    fb_launch(k_commit, (const void*)k_commit_fused, 1, 1, 0, st, s->st, s->ctr, s->d_out, tracked_path);
+int fetch_result(fb_session* s, cudaStream_t st) {
+    if (!s->h_out_dev) FB_CUDA(cudaMemcpyAsync(s->h_out, s->d_out, sizeof(FrameOut), cudaMemcpyDeviceToHost, st));
+    return FB_OK;
 }
 
 }  // namespace fb
@@ -1000,7 +1002,8 @@ int fb_grab_frame(fb_session* s, const uint16_t* depth, size_t depth_pitch, cons
     unsigned ran = 0;
     rc = enqueue_frame(s, p, s->stream, &ran);
     if (rc) return rc;
-    FB_CUDA(cudaMemcpyAsync(s->h_out, s->d_out, sizeof(FrameOut), cudaMemcpyDeviceToHost, s->stream));
+    rc = fetch_result(s, s->stream);
+    if (rc) return rc;
     FB_CUDA(cudaStreamSynchronize(s->stream));
     if (s->profile)
         for (int k = 0; k < kStages; ++k) {

@@ -205,9 +205,9 @@ int issue_frame(fb_session* s, bool track, bool fuse, bool render, bool init, un
 // frame) and, after the caller's launches, the frame result.
 void launch_track_reloc(fb_session* s, const double* T, cudaStream_t st);
 void launch_commit(fb_session* s, int tracked_path, cudaStream_t st);
-// The frame result from the device into the session's pinned h_out by a
-// kernel (the fused batch step's replacement of the per-session copy).
-void launch_result_out(fb_session* s, cudaStream_t st);
+// Issued after the frame (launch_commit): its result into h_out, where the
+// kernel has not written it there itself.
+int fetch_result(fb_session* s, cudaStream_t st);
 int image_ok(const fb_image* im, size_t elem);
 cudaStream_t as_stream(void* s);
 DevPose pose_from(const float R[9], const float Rinv[9], const float t[3]);

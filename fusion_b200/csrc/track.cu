@@ -548,23 +548,11 @@ __device__ double euler_sin_norm(const double* T) {
 
 // ------------------------------------------------------------------ kernels
 
-// Frame start: the next pose starts from the last pose (TrackFrame's
-// bootstrap fallback, Tracking.cc:156-159) and delta is the identity.
 __device__ __forceinline__ void track_begin_body(const BlockCtx&, TrackState* st, TrackSync* sync, unsigned step) {
-    sync->epoch += step;   // the frame's exchanges (k_track_loop) are numbered from here
-    for (int i = 0; i < 16; ++i) {
-        st->pose[i] = st->last_pose[i];
-        st->init_pose[i] = st->last_pose[i];
-        st->delta[i] = (i % 5 == 0) ? 1.0 : 0.0;
-    }
-    st->cur = make_dev_pose_d(st->pose);
-    st->last = make_dev_pose_d(st->last_pose);
-    st->failed = 0;
-    st->icp_error = st->rgb_error = qnan();
-    st->icp_count = st->rgb_count = 0;
+    track_begin(st, sync, step);
 }
 __global__ void k_track_begin(TrackState* st, TrackSync* sync, unsigned step) {
-    track_begin_body(own_ctx(), st, sync, step);
+    if (threadIdx.x == 0) track_begin(st, sync, step);
 }
 FB_FUSED_KERNEL(k_track_begin, track_begin_body, 32)
 
@@ -1761,8 +1749,7 @@ int track_grid(int n) {
 }
 
 int launch_track_begin(TrackState* st, TrackSync* sync, const int iters[3], cudaStream_t s) {
-    const unsigned step = (unsigned)(iters[0] + iters[1] + iters[2]) + 1u;
-    fb_launch(k_track_begin, (const void*)k_track_begin_fused, 1, 1, 0, s, st, sync, step);
+    fb_launch(k_track_begin, (const void*)k_track_begin_fused, 1, 1, 0, s, st, sync, track_exchanges(iters));
     return 1;
 }
 
