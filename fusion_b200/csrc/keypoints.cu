@@ -128,8 +128,12 @@ struct Integral {
         y0 = min(max(y0, 0), H);
         y1 = min(max(y1, 0), H);
         if (x1 <= x0 || y1 <= y0) return 0;
-        const int s = W + 1;
-        return (int)(I[(size_t)y1 * s + x1] - I[(size_t)y0 * s + x1] - I[(size_t)y1 * s + x0] + I[(size_t)y0 * s + x0]);
+        return inner(x0, y0, x1, y1);
+    }
+    // the same for a box inside the image that is not empty
+    __device__ __forceinline__ int inner(int x0, int y0, int x1, int y1) const {
+        const uint32_t *a = I + (size_t)y0 * (W + 1), *b = I + (size_t)y1 * (W + 1);
+        return (int)(b[x1] - a[x1] - b[x0] + a[x0]);
     }
 };
 
@@ -140,21 +144,31 @@ struct Integral {
 // l x l squares around the centre, each normalised by L^2; Dxy weighted 0.9.
 // One rounding per operation (no contraction), so a CPU restatement
 // reproduces every response.
+// The filter must fit in the image around (x, y).
 __device__ __forceinline__ float hessian_det(const Integral& it, int x, int y, int L) {
     const int l = L / 3, h = (3 * l - 1) / 2, m = (l - 1) / 2;
-    const int dyy = it.box(x - (l - 1), y - h, x + l, y + h + 1) - 3 * it.box(x - (l - 1), y - m, x + l, y + m + 1);
-    const int dxx = it.box(x - h, y - (l - 1), x + h + 1, y + l) - 3 * it.box(x - m, y - (l - 1), x + m + 1, y + l);
-    const int dxy = it.box(x - l, y - l, x, y) + it.box(x + 1, y + 1, x + l + 1, y + l + 1) -
-                    it.box(x + 1, y - l, x + l + 1, y) - it.box(x - l, y + 1, x, y + l + 1);
+    const int dyy = it.inner(x - (l - 1), y - h, x + l, y + h + 1) - 3 * it.inner(x - (l - 1), y - m, x + l, y + m + 1);
+    const int dxx = it.inner(x - h, y - (l - 1), x + h + 1, y + l) - 3 * it.inner(x - m, y - (l - 1), x + m + 1, y + l);
+    const int dxy = it.inner(x - l, y - l, x, y) + it.inner(x + 1, y + 1, x + l + 1, y + l + 1) -
+                    it.inner(x + 1, y - l, x + l + 1, y) - it.inner(x - l, y + 1, x, y + l + 1);
     const float inv = fd(1.0f, fm((float)L, (float)L));
     const float fxx = fm((float)dxx, inv), fyy = fm((float)dyy, inv), fxy = fm((float)dxy, inv);
     return fs(fm(fxx, fyy), fm(fm(0.81f, fxy), fxy));
 }
 
-// All layers of one octave at its samples (pixel = sample << o); zero where
-// the octave's largest filter does not fit.  map: [layer][oh][ow].
-__global__ void k_hessian(Integral it, float* __restrict__ map, int ow, int oh, int o) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x, j = blockIdx.y * blockDim.y + threadIdx.y;
+// The octaves of a detection: their response maps ([layer][oh][ow]) and the
+// first sample code of each (k_extrema).
+struct Octaves {
+    float* map[kSurfOctaves];
+    int ow[kSurfOctaves], oh[kSurfOctaves], code0[kSurfOctaves];
+};
+
+// All layers of one octave (blockIdx.z) at its samples (pixel = sample << o);
+// zero where the octave's largest filter does not fit.  All octaves in one
+// launch: as four, with clipped boxes, they took 43 us at 640x480, so 19.
+template <int o>
+__device__ __forceinline__ void hessian_octave(const Integral& it, float* __restrict__ map, int ow, int oh, int i,
+                                               int j) {
     if (i >= ow || j >= oh) return;
     const int x = i << o, y = j << o, mg = surf_margin(o);
     const bool in = x >= mg && y >= mg && x < it.W - mg && y < it.H - mg;
@@ -162,15 +176,27 @@ __global__ void k_hessian(Integral it, float* __restrict__ map, int ow, int oh, 
     for (int l = 0; l < kSurfLayers; ++l)
         map[((size_t)l * oh + j) * ow + i] = in ? hessian_det(it, x, y, surf_filter(o, l)) : 0.f;
 }
+__global__ void __launch_bounds__(256) k_hessian(Integral it, Octaves oc) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x, j = blockIdx.y * blockDim.y + threadIdx.y;
+    static_assert(kSurfOctaves == 4, "the octaves below");
+    switch (blockIdx.z) {
+    case 0: hessian_octave<0>(it, oc.map[0], oc.ow[0], oc.oh[0], i, j); break;
+    case 1: hessian_octave<1>(it, oc.map[1], oc.ow[1], oc.oh[1], i, j); break;
+    case 2: hessian_octave<2>(it, oc.map[2], oc.ow[2], oc.oh[2], i, j); break;
+    default: hessian_octave<3>(it, oc.map[3], oc.ow[3], oc.oh[3], i, j); break;
+    }
+}
 
-// Candidates of one octave: samples of the middle layers above the threshold
+// Candidates of one octave (blockIdx.z): samples of the middle layers above the threshold
 // and above their 26 neighbours, refined by a quadratic fit (offsets below
 // half a sample).  cand = {x, y, scale, response}; key = response bits << 32
 // | sample index over all octaves' middle layers (unique: a total order, as
 // responses are positive); slotmap[sample index] = the candidate's slot.
-__global__ void k_extrema(const float* __restrict__ M, int ow, int oh, int o, int code0, float threshold,
-                          float4* __restrict__ cand, unsigned long long* __restrict__ keys, int* __restrict__ slotmap,
-                          int* __restrict__ counter, int cap) {
+__global__ void __launch_bounds__(256) k_extrema(Octaves oc, float threshold, float4* __restrict__ cand,
+                                                 unsigned long long* __restrict__ keys, int* __restrict__ slotmap,
+                                                 int* __restrict__ counter, int cap) {
+    const int o = blockIdx.z, ow = oc.ow[o], oh = oc.oh[o], code0 = oc.code0[o];
+    const float* __restrict__ M = oc.map[o];
     const int i = blockIdx.x * blockDim.x + threadIdx.x, j = blockIdx.y * blockDim.y + threadIdx.y;
     const int mg = (surf_margin(o) + (1 << o) - 1) >> o;   // margin in samples
     if (i < mg + 1 || j < mg + 1 || i >= ow - mg - 1 || j >= oh - mg - 1) return;
@@ -178,16 +204,14 @@ __global__ void k_extrema(const float* __restrict__ M, int ow, int oh, int o, in
     for (int l = 1; l < kSurfLayers - 1; ++l) {
         const float v = at(l, j, i);
         if (!(v > threshold)) continue;
+        // the 26 neighbours together (one after another until one is larger:
+        // 21 us at 640x480, so 18)
+        float nb[27];
+#pragma unroll
+        for (int q = 0; q < 27; ++q) nb[q] = at(l + q / 9 - 1, j + (q / 3) % 3 - 1, i + q % 3 - 1);
         bool peak = true;
-        for (int dl = -1; dl <= 1 && peak; ++dl)
-            for (int dj = -1; dj <= 1 && peak; ++dj)
-                for (int di = -1; di <= 1; ++di) {
-                    if (!dl && !dj && !di) continue;
-                    if (!(v > at(l + dl, j + dj, i + di))) {
-                        peak = false;
-                        break;
-                    }
-                }
+#pragma unroll
+        for (int q = 0; q < 27; ++q) peak = peak && (q == 13 || v > nb[q]);
         if (!peak) continue;
         // gradient and Hessian by central differences in (x, y, layer)
         const float gx = 0.5f * (at(l, j, i + 1) - at(l, j, i - 1));
@@ -248,14 +272,45 @@ __global__ void __launch_bounds__(1024) k_sort_keys(unsigned long long* __restri
 
 __device__ __forceinline__ void haar(const Integral& it, int x, int y, int h, float& dx, float& dy) {
     const int r = h / 2;
+    if (x - r >= 0 && y - r >= 0 && x + r <= it.W && y + r <= it.H) {
+        // inside the image: the halves share their corners (integers: exact)
+        const uint32_t *a = it.I + (size_t)(y - r) * (it.W + 1) + x, *b = it.I + (size_t)y * (it.W + 1) + x,
+                       *c = it.I + (size_t)(y + r) * (it.W + 1) + x;
+        const uint32_t a0 = a[-r], a1 = a[0], a2 = a[r], b0 = b[-r], b2 = b[r], c0 = c[-r], c1 = c[0], c2 = c[r];
+        dx = (float)((int)(c2 - a2 - c1 + a1) - (int)(c1 - a1 - c0 + a0));
+        dy = (float)((int)(c2 - b2 - c0 + b0) - (int)(b2 - a2 - b0 + a0));
+        return;
+    }
     dx = (float)(it.box(x, y - r, x + r, y + r) - it.box(x - r, y - r, x, y + r));
     dy = (float)(it.box(x - r, y, x + r, y + r) - it.box(x - r, y - r, x + r, y));
 }
 
 __device__ __forceinline__ int even_size(float v) { return max(2, 2 * __float2int_rn(0.5f * v)); }
 
+// The orientation's samples (a, b) with a^2 + b^2 < 36, by b, then a.
+constexpr int kOrient = 109;
+struct OrientSamples {
+    signed char a[kOrient], b[kOrient];
+};
+constexpr OrientSamples orient_samples() {
+    OrientSamples s{};
+    int m = 0;
+    for (int b = -5; b <= 5; ++b)
+        for (int a = -5; a <= 5; ++a)
+            if (a * a + b * b < 36) {
+                s.a[m] = (signed char)a;
+                s.b[m] = (signed char)b;
+                ++m;
+            }
+    return s;
+}
+__constant__ OrientSamples c_orient = orient_samples();
+
 // One warp per selected key point: orientation, then the 64 descriptor
-// values.  kp out: {x, y, scale, angle}.
+// values.  kp out: {x, y, scale, angle}.  Bound by the latency of the integral
+// image's gathers; the samples are dealt to the lanes from a table (counted
+// off in a loop, each was one lane's alone: 112 us for 3000 keys, now 26),
+// and a lane's windows share their reads of the samples.
 __global__ void __launch_bounds__(256) k_describe(Integral it, const float4* __restrict__ cand,
                                                   const unsigned long long* __restrict__ keys,
                                                   const int* __restrict__ slotmap, int n, float4* __restrict__ kp,
@@ -263,51 +318,51 @@ __global__ void __launch_bounds__(256) k_describe(Integral it, const float4* __r
     const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
     const int k = blockIdx.x * 8 + wib;
     if (k >= n) return;
-    __shared__ float s_dx[8][112], s_dy[8][112], s_ang[8][112];
+    __shared__ float4 s_or[8][kOrient];   // dx, dy, angle
     const int slot = slotmap[(unsigned)(keys[k] & 0xffffffffull)];
     const float4 c = cand[slot];
     const float x = c.x, y = c.y, s = c.z;
     // orientation: Haar responses of side 4s within radius 6s, step s,
     // Gaussian sigma 2s
     const int h4 = even_size(4.f * s);
-    int m = 0;
-    for (int b = -5; b <= 5; ++b)
-        for (int a = -5; a <= 5; ++a) {
-            if (a * a + b * b >= 36) continue;
-            if ((m & 31) == lane) {
-                float dx, dy;
-                haar(it, __float2int_rn(x + a * s), __float2int_rn(y + b * s), h4, dx, dy);
-                const float g = expf(-(float)(a * a + b * b) / 8.f);
-                dx *= g;
-                dy *= g;
-                float ang = atan2f(dy, dx);
-                if (ang < 0.f) ang += 6.2831853f;
-                s_dx[wib][m] = dx;
-                s_dy[wib][m] = dy;
-                s_ang[wib][m] = ang;
-            }
-            ++m;
-        }
+    for (int m = lane; m < kOrient; m += 32) {
+        const int a = c_orient.a[m], b = c_orient.b[m];
+        float dx, dy;
+        haar(it, __float2int_rn(x + a * s), __float2int_rn(y + b * s), h4, dx, dy);
+        const float g = expf(-(float)(a * a + b * b) / 8.f);
+        dx *= g;
+        dy *= g;
+        float ang = atan2f(dy, dx);
+        if (ang < 0.f) ang += 6.2831853f;
+        s_or[wib][m] = make_float4(dx, dy, ang, 0.f);
+    }
     __syncwarp();
     // 72 windows of pi/3 starting every 5 degrees; the longest summed vector
+    // (windows lane, lane + 32 and, in 8 lanes, lane + 64)
     float best = -1.f, bx = 0.f, by = 0.f;
     int bw = 0;
-    for (int w = lane; w < 72; w += 32) {
-        const float start = (float)w * (6.2831853f / 72.f);
-        float sx = 0.f, sy = 0.f;
-        for (int q = 0; q < m; ++q) {
-            float d = s_ang[wib][q] - start;
+    float sx[3] = {0.f, 0.f, 0.f}, sy[3] = {0.f, 0.f, 0.f};
+#pragma unroll 4
+    for (int q = 0; q < kOrient; ++q) {
+        const float4 v = s_or[wib][q];
+#pragma unroll
+        for (int j = 0; j < 3; ++j) {
+            float d = v.z - (float)(lane + 32 * j) * (6.2831853f / 72.f);
             if (d < 0.f) d += 6.2831853f;
             if (d < 1.0471976f) {
-                sx += s_dx[wib][q];
-                sy += s_dy[wib][q];
+                sx[j] += v.x;
+                sy[j] += v.y;
             }
         }
-        const float mag = sx * sx + sy * sy;
-        if (mag > best) {
+    }
+#pragma unroll
+    for (int j = 0; j < 3; ++j) {
+        const int w = lane + 32 * j;
+        const float mag = sx[j] * sx[j] + sy[j] * sy[j];
+        if (w < 72 && mag > best) {
             best = mag;
-            bx = sx;
-            by = sy;
+            bx = sx[j];
+            by = sy[j];
             bw = w;
         }
     }
@@ -419,6 +474,7 @@ __global__ void __launch_bounds__(1024) k_backproject(const float4* __restrict__
                                                       float cutoff, KeySet out, int* __restrict__ n_out) {
     __shared__ int warp_tot[32];
     __shared__ int base;
+    __shared__ int s_src[1024];   // where the chunk's keys go, -1: dropped
     if (threadIdx.x == 0) base = 0;
     __syncthreads();
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
@@ -448,7 +504,16 @@ __global__ void __launch_bounds__(1024) k_backproject(const float4* __restrict__
             out.kp[o] = key;
             out.pt[o] = pt;
             out.nrm[o] = nl;
-            for (int q = 0; q < kKeyDesc; ++q) out.desc[(size_t)o * kKeyDesc + q] = kdesc[(size_t)i * kKeyDesc + q];
+        }
+        // the kept descriptors, in order: a row per 16 lanes (one per thread,
+        // 64 values one after another: 17 us for the kernel, now 7)
+        s_src[threadIdx.x] = keep && o < out.cap ? o : -1;
+        __syncthreads();
+        for (int r = threadIdx.x >> 4; r < 1024 && k0 + r < n; r += 64) {
+            const int to = s_src[r];
+            if (to >= 0)
+                reinterpret_cast<float4*>(out.desc + (size_t)to * kKeyDesc)[threadIdx.x & 15] =
+                    reinterpret_cast<const float4*>(kdesc + (size_t)(k0 + r) * kKeyDesc)[threadIdx.x & 15];
         }
         __syncthreads();
         if (threadIdx.x == 0) {
@@ -707,24 +772,24 @@ int launch_surf(const uint8_t* gray, int gp, float threshold, const KeyScratch& 
     k_integral_rows<<<H, 256, 0, st>>>(gray, gp, W, H, ks.integral);
     k_integral_cols<<<(W + 1 + 31) / 32, dim3(32, 16), 0, st>>>(ks.integral, W, H);
     const Integral it{ks.integral, W, H};
-    int code0[kSurfOctaves], code = 0;
+    Octaves oc;
+    int code = 0;
     for (int o = 0; o < kSurfOctaves; ++o) {
-        code0[o] = code;
+        oc.map[o] = ks.det[o];
+        oc.ow[o] = ks.ow[o];
+        oc.oh[o] = ks.oh[o];
+        oc.code0[o] = code;
         code += (kSurfLayers - 2) * ks.ow[o] * ks.oh[o];
-        dim3 b(32, 8), g((ks.ow[o] + 31) / 32, (ks.oh[o] + 7) / 8);
-        k_hessian<<<g, b, 0, st>>>(it, ks.det[o], ks.ow[o], ks.oh[o], o);
     }
+    const dim3 b(32, 8), g((ks.ow[0] + 31) / 32, (ks.oh[0] + 7) / 8, kSurfOctaves);
+    k_hessian<<<g, b, 0, st>>>(it, oc);
     // candidates; a set larger than the buffer is found again with a doubled
     // threshold (which candidates are kept must not depend on arrival order)
     int count = 0;
     float thr = threshold;
     for (int attempt = 0; attempt < 8; ++attempt) {
         if (cudaMemsetAsync(ks.counter, 0, 4, st) != cudaSuccess) return FB_ECUDA;
-        for (int o = 0; o < kSurfOctaves; ++o) {
-            dim3 b(32, 8), g((ks.ow[o] + 31) / 32, (ks.oh[o] + 7) / 8);
-            k_extrema<<<g, b, 0, st>>>(ks.det[o], ks.ow[o], ks.oh[o], o, code0[o], thr, ks.cand, ks.keys, ks.slotmap,
-                                       ks.counter, kSurfMaxCand);
-        }
+        k_extrema<<<g, b, 0, st>>>(oc, thr, ks.cand, ks.keys, ks.slotmap, ks.counter, kSurfMaxCand);
         if (cudaMemcpyAsync(&count, ks.counter, 4, cudaMemcpyDeviceToHost, st) != cudaSuccess) return FB_ECUDA;
         if (cudaStreamSynchronize(st) != cudaSuccess) return FB_ECUDA;
         if (count <= kSurfMaxCand) break;
