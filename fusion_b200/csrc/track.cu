@@ -125,10 +125,11 @@ __device__ __forceinline__ int rgb_corresp(const TrackLevel& L, const DevPose& c
         if (!L.rgbok[(size_t)y * L.sp + x]) return -1;
     } else {
         if (!(x >= 5 && x < W - 5 && y >= 5 && y < H - 5)) return -1;
-        // the window is y-2..y+1, x-2..x+1 (Reduction.cu:416-417)
-        for (int u = y - 2; u < y + 2; ++u)
-            for (int v = x - 2; v < x + 2; ++v)
-                if (L.gcurr[(size_t)u * L.gp + v] == 0) return -1;
+        // the window is y-2..y+1, x-2..x+1 (Reduction.cu:416-417), loaded together
+        bool any0 = false;
+#pragma unroll
+        for (int q = 0; q < 16; ++q) any0 |= L.gcurr[(size_t)(y - 2 + q / 4) * L.gp + x - 2 + q % 4] == 0;
+        if (any0) return -1;
         int gx = L.dx[(size_t)y * L.sp + x], gy = L.dy[(size_t)y * L.sp + x];
         if (gx == 0 && gy == 0) return -1;  // sqrtf(gx*gx + gy*gy) > 0
     }
@@ -414,38 +415,12 @@ __device__ __forceinline__ void add_segment_rows(const TrackLevel& L, const DevP
 
 // ------------------------------------------------------------- reductions
 
-// Block-wide sum of NV floats (deterministic).  Result valid in thread 0.
-template <int NV>
-__device__ __forceinline__ void block_sum(float v[NV], float* smem /* [32][NV] */) {
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
-#pragma unroll
-    for (int k = 0; k < NV; ++k) {
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) v[k] += __shfl_down_sync(0xffffffffu, v[k], o);
-    }
-    if (lane == 0)
-#pragma unroll
-        for (int k = 0; k < NV; ++k) smem[wid * NV + k] = v[k];
-    __syncthreads();
-    if (wid == 0) {
-#pragma unroll
-        for (int k = 0; k < NV; ++k) v[k] = lane < nw ? smem[lane * NV + k] : 0.f;
-#pragma unroll
-        for (int k = 0; k < NV; ++k) {
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) v[k] += __shfl_down_sync(0xffffffffu, v[k], o);
-        }
-    }
-}
-
-// Block-wide sum of the 29 per-thread values of the normal equations.  Each
-// warp first reduces its 32 lanes by recursive halving (at every step a lane
-// keeps one half of its values, sends the other half to its partner and adds
-// what it receives: 31 shuffles in all), after which lane l holds the warp
-// sum of value l; warp 0 then adds the warps' sums in warp order.  Result:
-// value l in lane l (< 29) of warp 0.  Deterministic.
-__device__ __forceinline__ float block_sum29(const float (&v)[29], float* smem /* [8][32] */) {
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
+// Warp sums of the 29 per-thread values of the normal equations by recursive
+// halving: at every step a lane keeps one half of its values, sends the other
+// half to its partner and adds what it receives (31 shuffles in all).  Lane l
+// then holds the warp sum of value l, added as the halving tree over the lanes.
+__device__ __forceinline__ float warp_sum29(const float (&v)[29]) {
+    const int lane = threadIdx.x & 31;
     float a[32];
 #pragma unroll
     for (int k = 0; k < 29; ++k) a[k] = v[k];
@@ -460,12 +435,29 @@ __device__ __forceinline__ float block_sum29(const float (&v)[29], float* smem /
             a[k] = keep + __shfl_xor_sync(0xffffffffu, send, off);
         }
     }
-    smem[wid * 32 + lane] = a[0];
+    return a[0];
+}
+
+// Block-wide sum of the 29 values: the warps' sums added in warp order by warp
+// 0.  Result: value l in lane l (< 29) of warp 0.  Deterministic.
+__device__ __forceinline__ float block_sum29(const float (&v)[29], float* smem /* [8][32] */) {
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
+    smem[wid * 32 + lane] = warp_sum29(v);
     __syncthreads();
     float r = 0.f;
     if (wid == 0)
         for (int w = 0; w < nw; ++w) r += smem[w * 32 + lane];
     return r;
+}
+
+// The same with the eight warps' sums added as a halving tree (the single-step
+// entry points' order).
+__device__ __forceinline__ float block_tree29(const float (&v)[29], float* smem /* [8][32] */) {
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    smem[wid * 32 + lane] = warp_sum29(v);
+    __syncthreads();
+    const float* w = smem + lane;
+    return wid == 0 ? ((w[0] + w[128]) + (w[64] + w[192])) + ((w[32] + w[160]) + (w[96] + w[224])) : 0.f;
 }
 
 __device__ __forceinline__ long long block_sum_ll(long long v, long long* smem) {
@@ -483,20 +475,6 @@ __device__ __forceinline__ long long block_sum_ll(long long v, long long* smem) 
     return v;
 }
 
-// Last-block-done: returns true in every thread of the last block to finish.
-__device__ __forceinline__ bool last_block(unsigned int* ticket) {
-    __shared__ bool is_last;
-    __threadfence();
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        unsigned int t = atomicAdd(ticket, 1u);
-        is_last = (t == gridDim.x - 1);
-    }
-    __syncthreads();
-    if (is_last) __threadfence();
-    return is_last;
-}
-
 // Ticket increment with release (this block's prior writes, ordered before it
 // by a block barrier) and acquire (the writes of the blocks that incremented
 // before) semantics at GPU scope.
@@ -504,6 +482,15 @@ __device__ __forceinline__ unsigned int ticket_acq_rel(unsigned int* t) {
     unsigned int old;
     asm volatile("atom.add.acq_rel.gpu.u32 %0, [%1], 1;" : "=r"(old) : "l"(t) : "memory");
     return old;
+}
+
+// Last-block-done: returns true in every thread of the last block to finish.
+__device__ __forceinline__ bool last_block(unsigned int* ticket) {
+    __shared__ bool is_last;
+    __syncthreads();
+    if (threadIdx.x == 0) is_last = ticket_acq_rel(ticket) == gridDim.x - 1;
+    __syncthreads();
+    return is_last;
 }
 
 // ----------------------------------------------------------- FP64 solver
@@ -560,7 +547,7 @@ FB_FUSED_KERNEL(k_track_begin, track_begin_body, 32)
 // partials[b * stride + v], computed by the whole block: thread t sums value
 // (t % 32) over the block chunk (t / 32), then the 8 chunk sums are added in
 // order.  Deterministic for a given nb.  out: shared array of nv doubles.
-__device__ void reduce_partials(const float* __restrict__ partials, int nb, int stride, int nv, double* out,
+__device__ void reduce_partials(const float* partials, int nb, int stride, int nv, double* out,
                                 double* scratch /* [8][32] shared */) {
     const int v = threadIdx.x & 31, c = threadIdx.x >> 5, nc = blockDim.x >> 5;
     const int per = (nb + nc - 1) / nc;
@@ -568,8 +555,15 @@ __device__ void reduce_partials(const float* __restrict__ partials, int nb, int 
         double s = 0;
         if (v0 + v < nv) {
             const int b0 = c * per, b1 = min(nb, b0 + per);
-#pragma unroll 8
-            for (int b = b0; b < b1; ++b) s += (double)partials[(size_t)b * stride + v0 + v];
+            for (int b = b0; b < b1; b += 16) {   // loaded together, added in order
+                float x[16];
+#pragma unroll
+                for (int q = 0; q < 16; ++q)
+                    if (b + q < b1) x[q] = __ldcg(partials + (size_t)(b + q) * stride + v0 + v);
+#pragma unroll
+                for (int q = 0; q < 16; ++q)
+                    if (b + q < b1) s += (double)x[q];
+            }
         }
         scratch[c * 32 + v] = s;
         __syncthreads();
@@ -1646,10 +1640,14 @@ __global__ void __cluster_dims__(kTrackCluster, 1, 1) __launch_bounds__(256, 2)
 }
 
 // Single-step entry points (the reference's ICPStep / RGBStep): reduce the
-// sums of one pass into out[29] (+ rgb count / sum of squares) in FP64.
+// sums of one pass into out[29] (+ rgb count / sum of squares) in FP64.  Bound
+// by latency: a block holds a few pixels a thread.  At 323x241 icp / rgb_a /
+// rgb_b take 7.0 / 5.9 / 6.3 us; with one value after another through the
+// block sum (145 shuffles a warp) and one thread adding the counts they took
+// 10.4 / 17.0 / 10.3.
 __global__ void __launch_bounds__(256) k_step_icp(TrackLevel L, DevPose cur, DevPose last, float* partials,
                                                   unsigned int* ticket, double* out) {
-    __shared__ float sm[32 * 29];
+    __shared__ float sm[8 * 32];
     float acc[29];
 #pragma unroll
     for (int k = 0; k < 29; ++k) acc[k] = 0.f;
@@ -1659,10 +1657,8 @@ __global__ void __launch_bounds__(256) k_step_icp(TrackLevel L, DevPose cur, Dev
         float row[7];
         if (icp_row(L, cur, last, x, y, row)) add_products(row, acc);
     }
-    block_sum<29>(acc, sm);
-    if (threadIdx.x == 0)
-#pragma unroll
-        for (int k = 0; k < 29; ++k) partials[(size_t)blockIdx.x * 32 + k] = acc[k];
+    const float bsum = block_tree29(acc, sm);
+    if (threadIdx.x < 29) partials[(size_t)blockIdx.x * 32 + threadIdx.x] = bsum;
     if (!last_block(ticket)) return;
     __shared__ double scratch[8 * 32];
     __shared__ double sums[32];
@@ -1693,9 +1689,16 @@ __global__ void __launch_bounds__(256) k_step_rgb_a(TrackLevel L, DevPose cur, D
         partials[2 * blockIdx.x + 1] = bs;
     }
     if (!last_block(ticket)) return;
+    // the blocks' counts, all threads together (integers: exact in any order;
+    // one thread after another took 10 us)
+    long long c = 0, q = 0;
+    for (int b = threadIdx.x; b < gridDim.x; b += blockDim.x) {
+        c += __ldcg(partials + 2 * b);
+        q += __ldcg(partials + 2 * b + 1);
+    }
+    c = block_sum_ll(c, smll);
+    q = block_sum_ll(q, smll);
     if (threadIdx.x == 0) {
-        long long c = 0, q = 0;
-        for (int b = 0; b < gridDim.x; ++b) { c += partials[2 * b]; q += partials[2 * b + 1]; }
         out[29] = (double)c;
         out[30] = (double)q;
         out[31] = sqrtf((float)q / (float)(c == 0 ? 1 : c));
@@ -1705,7 +1708,7 @@ __global__ void __launch_bounds__(256) k_step_rgb_a(TrackLevel L, DevPose cur, D
 
 __global__ void __launch_bounds__(256) k_step_rgb_b(TrackLevel L, DevPose cur, DevPose last, float* partials,
                                                     unsigned int* ticket, const int* residual, double* out) {
-    __shared__ float sm[32 * 29];
+    __shared__ float sm[8 * 32];
     const float sigma = (float)out[31];
     float acc[29];
 #pragma unroll
@@ -1719,10 +1722,8 @@ __global__ void __launch_bounds__(256) k_step_rgb_b(TrackLevel L, DevPose cur, D
         rgb_row(L, cur, last, x, y, r, sigma, row);
         add_products(row, acc);
     }
-    block_sum<29>(acc, sm);
-    if (threadIdx.x == 0)
-#pragma unroll
-        for (int k = 0; k < 29; ++k) partials[(size_t)blockIdx.x * 32 + k] = acc[k];
+    const float bsum = block_tree29(acc, sm);
+    if (threadIdx.x < 29) partials[(size_t)blockIdx.x * 32 + threadIdx.x] = bsum;
     if (!last_block(ticket)) return;
     __shared__ double scratch[8 * 32];
     __shared__ double sums[32];
