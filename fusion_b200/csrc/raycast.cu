@@ -364,88 +364,208 @@ __device__ __forceinline__ float read_sdf(const MapView& m, const GridView& gv, 
     return sdf;
 }
 
-// One corner of a trilinear read: the voxel's TSDF in block q, NaN for a
-// missing block (q < 0).  The load always reads a voxel of the pool (block
-// 0 for a missing block) so that the eight loads issue without branches.
-template <class VR>
-__device__ __forceinline__ float corner_sdf(const MapView& m, int q, int idx) {
-    const float v = VR::sdf(VR::at(m, max(q, 0), idx));
-    return q < 0 ? qnan() : v;
+// The eight blocks {x0, x1} x {y0, y1} x {z0, z1}, each coordinate pair equal
+// or adjacent: q[i + 2 j + 4 k] is lookup_block of the block with x index i, y
+// index j, z index k; a missing one is negative.  Where all eight lie in the
+// dense index, the eight loads issue together, equal blocks from the same
+// address (looking up only the distinct ones took a branch each, and the lanes
+// of a warp cross block boundaries at different places).
+__device__ __forceinline__ void lookup_blocks(const MapView& m, const GridView& gv, int x0, int x1, int y0, int y1,
+                                              int z0, int z1, int (&q)[8]) {
+    const int gx0 = x0 - gv.ox, gx1 = x1 - gv.ox, gy0 = y0 - gv.oy, gy1 = y1 - gv.oy, gz0 = z0 - gv.oz,
+              gz1 = z1 - gv.oz;
+    if ((unsigned)gx0 < (unsigned)gv.nx && (unsigned)gx1 < (unsigned)gv.nx && (unsigned)gy0 < (unsigned)gv.ny &&
+        (unsigned)gy1 < (unsigned)gv.ny && (unsigned)gz0 < (unsigned)gv.nz && (unsigned)gz1 < (unsigned)gv.nz) {
+        const int r00 = (gz0 * gv.ny + gy0) * gv.nx, r10 = (gz0 * gv.ny + gy1) * gv.nx;
+        const int r01 = (gz1 * gv.ny + gy0) * gv.nx, r11 = (gz1 * gv.ny + gy1) * gv.nx;
+        q[0] = __ldg(m.grid + r00 + gx0);
+        q[1] = __ldg(m.grid + r00 + gx1);
+        q[2] = __ldg(m.grid + r10 + gx0);
+        q[3] = __ldg(m.grid + r10 + gx1);
+        q[4] = __ldg(m.grid + r01 + gx0);
+        q[5] = __ldg(m.grid + r01 + gx1);
+        q[6] = __ldg(m.grid + r11 + gx0);
+        q[7] = __ldg(m.grid + r11 + gx1);
+        return;
+    }
+    const bool sx = x1 != x0, sy = y1 != y0, sz = z1 != z0;
+    q[0] = lookup_block(m, gv, x0, y0, z0);
+    q[1] = sx ? lookup_block(m, gv, x1, y0, z0) : q[0];
+    q[2] = sy ? lookup_block(m, gv, x0, y1, z0) : q[0];
+    q[3] = sy ? (sx ? lookup_block(m, gv, x1, y1, z0) : q[2]) : q[1];
+    q[4] = sz ? lookup_block(m, gv, x0, y0, z1) : q[0];
+    q[5] = sz ? (sx ? lookup_block(m, gv, x1, y0, z1) : q[4]) : q[1];
+    q[6] = sz ? (sy ? lookup_block(m, gv, x0, y1, z1) : q[4]) : q[2];
+    q[7] = sz ? (sy ? (sx ? lookup_block(m, gv, x1, y1, z1) : q[6]) : q[5]) : q[3];
 }
+
+__device__ __forceinline__ float lerp_sdf(float a, float b, float t) { return fa(fm(fs(1.0f, t), a), fm(t, b)); }
 
 // Rendering::readSdfInterped (RenderScene.cu:297-319).  The eight corners are
 // the voxels at the truncated coordinates of pt and of pt + 1 per axis (each
-// sum rounded as the reference rounds it), read in the reference's order and
-// blended by its lerp sequence; `valid` ends as the last corner's (x+1, y+1,
-// z+1) lookup leaves it.  The corners lie in at most eight blocks, one per
-// axis combination whose coordinates cross a block boundary: each distinct
-// block is looked up once (the first through the entry cache), then the
-// eight TSDF loads issue together.  Every lane of a warp runs the same code
-// whether or not its corners straddle blocks (only the extra lookups are
-// conditional), where a per-corner lookup through the one-entry cache made
-// straddling lanes run a second, eight-lookup path.
+// sum rounded as the reference rounds it), blended by the reference's lerp
+// sequence.  The corners lie in at most eight blocks, one per axis combination
+// whose coordinates cross a block boundary; the first is found through the
+// entry cache.  A missing corner is NaN and makes every lerp over it NaN, so a
+// read with a missing corner returns NaN without loading the others.
 template <class VR>
-__device__ float read_sdf_interp(const MapView& m, const GridView& gv, f3 pt, EntryCache& c, bool& valid) {
+__device__ __forceinline__ float read_sdf_interp(const MapView& m, const GridView& gv, f3 pt, EntryCache& c) {
     const f3 f = mk3(fs(pt.x, floorf(pt.x)), fs(pt.y, floorf(pt.y)), fs(pt.z, floorf(pt.z)));
-    auto lerp = [](float a, float b, float t) { return fa(fm(fs(1.0f, t), a), fm(t, b)); };
     const int x0 = __float2int_rz(pt.x), x1 = __float2int_rz(fa(pt.x, 1.f));
     const int y0 = __float2int_rz(pt.y), y1 = __float2int_rz(fa(pt.y, 1.f));
     const int z0 = __float2int_rz(pt.z), z1 = __float2int_rz(fa(pt.z, 1.f));
     const int bx0 = block_of(x0), bx1 = block_of(x1);
     const int by0 = block_of(y0), by1 = block_of(y1);
     const int bz0 = block_of(z0), bz1 = block_of(z1);
-    const bool sx = bx1 != bx0, sy = by1 != by0, sz = bz1 != bz0;
-    const int q000 = find_block(m, gv, bx0, by0, bz0, c);
-    const int q100 = sx ? lookup_block(m, gv, bx1, by0, bz0) : q000;
-    const int q010 = sy ? lookup_block(m, gv, bx0, by1, bz0) : q000;
-    const int q110 = sy ? (sx ? lookup_block(m, gv, bx1, by1, bz0) : q010) : q100;
-    int q001 = q000, q101 = q100, q011 = q010, q111 = q110;
-    if (sz) {
-        q001 = lookup_block(m, gv, bx0, by0, bz1);
-        q101 = sx ? lookup_block(m, gv, bx1, by0, bz1) : q001;
-        q011 = sy ? lookup_block(m, gv, bx0, by1, bz1) : q001;
-        q111 = sy ? (sx ? lookup_block(m, gv, bx1, by1, bz1) : q011) : q101;
+    int q[8];
+    if (bx1 != bx0 || by1 != by0 || bz1 != bz0) {
+        lookup_blocks(m, gv, bx0, bx1, by0, by1, bz0, bz1, q);
+    } else {
+        q[0] = find_block(m, gv, bx0, by0, bz0, c);
+#pragma unroll
+        for (int i = 1; i < 8; ++i) q[i] = q[0];
     }
-    valid = q111 >= 0;
+    if (((q[0] | q[1]) | (q[2] | q[3]) | (q[4] | q[5]) | (q[6] | q[7])) < 0) return qnan();
     const int ax = local_of(x0), bxl = local_of(x1);
     const int ay = local_of(y0) * 8, byl = local_of(y1) * 8;
     const int az = local_of(z0) * 64, bzl = local_of(z1) * 64;
-    const float s000 = corner_sdf<VR>(m, q000, az + ay + ax);
-    const float s100 = corner_sdf<VR>(m, q100, az + ay + bxl);
-    const float s010 = corner_sdf<VR>(m, q010, az + byl + ax);
-    const float s110 = corner_sdf<VR>(m, q110, az + byl + bxl);
-    const float s001 = corner_sdf<VR>(m, q001, bzl + ay + ax);
-    const float s101 = corner_sdf<VR>(m, q101, bzl + ay + bxl);
-    const float s011 = corner_sdf<VR>(m, q011, bzl + byl + ax);
-    const float s111 = corner_sdf<VR>(m, q111, bzl + byl + bxl);
-    const float r0 = lerp(s000, s100, f.x), r1 = lerp(s010, s110, f.x);
-    const float r2 = lerp(r0, r1, f.y);
-    const float r0b = lerp(s001, s101, f.x), r1b = lerp(s011, s111, f.x);
-    const float r3 = lerp(r0b, r1b, f.y);
-    return lerp(r2, r3, f.z);
+    const float s000 = VR::sdf(VR::at(m, q[0], az + ay + ax));
+    const float s100 = VR::sdf(VR::at(m, q[1], az + ay + bxl));
+    const float s010 = VR::sdf(VR::at(m, q[2], az + byl + ax));
+    const float s110 = VR::sdf(VR::at(m, q[3], az + byl + bxl));
+    const float s001 = VR::sdf(VR::at(m, q[4], bzl + ay + ax));
+    const float s101 = VR::sdf(VR::at(m, q[5], bzl + ay + bxl));
+    const float s011 = VR::sdf(VR::at(m, q[6], bzl + byl + ax));
+    const float s111 = VR::sdf(VR::at(m, q[7], bzl + byl + bxl));
+    const float r2 = lerp_sdf(lerp_sdf(s000, s100, f.x), lerp_sdf(s010, s110, f.x), f.y);
+    const float r3 = lerp_sdf(lerp_sdf(s001, s101, f.x), lerp_sdf(s011, s111, f.x), f.y);
+    return lerp_sdf(r2, r3, f.z);
 }
 
-// Rendering::readNormal (RenderScene.cu:321-352): the six samples at
-// pt +- 1 per axis, in the reference's order, and the normal from their three
-// differences.  Offsets and differences stay in registers (a dynamically
-// indexed table of samples would live in local memory).
+// One axis of the normal's samples: the voxel coordinates that the samples at
+// p - 1, p and p + 1 read (the truncated p - 1, p, p + 1 and p + 2, each sum
+// rounded as the reference rounds it), their fractions, and the at most two
+// blocks the coordinates lie in.  ok: the upper voxel of the sample at p - 1
+// is the lower one of the sample at p (rounding can part them).
+struct NormalAxis {
+    int vm, v0, v1, v2;      // voxel coordinates
+    int lo, hi;              // blocks of vm and v2
+    bool h0, h1;             // v0 / v1 lie in block hi
+    float f0, fp, fm;        // fractions at p, p + 1, p - 1
+    bool ok;
+};
+__device__ __forceinline__ NormalAxis normal_axis(float p) {
+    NormalAxis a;
+    const float pp = fa(p, 1.0f), pm = fa(p, -1.0f);
+    a.vm = __float2int_rz(pm);
+    a.v0 = __float2int_rz(p);
+    a.v1 = __float2int_rz(pp);
+    a.v2 = __float2int_rz(fa(pp, 1.0f));
+    a.ok = __float2int_rz(fa(pm, 1.0f)) == a.v0;
+    a.lo = block_of(a.vm);
+    a.hi = block_of(a.v2);
+    a.h0 = block_of(a.v0) != a.lo;
+    a.h1 = block_of(a.v1) != a.lo;
+    a.f0 = fs(p, floorf(p));
+    a.fp = fs(pp, floorf(pp));
+    a.fm = fs(pm, floorf(pm));
+    return a;
+}
+
+// Rendering::readNormal (RenderScene.cu:321-352): the six samples at pt +- 1
+// per axis and the normal from their three differences.  The six trilinear
+// reads share their voxels: the eight around pt and four more per sample, 32
+// in all, in at most eight blocks.  Taken one after another the reads were six
+// dependent look-ups and load rounds (48 voxels) and took half of a ray's
+// time: 21 k of 45 k cycles a warp at 640x480.  Here the blocks are looked up
+// once, the loads of a group issue together and the lerps along x of the eight
+// inner voxels are computed once; every sample is blended in the reference's
+// order.  Where rounding parts the samples' voxels, the general form below
+// reads one sample after another.
 template <class VR>
-__device__ bool read_normal(const MapView& m, const GridView& gv, f3 pt, EntryCache& c, const M3& Rinv, f3& n) {
-    bool valid;
-    float prev = 0.0f, gx = 0.0f, gy = 0.0f, gz = 0.0f;
-    for (int q = 0; q < 6; ++q) {
-        const float d = (q & 1) ? -1.0f : 1.0f;
-        const int a = q >> 1;
-        const f3 ps = mk3(fa(pt.x, a == 0 ? d : 0.0f), fa(pt.y, a == 1 ? d : 0.0f), fa(pt.z, a == 2 ? d : 0.0f));
-        const float sq = read_sdf_interp<VR>(m, gv, ps, c, valid);
-        if (isnan(sq) || sq == 1.0f || !valid) return false;
-        if (q & 1) {
-            const float g = fs(prev, sq);
-            gx = a == 0 ? g : gx;
-            gy = a == 1 ? g : gy;
-            gz = a == 2 ? g : gz;
+__device__ __forceinline__ bool read_normal(const MapView& m, const GridView& gv, f3 pt, EntryCache& c,
+                                            const M3& Rinv, f3& n) {
+    float gx, gy, gz;
+    const NormalAxis X = normal_axis(pt.x), Y = normal_axis(pt.y), Z = normal_axis(pt.z);
+    auto bad = [](float s) { return isnan(s) || s == 1.0f; };
+    if (X.ok && Y.ok && Z.ok) {
+        int q[8];
+        lookup_blocks(m, gv, X.lo, X.hi, Y.lo, Y.hi, Z.lo, Z.hi, q);
+        // a voxel's block by its coordinates' sides
+        auto blk = [&](bool hx, bool hy, bool hz) {
+            const int a = hx ? q[1] : q[0], b = hx ? q[3] : q[2], d = hx ? q[5] : q[4], e = hx ? q[7] : q[6];
+            const int l = hy ? b : a, h = hy ? e : d;
+            return hz ? h : l;
+        };
+        int miss = 0;
+        auto ld = [&](int vx, bool hx, int vy, bool hy, int vz, bool hz) {
+            const int p = blk(hx, hy, hz);
+            miss |= p;
+            return VR::sdf(VR::at(m, max(p, 0), local_of(vz) * 64 + local_of(vy) * 8 + local_of(vx)));
+        };
+        // the eight inner voxels c(xyz)
+        const float c000 = ld(X.v0, X.h0, Y.v0, Y.h0, Z.v0, Z.h0), c100 = ld(X.v1, X.h1, Y.v0, Y.h0, Z.v0, Z.h0);
+        const float c010 = ld(X.v0, X.h0, Y.v1, Y.h1, Z.v0, Z.h0), c110 = ld(X.v1, X.h1, Y.v1, Y.h1, Z.v0, Z.h0);
+        const float c001 = ld(X.v0, X.h0, Y.v0, Y.h0, Z.v1, Z.h1), c101 = ld(X.v1, X.h1, Y.v0, Y.h0, Z.v1, Z.h1);
+        const float c011 = ld(X.v0, X.h0, Y.v1, Y.h1, Z.v1, Z.h1), c111 = ld(X.v1, X.h1, Y.v1, Y.h1, Z.v1, Z.h1);
+        float sp, sm;
+        {
+            const float p00 = ld(X.v2, true, Y.v0, Y.h0, Z.v0, Z.h0), p10 = ld(X.v2, true, Y.v1, Y.h1, Z.v0, Z.h0);
+            const float p01 = ld(X.v2, true, Y.v0, Y.h0, Z.v1, Z.h1), p11 = ld(X.v2, true, Y.v1, Y.h1, Z.v1, Z.h1);
+            const float m00 = ld(X.vm, false, Y.v0, Y.h0, Z.v0, Z.h0), m10 = ld(X.vm, false, Y.v1, Y.h1, Z.v0, Z.h0);
+            const float m01 = ld(X.vm, false, Y.v0, Y.h0, Z.v1, Z.h1), m11 = ld(X.vm, false, Y.v1, Y.h1, Z.v1, Z.h1);
+            sp = lerp_sdf(lerp_sdf(lerp_sdf(c100, p00, X.fp), lerp_sdf(c110, p10, X.fp), Y.f0),
+                          lerp_sdf(lerp_sdf(c101, p01, X.fp), lerp_sdf(c111, p11, X.fp), Y.f0), Z.f0);
+            sm = lerp_sdf(lerp_sdf(lerp_sdf(m00, c000, X.fm), lerp_sdf(m10, c010, X.fm), Y.f0),
+                          lerp_sdf(lerp_sdf(m01, c001, X.fm), lerp_sdf(m11, c011, X.fm), Y.f0), Z.f0);
         }
-        prev = sq;
+        if (bad(sp) || bad(sm)) miss = -1;
+        gx = fs(sp, sm);
+        const float l00 = lerp_sdf(c000, c100, X.f0), l10 = lerp_sdf(c010, c110, X.f0);
+        const float l01 = lerp_sdf(c001, c101, X.f0), l11 = lerp_sdf(c011, c111, X.f0);
+        {
+            const float p00 = ld(X.v0, X.h0, Y.v2, true, Z.v0, Z.h0), p10 = ld(X.v1, X.h1, Y.v2, true, Z.v0, Z.h0);
+            const float p01 = ld(X.v0, X.h0, Y.v2, true, Z.v1, Z.h1), p11 = ld(X.v1, X.h1, Y.v2, true, Z.v1, Z.h1);
+            const float m00 = ld(X.v0, X.h0, Y.vm, false, Z.v0, Z.h0), m10 = ld(X.v1, X.h1, Y.vm, false, Z.v0, Z.h0);
+            const float m01 = ld(X.v0, X.h0, Y.vm, false, Z.v1, Z.h1), m11 = ld(X.v1, X.h1, Y.vm, false, Z.v1, Z.h1);
+            sp = lerp_sdf(lerp_sdf(l10, lerp_sdf(p00, p10, X.f0), Y.fp), lerp_sdf(l11, lerp_sdf(p01, p11, X.f0), Y.fp),
+                          Z.f0);
+            sm = lerp_sdf(lerp_sdf(lerp_sdf(m00, m10, X.f0), l00, Y.fm), lerp_sdf(lerp_sdf(m01, m11, X.f0), l01, Y.fm),
+                          Z.f0);
+        }
+        if (bad(sp) || bad(sm)) miss = -1;
+        gy = fs(sp, sm);
+        {
+            const float p00 = ld(X.v0, X.h0, Y.v0, Y.h0, Z.v2, true), p10 = ld(X.v1, X.h1, Y.v0, Y.h0, Z.v2, true);
+            const float p01 = ld(X.v0, X.h0, Y.v1, Y.h1, Z.v2, true), p11 = ld(X.v1, X.h1, Y.v1, Y.h1, Z.v2, true);
+            const float m00 = ld(X.v0, X.h0, Y.v0, Y.h0, Z.vm, false), m10 = ld(X.v1, X.h1, Y.v0, Y.h0, Z.vm, false);
+            const float m01 = ld(X.v0, X.h0, Y.v1, Y.h1, Z.vm, false), m11 = ld(X.v1, X.h1, Y.v1, Y.h1, Z.vm, false);
+            sp = lerp_sdf(lerp_sdf(l01, l11, Y.f0),
+                          lerp_sdf(lerp_sdf(p00, p10, X.f0), lerp_sdf(p01, p11, X.f0), Y.f0), Z.fp);
+            sm = lerp_sdf(lerp_sdf(lerp_sdf(m00, m10, X.f0), lerp_sdf(m01, m11, X.f0), Y.f0), lerp_sdf(l00, l10, Y.f0),
+                          Z.fm);
+        }
+        if (bad(sp) || bad(sm)) miss = -1;
+        gz = fs(sp, sm);
+        if (miss < 0) return false;   // a missing voxel is NaN, and so is its sample
+    } else {
+        float prev = 0.0f;
+        gx = gy = gz = 0.0f;
+#pragma unroll 1
+        for (int q = 0; q < 6; ++q) {
+            const float d = (q & 1) ? -1.0f : 1.0f;
+            const int a = q >> 1;
+            const f3 ps = mk3(fa(pt.x, a == 0 ? d : 0.0f), fa(pt.y, a == 1 ? d : 0.0f), fa(pt.z, a == 2 ? d : 0.0f));
+            const float sq = read_sdf_interp<VR>(m, gv, ps, c);
+            if (bad(sq)) return false;
+            if (q & 1) {
+                const float g = fs(prev, sq);
+                gx = a == 0 ? g : gx;
+                gy = a == 1 ? g : gy;
+                gz = a == 2 ? g : gz;
+            }
+            prev = sq;
+        }
     }
     n = normalised3(mv(Rinv, mk3(gx, gy, gz)));
     return true;
@@ -510,7 +630,7 @@ __device__ __forceinline__ bool ray_step(const MapView& m, const GridView& gv, f
     if (!valid) {
         step = 8.0f;
     } else {
-        if (r.sdf <= 0.1f && r.sdf >= -0.5f) r.sdf = read_sdf_interp<VR>(m, gv, r.result, c, valid);
+        if (r.sdf <= 0.1f && r.sdf >= -0.5f) r.sdf = read_sdf_interp<VR>(m, gv, r.result, c);
         if (r.sdf <= 0.0f) return true;
         step = !isnan(r.sdf) ? fmaxf(fm(r.sdf, stepScale), 1.0f) : 8.0f;
     }
@@ -529,10 +649,9 @@ __device__ __forceinline__ void ray_finish(const MapView& m, const GridView& gv,
     vout = nan4;
     nout = nan4;
     if (!(r.sdf <= 0.0f)) return;
-    bool valid;
     float step = fm(r.sdf, stepScale);
     r.result = add3(r.result, smul3(step, r.dir));
-    r.sdf = read_sdf_interp<VR>(m, gv, r.result, c, valid);
+    r.sdf = read_sdf_interp<VR>(m, gv, r.result, c);
     step = fm(r.sdf, stepScale);
     r.result = add3(r.result, smul3(step, r.dir));
     f3 n;
@@ -595,10 +714,15 @@ __device__ __forceinline__ void raycast_body(const BlockCtx& ctx, MapView m, flo
         atomicMax(&m.rc_cost[s_tile[wq]], (uint32_t)min(clock64() - s_t0[wq], 0xffffffffLL));
 }
 
-// Nine CTAs of 128 threads per SM (56 registers; the compiler's own choice
-// of 72 leaves seven, and the tail of the launch is longer).
+// Bound by latency: a ray is a chain of look-ups and voxel loads, and the warps
+// of an SM cover about half of it.  640x480 / 1280x960 live frames 45 / 112 us
+// (57 / 155 when the normal's samples were read one after another, see
+// read_normal).  Eight CTAs of 128 threads per SM (64 registers): with nine
+// (56, spills) 46 / 117 us, with seven 44 / 114.  Following a ray through
+// missing blocks with two to four look-ups ahead of it cost more (57 us): the
+// warp's other lanes wait, and few rays pass many missing blocks.
 template <class VR>
-__global__ void __launch_bounds__(128, 9) k_raycast(MapView m, float4* __restrict__ vmap, float4* __restrict__ nmap,
+__global__ void __launch_bounds__(128, 8) k_raycast(MapView m, float4* __restrict__ vmap, float4* __restrict__ nmap,
                                                  int vp, int W, int H, Intr k, const DevPose* __restrict__ posep,
                                                  const int* __restrict__ skip) {
     raycast_body<VR>(own_ctx(), m, vmap, nmap, vp, W, H, k, posep, skip);
