@@ -480,65 +480,164 @@ __global__ void k_fuse_records(MapView m, const float* __restrict__ raw, int rp,
                     m.frec + (size_t)y * W + x, m.fcol + (size_t)y * W + x);
 }
 
-// Fusion::integrateColor (FuseMap.cu:140-191) for one voxel, every operation
-// rounded as the reference's float expression.  rec / col: the frame's fusion
-// records (W wide).  Returns true when the voxel changed.
-__device__ __forceinline__ bool integrate_voxel(Voxel& vox, int vx, int vy, int vz, const float4* __restrict__ rec,
-                                                const uint32_t* __restrict__ col, int W, int H, const Intr& k,
-                                                const DevPose& P, const MapGeom& g,
-                                                const float* __restrict__ div255) {
-    f3 pos = mk3(fm((float)vx, g.voxel_size), fm((float)vy, g.voxel_size), fm((float)vz, g.voxel_size));
-    pos = mv(P.Rinv, sub3(pos, P.t));
-    // the two quotients by pos.z share one reciprocal (fd_rcp); positions are
-    // sums of products of voxel-scale values, normal floats or exactly zero
-    float pu, pv;
-    if (pos.z != 0.0f) {
-        const float rz = __frcp_rn(pos.z);
-        pu = fa(fd_rcp(fm(k.fx, pos.x), pos.z, rz), k.cx);
-        pv = fa(fd_rcp(fm(k.fy, pos.y), pos.z, rz), k.cy);
-    } else {
-        pu = fa(fd(fm(k.fx, pos.x), pos.z), k.cx);
-        pv = fa(fd(fm(k.fy, pos.y), pos.z), k.cy);
+// Two floats in one register pair (Blackwell's packed FP32: one issue slot for
+// both lanes of an operation; each lane is rounded as its scalar form).
+using f2 = unsigned long long;
+__device__ __forceinline__ f2 f2_of(float a, float b) {
+    f2 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+    return r;
+}
+__device__ __forceinline__ float f2_lo(f2 v) {
+    float a, b;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v));
+    return a;
+}
+__device__ __forceinline__ float f2_hi(f2 v) {
+    float a, b;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v));
+    return b;
+}
+__device__ __forceinline__ f2 f2_add(f2 a, f2 b) {
+    f2 r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ f2 f2_fma(f2 a, f2 b, f2 c) {
+    f2 r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+
+// Per-launch constants of integrate_pair, both lanes equal.  nz holds -0.0f: a
+// product is written a b + (-0), which rounds as a b alone, because the
+// compiler merges a packed multiply and the add that follows it into one FMA.
+struct PairConst {
+    f2 nz, m1;
+    f2 nfx, nfy, cx, cy;     // -fx, -fy
+    f2 nT, rT;               // -trunc_dist, 1 / trunc_dist
+};
+__device__ __forceinline__ f2 f2_mul(f2 a, f2 b, const PairConst& pc) { return f2_fma(a, b, pc.nz); }
+
+__device__ __forceinline__ PairConst pair_const(const Intr& k, float T, int W) {
+    PairConst pc;
+    // not a constant the compiler can fold (W > 0 at every launch)
+    const float nz = __uint_as_float(0x80000000u | (W < 0 ? 1u : 0u));
+    const float rT = __frcp_rn(T);
+    pc.nz = f2_of(nz, nz);
+    pc.m1 = f2_of(-1.0f, -1.0f);
+    pc.nfx = f2_of(-k.fx, -k.fx);
+    pc.nfy = f2_of(-k.fy, -k.fy);
+    pc.cx = f2_of(k.cx, k.cx);
+    pc.cy = f2_of(k.cy, k.cy);
+    pc.nT = f2_of(-T, -T);
+    pc.rT = f2_of(rT, rT);
+    return pc;
+}
+
+// Fusion::integrateColor (FuseMap.cu:140-191) for the voxels (vx, vy, vz) and
+// (vx + 1, vy, vz), every operation rounded as the reference's float
+// expression.  rec / col: the frame's fusion records (W wide).  Returns true
+// when a voxel changed.
+//
+// Quotients by one divisor share its reciprocal (fd_rcp's correction step
+// without its test for a zero remainder, which only keeps the sign of a zero
+// quotient: a projected coordinate adds the centre, a normal's component adds
+// a positive term, and a signed distance is never -0).  Some are computed
+// negated, so that the packed forms need no negation: -(a b) and (-a) b are
+// the same bits.
+//
+// Bound by issue slots (74 % busy at 20 k blocks, DRAM at 1.2 TB/s): two voxels
+// a thread share the packed operations.  20 k blocks at 640x480 111 -> 95 us,
+// a live 640x480 frame 37 -> 31, against one scalar voxel after the other.
+__device__ __forceinline__ bool integrate_pair(Voxel& v0, Voxel& v1, int vx, int vy, int vz,
+                                               const float4* __restrict__ rec, const uint32_t* __restrict__ col,
+                                               int W, int H, const Intr& k, const DevPose& P, const MapGeom& g,
+                                               const float* __restrict__ div255, const PairConst& pc) {
+    const float wx0 = fs(fm((float)vx, g.voxel_size), P.t.x), wx1 = fs(fm((float)(vx + 1), g.voxel_size), P.t.x);
+    const float wy = fs(fm((float)vy, g.voxel_size), P.t.y), wz = fs(fm((float)vz, g.voxel_size), P.t.z);
+    const f3 p0 = mv(P.Rinv, mk3(wx0, wy, wz)), p1 = mv(P.Rinv, mk3(wx1, wy, wz));
+    const f2 px = f2_of(p0.x, p1.x), py = f2_of(p0.y, p1.y), pz = f2_of(p0.z, p1.z);
+    // u, v = f p / z + c: -a = (-f) p, q = (-a)(-1/z), q z - a = -(remainder)
+    f2 pu, pv;
+    {
+        const f2 nrz = f2_of(__frcp_rn(-p0.z), __frcp_rn(-p1.z));
+        const f2 nax = f2_mul(pc.nfx, px, pc), nay = f2_mul(pc.nfy, py, pc);
+        const f2 qx = f2_mul(nax, nrz, pc), qy = f2_mul(nay, nrz, pc);
+        pu = f2_add(f2_fma(f2_fma(qx, pz, nax), nrz, qx), pc.cx);
+        pv = f2_add(f2_fma(f2_fma(qy, pz, nay), nrz, qy), pc.cy);
     }
-    const int u = __float2int_rz(pu), v = __float2int_rz(pv);  // make_int2(float2)
-    if (u < 0 || v < 0 || u >= W || v >= H) return false;
-    const int pix = v * W + u;
-    const float4 r = __ldg(rec + pix);   // r.x: the raw depth, NaN where the pixel is skipped
-    const float thresh = g.trunc_dist;
-    float sdf = fs(r.x, pos.z);
-    if (!(sdf >= -thresh)) return false;
-    sdf = fminf(1.0f, fd_rcp(sdf, thresh, __frcp_rn(thresh)));
+    int u0 = __float2int_rz(f2_lo(pu)), u1 = __float2int_rz(f2_hi(pu));   // make_int2(float2)
+    int w0 = __float2int_rz(f2_lo(pv)), w1 = __float2int_rz(f2_hi(pv));
+    if (p0.z == 0.0f) {   // the IEEE quotients by zero
+        u0 = __float2int_rz(fa(fd(fm(k.fx, p0.x), p0.z), k.cx));
+        w0 = __float2int_rz(fa(fd(fm(k.fy, p0.y), p0.z), k.cy));
+    }
+    if (p1.z == 0.0f) {
+        u1 = __float2int_rz(fa(fd(fm(k.fx, p1.x), p1.z), k.cx));
+        w1 = __float2int_rz(fa(fd(fm(k.fy, p1.y), p1.z), k.cy));
+    }
+    const bool in0 = (unsigned)u0 < (unsigned)W && (unsigned)w0 < (unsigned)H;
+    const bool in1 = (unsigned)u1 < (unsigned)W && (unsigned)w1 < (unsigned)H;
+    if (!in0 && !in1) return false;
+    const int pix0 = in0 ? w0 * W + u0 : 0, pix1 = in1 ? w1 * W + u1 : 0;
+    const float4 r0 = __ldg(rec + pix0), r1 = __ldg(rec + pix1);   // .x: the raw depth, NaN where the pixel is skipped
+    const uint32_t c0 = __ldg(col + pix0), c1 = __ldg(col + pix1);
+    const float s0 = fs(r0.x, p0.z), s1 = fs(r1.x, p1.z);
+    const bool on0 = in0 && s0 >= -g.trunc_dist, on1 = in1 && s1 >= -g.trunc_dist;
+    if (!on0 && !on1) return false;
+    f2 sd = f2_of(s0, s1);
+    {
+        const f2 q = f2_mul(sd, pc.rT, pc);
+        sd = f2_fma(f2_fma(q, pc.nT, sd), pc.rT, q);
+    }
+    const float sdf0 = fminf(1.0f, f2_lo(sd)), sdf1 = fminf(1.0f, f2_hi(sd));
+    sd = f2_of(sdf0, sdf1);
     // w = nl * normalised(float4(pos, 1)): the dot runs over all four lanes
     // (the normal's w lane is 1, so its term is 1 / nrm)
-    const float nrm = fsq(fa(fa(fa(fm(pos.x, pos.x), fm(pos.y, pos.y)), fm(pos.z, pos.z)), 1.0f));
-    // nrm >= 1: the four quotients share its reciprocal (1 / nrm is that
-    // reciprocal itself)
-    const float rn = __frcp_rn(nrm);
-    const float w = fa(fa(fa(fm(r.y, fd_rcp(pos.x, nrm, rn)), fm(r.z, fd_rcp(pos.y, nrm, rn))),
-                          fm(r.w, fd_rcp(pos.z, nrm, rn))),
-                       rn);
-    const uint32_t c = __ldg(col + pix);
-    const uint32_t cr = c & 255u, cg = (c >> 8) & 255u, cb = c >> 16;
-    if (vox.weight == 0) {
-        vox.sdf = sdf;
-        vox.weight = 1;
-        vox.r = (unsigned char)cr;
-        vox.g = (unsigned char)cg;
-        vox.b = (unsigned char)cb;
-        return true;
-    }
-    const float a = fm(w, 0.2f), oa = fs(1.0f, a);
-    const float W0 = (float)vox.weight;
+    const f2 nn = f2_add(f2_add(f2_add(f2_mul(px, px, pc), f2_mul(py, py, pc)), f2_mul(pz, pz, pc)),
+                         f2_of(1.0f, 1.0f));
+    const float n0 = fsq(f2_lo(nn)), n1 = fsq(f2_hi(nn));
+    const float rn0 = __frcp_rn(n0), rn1 = __frcp_rn(n1);
+    const f2 nrm = f2_of(n0, n1), nrn = f2_of(-rn0, -rn1);
+    // minus each component's term (-q = p (-1/n), p - q n, -(q + r / n))
+    auto term = [&](f2 p, float a, float b) {
+        const f2 nq = f2_mul(p, nrn, pc);
+        return f2_mul(f2_of(a, b), f2_fma(f2_fma(nq, nrm, p), nrn, nq), pc);
+    };
+    const f2 nsum = f2_add(f2_add(term(px, r0.y, r1.y), term(py, r0.z, r1.z)), term(pz, r0.w, r1.w));
+    const f2 w = f2_fma(nsum, pc.m1, f2_of(rn0, rn1));
+    const f2 a = f2_mul(w, f2_of(0.2f, 0.2f), pc), oa = f2_fma(a, pc.m1, f2_of(1.0f, 1.0f));
+    const f2 W0 = f2_of((float)v0.weight, (float)v1.weight);
     // (float)c / 255 of a byte c: the table holds those 256 IEEE quotients
-    float rr = fm(fa(fm(a, div255[cr]), fm(oa, div255[vox.r])), 255.f);
-    float gg = fm(fa(fm(a, div255[cg]), fm(oa, div255[vox.g])), 255.f);
-    float bb = fm(fa(fm(a, div255[cb]), fm(oa, div255[vox.b])), 255.f);
-    vox.sdf = fd(fa(fm(vox.sdf, W0), fm(w, sdf)), fa(W0, w));
-    vox.weight = (unsigned char)min(255, (int)vox.weight + 1);
-    // make_uchar3(float3): truncate to int, then to the low byte
-    vox.r = (unsigned char)__float2int_rz(rr);
-    vox.g = (unsigned char)__float2int_rz(gg);
-    vox.b = (unsigned char)__float2int_rz(bb);
+    auto blend = [&](uint32_t ca, uint32_t cb, uint32_t va, uint32_t vb) {
+        return f2_mul(f2_add(f2_mul(a, f2_of(div255[ca], div255[cb]), pc),
+                             f2_mul(oa, f2_of(div255[va], div255[vb]), pc)),
+                      f2_of(255.f, 255.f), pc);
+    };
+    const f2 rr = blend(c0 & 255u, c1 & 255u, v0.r, v1.r);
+    const f2 gg = blend((c0 >> 8) & 255u, (c1 >> 8) & 255u, v0.g, v1.g);
+    const f2 bb = blend(c0 >> 16, c1 >> 16, v0.b, v1.b);
+    const f2 num = f2_add(f2_mul(f2_of(v0.sdf, v1.sdf), W0, pc), f2_mul(w, sd, pc)), den = f2_add(W0, w);
+    // the first observation, else the running average; make_uchar3(float3):
+    // truncate to int, then to the low byte
+    auto put = [](Voxel& v, float sdf, uint32_t c, float n, float d, float r, float gr, float b) {
+        if (v.weight == 0) {
+            v.sdf = sdf;
+            v.weight = 1;
+            v.r = (unsigned char)(c & 255u);
+            v.g = (unsigned char)((c >> 8) & 255u);
+            v.b = (unsigned char)(c >> 16);
+        } else {
+            v.sdf = fd(n, d);
+            v.weight = (unsigned char)min(255, (int)v.weight + 1);
+            v.r = (unsigned char)__float2int_rz(r);
+            v.g = (unsigned char)__float2int_rz(gr);
+            v.b = (unsigned char)__float2int_rz(b);
+        }
+    };
+    if (on0) put(v0, sdf0, c0, f2_lo(num), f2_lo(den), f2_lo(rr), f2_lo(gg), f2_lo(bb));
+    if (on1) put(v1, sdf1, c1, f2_hi(num), f2_hi(den), f2_hi(rr), f2_hi(gg), f2_hi(bb));
     return true;
 }
 
@@ -551,6 +650,7 @@ __device__ __forceinline__ void integrate_body(const BlockCtx& ctx, MapView m, i
     s_div255[threadIdx.x] = fd((float)threadIdx.x, 255.f);   // blockDim.x == 256
     __syncthreads();
     const DevPose P = *posep;
+    const PairConst pc = pair_const(k, m.g.trunc_dist, W);
     const int n = min(m.ctr->n_visible, m.NS);
     const int t = threadIdx.x;
     const int lx = (2 * t) & 7, ly = (t >> 2) & 7, lz = t >> 5;
@@ -574,9 +674,7 @@ __device__ __forceinline__ void integrate_body(const BlockCtx& ctx, MapView m, i
             raw_nx = *((const uint4*)(m.voxels + (size_t)e_nx.ptr * 512) + t);
         }
         Voxel v0 = *(const Voxel*)&raw2.x, v1 = *(const Voxel*)&raw2.z;
-        bool c0 = integrate_voxel(v0, vx, vy, vz, rec, col, W, H, k, P, m.g, s_div255);
-        bool c1 = integrate_voxel(v1, vx + 1, vy, vz, rec, col, W, H, k, P, m.g, s_div255);
-        if (c0 || c1) {
+        if (integrate_pair(v0, v1, vx, vy, vz, rec, col, W, H, k, P, m.g, s_div255, pc)) {
             uint4 o;
             *(Voxel*)&o.x = v0;
             *(Voxel*)&o.z = v1;
