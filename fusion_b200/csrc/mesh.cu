@@ -23,12 +23,12 @@
 // classic table leaves holes on some ambiguous faces).  Triangles wind so
 // that their right-hand normal points to the negative side.
 //
-// GPU layout: CTAs of 288 threads walk the allocated blocks, two voxels per
-// thread.  A CTA stages the 11^3 voxel region the block's cubes and gradients
-// read (local coordinates -1 .. 9) in shared memory, so each voxel costs
-// shared-memory reads instead of the reference's 32 hash lookups; the 27
-// blocks it comes from are looked up by a warp of their own while the block
-// before is worked on.  Two passes make the output deterministic: triangle
+// GPU layout: CTAs of 288 threads walk the allocated blocks.  A CTA stages the
+// 11^3 voxel region the block's cubes and gradients read (local coordinates
+// -1 .. 9) in shared memory, instead of the reference's 32 hash lookups per
+// voxel; the 27 blocks it comes from are looked up by a warp of their own while
+// the block before is worked on.  Which voxels hold surface is found a row of
+// eight at a time, from a word of bits per row of the region.  Two passes make the output deterministic: triangle
 // counts per block, an exclusive scan, then every block writes its triangles
 // at its offset in voxel order.  In the second pass the block's triangles are
 // listed first and then every thread makes a vertex (few voxels of a block
@@ -163,8 +163,10 @@ int build_case(int ci, int8_t tri[16]) {
     return n;
 }
 
-__constant__ int8_t c_tri[256][16];
-__constant__ int c_ntri[256];
+// (global memory, copied to shared memory by each CTA: constant memory serves
+// one address at a time, and every lane reads its own case)
+__device__ __align__(16) int8_t c_tri[256][16];
+__device__ __align__(16) uint8_t c_ntri[256];
 
 static int build_tables(int8_t tri[256][16], int ntri[256]) {
     for (int ci = 0; ci < 256; ++ci) {
@@ -184,9 +186,11 @@ static int ensure_tables() {
     if (done[dev]) return FB_OK;
     int8_t tri[256][16];
     int ntri[256];
+    uint8_t n8[256];
     if (build_tables(tri, ntri) != FB_OK) return FB_EINVAL;
+    for (int i = 0; i < 256; ++i) n8[i] = (uint8_t)ntri[i];
     if (cudaMemcpyToSymbol(c_tri, tri, sizeof tri) != cudaSuccess) return FB_ECUDA;
-    if (cudaMemcpyToSymbol(c_ntri, ntri, sizeof ntri) != cudaSuccess) return FB_ECUDA;
+    if (cudaMemcpyToSymbol(c_ntri, n8, sizeof n8) != cudaSuccess) return FB_ECUDA;
     done[dev] = true;
     return FB_OK;
 }
@@ -195,24 +199,27 @@ static int ensure_tables() {
 
 constexpr int kMeshWork = 256;                     // threads on voxels and vertices ...
 constexpr int kMeshThreads = kMeshWork + 32;       // ... and the warp that looks blocks up
-constexpr int kMeshCtas = 7;                       // resident per SM
+constexpr int kMeshCtas = 7;                       // resident per SM (five: 97 us for the triangles, seven: 95)
 constexpr int kHalo = 11;                          // local coordinates -1 .. 9
-constexpr int kRegion = kHalo * kHalo * kHalo;     // 1331
-constexpr int kColSide = 9;                        // colours of local 0 .. 8
+constexpr int kRows = kHalo * kHalo;
+constexpr int kRegion = kHalo * kRows;             // 1331
+constexpr int kEach = (kRegion + kMeshWork - 1) / kMeshWork;
 
 struct MeshSmem {
     int ptr[2][27];              // blocks around one, (dx + 1) + 3 (dy + 1) + 9 (dz + 1): this block's, the next one's
     int3 pos[2];                 // their block coordinates
     float sdf[kRegion];          // NaN where no block (Voxel(), DeviceMap.h:63-65)
-    int warp_sum[kMeshWork / 32];
+    uint32_t row[kRows];         // the rows' voxels as bits (see row_bits)
+    alignas(16) uint8_t ntri[256];
 };
 // The second pass's additions.
 struct EmitSmem {
-    uint32_t rgb[kColSide * kColSide * kColSide];
+    uint32_t rgb[kRegion];
     uint16_t tri[512 * 5];       // the block's triangles in order: voxel | triangle of the voxel << 9
     uint8_t cubes[512];          // the voxels' cases
     float v[kMeshWork * 3], n[kMeshWork * 3];
     uint8_t c[kMeshWork * 3];
+    alignas(16) int8_t table[256][16];
 };
 
 // Barrier of the voxel threads alone (the look-up warp does not take part).
@@ -242,26 +249,55 @@ __device__ __forceinline__ void look_up(const MapView& m, int blk, int lane, Mes
     if (lane == 0) s.pos[buf] = make_int3(self.x, self.y, self.z);
 }
 
-// The region of the block whose neighbours are in s.ptr[buf] (voxel threads):
-// a thread's voxels are loaded together, then stored.
+// Where a thread's region voxels lie, the same for every block: slot in s.ptr
+// << 9 | voxel, or -1 beyond the region.
+struct Region {
+    int at[kEach];
+};
+__device__ __forceinline__ Region region_of(int t) {
+    Region g;
+#pragma unroll
+    for (int q = 0; q < kEach; ++q) {
+        const int r = t + q * kMeshWork;
+        const int lx = r % kHalo - 1, ly = (r / kHalo) % kHalo - 1, lz = r / kRows - 1;
+        const int ox = lx < 0 ? -1 : (lx > 7 ? 1 : 0);
+        const int oy = ly < 0 ? -1 : (ly > 7 ? 1 : 0);
+        const int oz = lz < 0 ? -1 : (lz > 7 ? 1 : 0);
+        g.at[q] = r < kRegion ? ((ox + 1) + 3 * (oy + 1) + 9 * (oz + 1)) << 9 |
+                                    ((lz - 8 * oz) * 64 + (ly - 8 * oy) * 8 + (lx - 8 * ox))
+                              : -1;
+    }
+    return g;
+}
+
+// A row's eleven voxels (local x = -1 .. 9): bits 0-10 the TSDF is not NaN,
+// 11-19 (local 0 .. 8) nor exactly 1, 20-28 (local 0 .. 8) it is negative.
+__device__ __forceinline__ uint32_t row_bits(const float* sdf) {
+    uint32_t b = 0;
+#pragma unroll
+    for (int u = 0; u < kHalo; ++u) {
+        const float v = sdf[u];
+        if (!isnan(v)) b |= 1u << u;
+        if (u >= 1 && u <= 9) {
+            if (!isnan(v) && v != 1.0f) b |= 1u << (10 + u);
+            if (v < 0) b |= 1u << (19 + u);
+        }
+    }
+    return b;
+}
+
+// The region of the block whose neighbours are in s.ptr[buf] and its rows'
+// bits (voxel threads): a thread's voxels are loaded together, then stored.
 template <bool kColour>
-__device__ __forceinline__ void stage_block(const MapView& m, MeshSmem& s, uint32_t* rgb, int buf) {
-    constexpr int kEach = (kRegion + kMeshWork - 1) / kMeshWork;
+__device__ __forceinline__ void stage_block(const MapView& m, const Region& g, MeshSmem& s, uint32_t* rgb, int buf) {
     float sdf[kEach];
     uint32_t col[kEach];
 #pragma unroll
     for (int q = 0; q < kEach; ++q) {
-        const int r = threadIdx.x + q * kMeshWork;
         sdf[q] = qnan();
         col[q] = 0;
-        if (r >= kRegion) continue;
-        const int u = r % kHalo, v = (r / kHalo) % kHalo, w = r / (kHalo * kHalo);
-        const int lx = u - 1, ly = v - 1, lz = w - 1;
-        const int ox = lx < 0 ? -1 : (lx > 7 ? 1 : 0);
-        const int oy = ly < 0 ? -1 : (ly > 7 ? 1 : 0);
-        const int oz = lz < 0 ? -1 : (lz > 7 ? 1 : 0);
-        const int p = s.ptr[buf][(ox + 1) + 3 * (oy + 1) + 9 * (oz + 1)];
-        const int idx = (lz - 8 * oz) * 64 + (ly - 8 * oy) * 8 + (lx - 8 * ox);
+        if (g.at[q] < 0) continue;
+        const int p = s.ptr[buf][g.at[q] >> 9], idx = g.at[q] & 511;
         if (p < 0) continue;
         if (m.cvox) {
             const uint8_t* blk = m.cvox + (size_t)p * kCBlockBytes;
@@ -277,52 +313,52 @@ __device__ __forceinline__ void stage_block(const MapView& m, MeshSmem& s, uint3
     }
 #pragma unroll
     for (int q = 0; q < kEach; ++q) {
-        const int r = threadIdx.x + q * kMeshWork;
-        if (r >= kRegion) continue;
-        s.sdf[r] = sdf[q];
-        if (kColour) {
-            const int u = r % kHalo, v = (r / kHalo) % kHalo, w = r / (kHalo * kHalo);
-            if (u >= 1 && u <= kColSide && v >= 1 && v <= kColSide && w >= 1 && w <= kColSide)
-                rgb[(u - 1) + kColSide * (v - 1) + kColSide * kColSide * (w - 1)] = col[q];
-        }
+        if (g.at[q] < 0) continue;
+        s.sdf[threadIdx.x + q * kMeshWork] = sdf[q];
+        if (kColour) rgb[threadIdx.x + q * kMeshWork] = col[q];
     }
+    work_barrier();
+    if (threadIdx.x < kRows) s.row[threadIdx.x] = row_bits(s.sdf + kHalo * threadIdx.x);
     work_barrier();
 }
 
 // Region index of local voxel (x, y, z), each in -1 .. 9.
-__device__ __forceinline__ int rix(int x, int y, int z) { return (x + 1) + kHalo * (y + 1) + kHalo * kHalo * (z + 1); }
+__device__ __forceinline__ int rix(int x, int y, int z) { return (x + 1) + kHalo * (y + 1) + kRows * (z + 1); }
 
-// readVertexAndColor + readNormal's NaN tests + the case index
-// (MeshScene.cu:43-183).  -1: no cube or no surface in it.
-__device__ __forceinline__ int classify(const MeshSmem& s, int x, int y, int z) {
-    float sd[8];
-#pragma unroll
-    for (int i = 0; i < 8; ++i) {
-        sd[i] = s.sdf[rix(x + corner_dx(i), y + corner_dy(i), z + corner_dz(i))];
-        if (sd[i] == 1.0f || isnan(sd[i])) return -1;
-    }
-    // the 24 gradient neighbours outside the cube
-#pragma unroll
-    for (int i = 0; i < 8; ++i) {
-        const int cx = x + corner_dx(i), cy = y + corner_dy(i), cz = z + corner_dz(i);
-        const float a = s.sdf[rix(corner_dx(i) ? cx + 1 : cx - 1, cy, cz)];
-        const float b = s.sdf[rix(cx, corner_dy(i) ? cy + 1 : cy - 1, cz)];
-        const float c = s.sdf[rix(cx, cy, corner_dz(i) ? cz + 1 : cz - 1)];
-        if (isnan(a) || isnan(b) || isnan(c)) return -1;
-    }
-    int ci = 0;
-#pragma unroll
-    for (int i = 0; i < 8; ++i)
-        if (sd[i] < 0) ci |= 1 << i;
-    return (ci == 0 || ci == 255) ? -1 : ci;
+// The cubes of a block's row (y, z) that hold surface, a bit each, and the
+// row's four corner rows: readVertexAndColor + readNormal's NaN tests
+// (MeshScene.cu:43-183) for the row's eight voxels together.
+struct CubeRow {
+    uint32_t mask, r00, r10, r01, r11;   // rdydz: rows (y + dy, z + dz)
+};
+__device__ __forceinline__ CubeRow cube_row(const MeshSmem& s, int y, int z) {
+    const uint32_t* r = s.row + (y + 1) + kHalo * (z + 1);
+    CubeRow c;
+    c.r00 = r[0];
+    c.r10 = r[1];
+    c.r01 = r[kHalo];
+    c.r11 = r[kHalo + 1];
+    const uint32_t all = c.r00 & c.r10 & c.r01 & c.r11, any = c.r00 | c.r10 | c.r01 | c.r11;
+    // the 24 gradient neighbours outside the cube: x - 1 and x + 2 of the four
+    // rows, and x and x + 1 of the rows beyond them in y and in z
+    const uint32_t out = r[-1] & r[2] & r[kHalo - 1] & r[kHalo + 2] & r[-kHalo] & r[-kHalo + 1] & r[2 * kHalo] &
+                         r[2 * kHalo + 1];
+    const uint32_t ok = all >> 11, nn = out >> 1, na = all >> 20, no = any >> 20;
+    c.mask = ok & (ok >> 1) & all & (all >> 3) & nn & (nn >> 1) & (no | (no >> 1)) & ~(na & (na >> 1)) & 0xffu;
+    return c;
+}
+// The case index of the row's cube x (bit i: corner i is negative).
+__device__ __forceinline__ int cube_case(const CubeRow& c, int x) {
+    const uint32_t a = c.r00 >> (20 + x), b = c.r10 >> (20 + x), d = c.r01 >> (20 + x), e = c.r11 >> (20 + x);
+    return (a & 3) | (b & 2) << 1 | (b & 1) << 3 | (d & 3) << 4 | (e & 2) << 5 | (e & 1) << 7;
 }
 
-// interp (MeshScene.cu:142-150); the thresholds compare in double, as the
-// reference's float-vs-double-literal comparisons do.
+// interp (MeshScene.cu:142-150).  The reference compares in double; for a
+// float f, (double)f < 1e-6 exactly when f <= 1e-6f (the float below 1e-6).
 __device__ __forceinline__ float interp(float v1, float v2) {
-    if ((double)fabsf(fs(0.f, v1)) < 1e-6) return 0.f;
-    if ((double)fabsf(fs(0.f, v2)) < 1e-6) return 1.f;
-    if ((double)fabsf(fs(v1, v2)) < 1e-6) return 0.f;
+    if (fabsf(v1) <= 1e-6f) return 0.f;
+    if (fabsf(v2) <= 1e-6f) return 1.f;
+    if (fabsf(fs(v1, v2)) <= 1e-6f) return 0.f;
     return fd(fs(0.f, v1), fs(v2, v1));
 }
 
@@ -359,28 +395,14 @@ __device__ __forceinline__ void edge_vertex(const MeshSmem& s, const uint32_t* r
     N[0] = fd(n.x, len);
     N[1] = fd(n.y, len);
     N[2] = fd(n.z, len);
-    const uint32_t ca = rgb[(x + ax) + kColSide * (y + ay) + kColSide * kColSide * (z + az)];
-    const uint32_t cb =
-        rgb[(x + corner_dx(b)) + kColSide * (y + corner_dy(b)) + kColSide * kColSide * (z + corner_dz(b))];
+    const uint32_t ca = rgb[rix(x + ax, y + ay, z + az)];
+    const uint32_t cb = rgb[rix(x + corner_dx(b), y + corner_dy(b), z + corner_dz(b))];
     const int k = (int)val;
 #pragma unroll
     for (int c = 0; c < 3; ++c) {
         const uint8_t ua = (uint8_t)(ca >> (8 * c)), ub = (uint8_t)(cb >> (8 * c));
         C[c] = (uint8_t)(ua + (uint8_t)((uint8_t)(ub - ua) * k));
     }
-}
-
-// Inclusive prefix of v in the warp; the warp's sum into s.warp_sum.
-__device__ __forceinline__ int warp_prefix(int v, MeshSmem& s) {
-    const int lane = threadIdx.x & 31;
-    int incl = v;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        const int y = __shfl_up_sync(0xffffffffu, incl, o);
-        if (lane >= o) incl += y;
-    }
-    if (lane == 31) s.warp_sum[threadIdx.x >> 5] = incl;
-    return incl;
 }
 
 // The walk both passes share: CTA c takes blocks c, c + grid, ...; body(blk,
@@ -400,37 +422,31 @@ __device__ __forceinline__ void walk_blocks(const MapView& m, int n, MeshSmem& s
     }
 }
 
-// Triangle counts of the allocated blocks: 45 us for 10 800 blocks (one CTA of
-// 512 threads per block, each beginning with its own chain of list, entry and
-// buckets: 83 us).  Bound by instruction issue: four to seven CTAs per SM
-// take the same time.
-__global__ void __launch_bounds__(kMeshThreads, kMeshCtas) k_mesh_count(MapView m, uint32_t* counts) {
+// Triangle counts of the allocated blocks.  The cubes are found a row of eight
+// at a time from bits (cube_row): two warps then walk the few that hold
+// surface.  10 800 blocks: 29 us; classifying every voxel from its 32 values
+// took 45, and one CTA of 512 threads per block, each beginning with its own
+// chain of list, entry and buckets, 83.
+__global__ void __launch_bounds__(kMeshThreads, kMeshCtas) k_mesh_count(MapView m, uint2* counts) {
     __shared__ MeshSmem s;
-    const int n = min(m.ctr->n_alloc, m.NS);
+    const int n = min(m.ctr->n_alloc, m.NS), t = threadIdx.x;
+    const Region g = region_of(t);
+    if (t < 64) reinterpret_cast<uint32_t*>(s.ntri)[t] = reinterpret_cast<const uint32_t*>(c_ntri)[t];
     walk_blocks(m, n, s, [&](int blk, int buf) {
-        stage_block<false>(m, s, nullptr, buf);
-        const int t = threadIdx.x, x = t & 7, y = (t >> 3) & 7, z = t >> 6;
+        stage_block<false>(m, g, s, nullptr, buf);
+        if (t >= 64) return;
+        const CubeRow c = cube_row(s, t & 7, t >> 3);
         int nt = 0;
-#pragma unroll
-        for (int h = 0; h < 2; ++h) {
-            const int ci = classify(s, x, y, z + 4 * h);
-            if (ci >= 0) nt += c_ntri[ci];
-        }
+        for (uint32_t k = c.mask; k; k &= k - 1) nt += s.ntri[cube_case(c, __ffs(k) - 1)];
+        __syncwarp();
         nt = __reduce_add_sync(0xffffffffu, nt);
-        if ((t & 31) == 0) s.warp_sum[t >> 5] = nt;
-        work_barrier();
-        if (t == 0) {
-            int total = 0;
-#pragma unroll
-            for (int w = 0; w < kMeshWork / 32; ++w) total += s.warp_sum[w];
-            counts[blk] = (uint32_t)total;
-        }
+        if ((t & 31) == 0) reinterpret_cast<uint32_t*>(counts)[2 * blk + (t >> 5)] = (uint32_t)nt;
     });
 }
 
-// Exclusive scan of the n counts into offsets[0 .. n] (offsets[n] = *total): one
+// Exclusive scan of the n counts (two halves each) into offsets[0 .. n] (offsets[n] = *total): one
 // CTA, each thread a run of consecutive counts.
-__global__ void __launch_bounds__(1024) k_mesh_scan(const MapView m, const uint32_t* counts,
+__global__ void __launch_bounds__(1024) k_mesh_scan(const MapView m, const uint2* counts,
                                                     unsigned long long* offsets, unsigned long long* total) {
     __shared__ unsigned long long warp_sum[32];
     const int n = min(m.ctr->n_alloc, m.NS);
@@ -438,7 +454,7 @@ __global__ void __launch_bounds__(1024) k_mesh_scan(const MapView m, const uint3
     const int per = (n + 1023) / 1024, i0 = min(n, t * per), i1 = min(n, i0 + per);
     unsigned long long sum = 0;
 #pragma unroll 8
-    for (int i = i0; i < i1; ++i) sum += counts[i];
+    for (int i = i0; i < i1; ++i) sum += counts[i].x + counts[i].y;
     unsigned long long incl = sum;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
@@ -452,7 +468,7 @@ __global__ void __launch_bounds__(1024) k_mesh_scan(const MapView m, const uint3
 #pragma unroll 8
     for (int i = i0; i < i1; ++i) {
         offsets[i] = run;
-        run += counts[i];
+        run += counts[i].x + counts[i].y;
     }
     if (t == 1023) offsets[n] = *total = run;
 }
@@ -474,47 +490,59 @@ __device__ __forceinline__ void copy_out(uint8_t* dst, const uint8_t* src, int b
 
 // The triangles.  One voxel per thread and its triangles one after another
 // left most lanes idle and wrote 4 bytes every 12 (10 800 blocks, 880 000
-// triangles: 211 us); here the block's vertices are dealt to its threads
-// (116 us, bound by instruction issue).
+// triangles: 211 us).  The block's triangles are listed from its rows' bits and
+// its vertices are dealt to its threads: 95 us (116 with every voxel classified
+// again, the tables in constant memory and the region's indices recomputed).
 __global__ void __launch_bounds__(kMeshThreads, kMeshCtas)
     k_mesh_emit(MapView m, const unsigned long long* offsets, unsigned long long cap, float* V, float* N, uint8_t* C) {
     __shared__ MeshSmem s;
     __shared__ EmitSmem em;
-    const int n = min(m.ctr->n_alloc, m.NS);
+    const int n = min(m.ctr->n_alloc, m.NS), t = threadIdx.x;
+    const Region g = region_of(t);
+    if (t < 64) reinterpret_cast<uint32_t*>(s.ntri)[t] = reinterpret_cast<const uint32_t*>(c_ntri)[t];
+    if (t < 256) reinterpret_cast<uint4*>(em.table)[t] = reinterpret_cast<const uint4*>(c_tri)[t];
     walk_blocks(m, n, s, [&](int blk, int buf) {
         const unsigned long long first = offsets[blk];
         const int total = (int)min(offsets[blk + 1] - first, first < cap ? cap - first : 0ull);
         if (total == 0) return;   // uniform: no surface in this block, or no room left
-        stage_block<true>(m, s, em.rgb, buf);
-        // list the triangles in voxel order: voxels t of the lower half, then
-        // of the upper (voxel index = t + 256 h)
-        const int t = threadIdx.x, x = t & 7, y = (t >> 3) & 7, z = t >> 6;
-        int base = 0;
+        stage_block<true>(m, g, s, em.rgb, buf);
+        // list the triangles in voxel order: row by row (thread t < 64: row
+        // (t & 7, t >> 3)), the rows before this one's counted by a prefix
+        // over both warps (warp 1 counts warp 0's rows again)
+        if (t < 64) {
+            const int lane = t & 31;
+            auto count = [&](const CubeRow& c) {
+                int nt = 0;
+                for (uint32_t k = c.mask; k; k &= k - 1) nt += s.ntri[cube_case(c, __ffs(k) - 1)];
+                __syncwarp();
+                return nt;
+            };
+            const CubeRow c = cube_row(s, t & 7, t >> 3);
+            const int nt = count(c);
+            int o = nt;
 #pragma unroll
-        for (int h = 0; h < 2; ++h) {
-            const int ci = classify(s, x, y, z + 4 * h);
-            const int nt = ci >= 0 ? c_ntri[ci] : 0;
-            em.cubes[t + kMeshWork * h] = (uint8_t)ci;
-            const int incl = warp_prefix(nt, s);
-            work_barrier();
-            int o = base + incl - nt;
-#pragma unroll
-            for (int w = 0; w < kMeshWork / 32; ++w) {
-                const int ws = s.warp_sum[w];
-                base += ws;
-                if (w < (t >> 5)) o += ws;
+            for (int d = 1; d < 32; d <<= 1) {
+                const int y = __shfl_up_sync(0xffffffffu, o, d);
+                if (lane >= d) o += y;
             }
-            for (int j = 0; j < nt; ++j) em.tri[o + j] = (uint16_t)((t + kMeshWork * h) | j << 9);
-            work_barrier();
+            o -= nt;
+            if (t >= 32) o += __reduce_add_sync(0xffffffffu, count(cube_row(s, lane & 7, lane >> 3)));
+            for (uint32_t k = c.mask; k; k &= k - 1) {
+                const int x = __ffs(k) - 1, vx = 8 * t + x, ci = cube_case(c, x), nc = s.ntri[ci];
+                em.cubes[vx] = (uint8_t)ci;
+                for (int j = 0; j < nc; ++j) em.tri[o + j] = (uint16_t)(vx | j << 9);
+                o += nc;
+            }
         }
-        const int3 g = make_int3(s.pos[buf].x * 8, s.pos[buf].y * 8, s.pos[buf].z * 8);
+        work_barrier();
+        const int3 b8 = make_int3(s.pos[buf].x * 8, s.pos[buf].y * 8, s.pos[buf].z * 8);
         for (int v0 = 0; v0 < 3 * total; v0 += kMeshWork) {
             const int cnt = min(kMeshWork, 3 * total - v0);
             if (t < cnt) {
                 const int id = v0 + t, tr = em.tri[id / 3], vx = tr & 511;
-                edge_vertex(s, em.rgb, vx & 7, (vx >> 3) & 7, vx >> 6, g,
-                            c_tri[em.cubes[vx]][3 * (tr >> 9) + id % 3], m.g.voxel_size, em.v + 3 * t, em.n + 3 * t,
-                            em.c + 3 * t);
+                edge_vertex(s, em.rgb, vx & 7, (vx >> 3) & 7, vx >> 6, b8,
+                            em.table[em.cubes[vx]][3 * (tr >> 9) + id % 3], m.g.voxel_size, em.v + 3 * t,
+                            em.n + 3 * t, em.c + 3 * t);
             }
             work_barrier();
             const size_t o = (size_t)(first * 3 + v0) * 3;
@@ -528,7 +556,7 @@ __global__ void __launch_bounds__(kMeshThreads, kMeshCtas)
     });
 }
 
-size_t mesh_scratch_bytes(int n_blocks) { return 8 * ((size_t)n_blocks + 2) + 4 * (size_t)n_blocks; }
+size_t mesh_scratch_bytes(int n_blocks) { return 8 * ((size_t)n_blocks + 2) + 8 * (size_t)n_blocks; }
 
 // Mesh of the map: *total = triangles found (all of them, also beyond `cap`);
 // the first min(total, cap) are written when V, N and C are given.  scratch:
@@ -541,7 +569,7 @@ int launch_mesh(const MapView& m, void* scratch, float* V, float* N, uint8_t* C,
     if (rc != FB_OK) return rc;
     unsigned long long* const sum = (unsigned long long*)scratch;
     unsigned long long* const offsets = sum + 1;
-    uint32_t* const counts = (uint32_t*)(offsets + m.NS + 1);
+    uint2* const counts = (uint2*)(offsets + m.NS + 1);
     int dev = 0, sms = 0;
     if (cudaGetDevice(&dev) != cudaSuccess ||
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
