@@ -52,12 +52,12 @@ struct fb_batch {
     // mode 2: fused plans by composition, the recorders of a step's frames
     std::map<std::vector<uint64_t>, FusedPlan> fused;
     std::vector<LaunchRecorder> recs;
-    int lanes = 4;
+    int lanes = 4;   // fb_batch_set_lanes
     // the step in flight between fb_batch_submit and fb_batch_collect
     bool pending = false;
     std::vector<fb_session*> pend_ss;
     std::vector<FramePlan> pend_plans;
-    cudaEvent_t pend_done = nullptr;                             // fb_batch_set_lanes
+    cudaEvent_t pend_done = nullptr;
     int last_launches = 0, last_kernels = 0;   // of the last fused step
 };
 
@@ -308,43 +308,132 @@ int ensure_slots(fb_batch* b, int n) {
     return FB_OK;
 }
 
-// The frames of a step on the slot streams (session i on slot i mod
-// kBatchSlots), forked from and joined back into the origin stream.  With
-// capture on, the same calls record one graph.  in: copy each session's input
-// on its slot stream and launch its cached frame graph (mode 0; on the origin
-// stream before the fork, no frame began before the last input had arrived:
-// 0.4 ms of a 3 ms step of 16 ragged sessions), null: issue the kernels
-// (captured into the composite graph, mode 1).
-int issue_step(fb_batch* b, fb_session* const* ss, int n, const FramePlan* plans, const fb_frame_input* in,
-               int* kernels) {
+// The slot streams of a step of n sessions (session i on slot i mod
+// kBatchSlots) start after what the origin stream holds ...
+int fork_slots(fb_batch* b, int n) {
     FB_CUDA(cudaEventRecord(b->fork, b->origin));
-    *kernels = 0;
-    const int used = std::min(n, kBatchSlots);
-    for (int k = 0; k < used; ++k) FB_CUDA(cudaStreamWaitEvent(b->slots[k], b->fork, 0));
-    for (int i = 0; i < n; ++i) {
-        fb_session* s = ss[i];
-        cudaStream_t st = b->slots[i % kBatchSlots];
-        if (in) {
-            unsigned ran = 0;
-            int rc = copy_frame_in(s, in[i].depth, in[i].depth_pitch, in[i].rgb, in[i].rgb_pitch, in[i].on_device, st);
-            if (rc) return rc;
-            rc = enqueue_frame(s, plans[i], st, &ran);
-            if (rc) return rc;
-        } else {
-            unsigned ran = 0;
-            cudaStream_t keep = s->stream;
-            s->stream = st;
-            *kernels += issue_frame(s, plans[i].track, plans[i].fuse, plans[i].render, plans[i].init, &ran);
-            s->stream = keep;
-        }
-        const int rc = fetch_result(s, st);
-        if (rc) return rc;
-    }
-    for (int k = 0; k < used; ++k) {
+    for (int k = 0; k < std::min(n, kBatchSlots); ++k) FB_CUDA(cudaStreamWaitEvent(b->slots[k], b->fork, 0));
+    return FB_OK;
+}
+
+// ... and the origin stream goes on after them.
+int join_slots(fb_batch* b, int n) {
+    for (int k = 0; k < std::min(n, kBatchSlots); ++k) {
         FB_CUDA(cudaEventRecord(b->done[k], b->slots[k]));
         FB_CUDA(cudaStreamWaitEvent(b->origin, b->done[k], 0));
     }
+    return FB_OK;
+}
+
+// Whether the runtime takes a copy of this input as what its flag says it is.
+bool input_fits(const fb_frame_input& in) {
+    for (const void* p : {(const void*)in.depth, (const void*)in.rgb}) {
+        cudaPointerAttributes a;
+        if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
+            cudaGetLastError();
+            return false;
+        }
+        const bool host = a.type == cudaMemoryTypeHost || a.type == cudaMemoryTypeUnregistered;
+        if (in.on_device ? a.type != cudaMemoryTypeDevice : !host) return false;
+    }
+    return true;
+}
+
+int copy_input(fb_batch* b, fb_session* const* ss, const fb_frame_input* in, int i) {
+    return copy_frame_in(ss[i], in[i].depth, in[i].depth_pitch, in[i].rgb, in[i].rgb_pitch, in[i].on_device,
+                         b->slots[i % kBatchSlots]);
+}
+
+// Mode 0, before any frame is planned: the inputs that the runtime may refuse
+// are copied, so that one that is refused ends the call with every session as
+// it was.  copied[i]: session i's was.
+int copy_unsure_inputs(fb_batch* b, fb_session* const* ss, int n, const fb_frame_input* in, std::vector<char>& copied) {
+    copied.assign(n, 0);
+    if (int rc = fork_slots(b, n)) return rc;
+    for (int i = 0; i < n; ++i) {
+        if (input_fits(in[i])) continue;
+        if (int rc = copy_input(b, ss, in, i)) return rc;
+        copied[i] = 1;
+    }
+    return FB_OK;
+}
+
+// Mode 0: each session's input and its cached frame graph on its slot stream,
+// so that its frame waits for its own input alone.  On the origin stream before
+// the fork, no frame began before the last input had arrived (0.4 ms of a 3 ms
+// step of 16 ragged sessions); with all copies issued before the first frame,
+// a step of 40 sessions of 160x120 took 2.48 ms instead of 2.19 (pageable
+// inputs 2.73).  *issued: the sessions whose frames were launched.
+int launch_frames(fb_batch* b, fb_session* const* ss, int n, const fb_frame_input* in, const std::vector<char>& copied,
+                  const FramePlan* plans, int* issued) {
+    for (int i = 0; i < n; ++i) {
+        cudaStream_t st = b->slots[i % kBatchSlots];
+        unsigned ran = 0;
+        if (!copied[i])
+            if (int rc = copy_input(b, ss, in, i)) return rc;
+        if (int rc = enqueue_frame(ss[i], plans[i], st, &ran)) return rc;
+        if (int rc = fetch_result(ss[i], st)) return rc;
+        *issued = i + 1;
+    }
+    return join_slots(b, n);
+}
+
+// Mode 1: the frames' kernels, captured into the composite graph.
+int issue_step(fb_batch* b, fb_session* const* ss, int n, const FramePlan* plans, int* kernels) {
+    if (int rc = fork_slots(b, n)) return rc;
+    *kernels = 0;
+    for (int i = 0; i < n; ++i) {
+        fb_session* s = ss[i];
+        unsigned ran = 0;
+        cudaStream_t keep = s->stream, st = b->slots[i % kBatchSlots];
+        s->stream = st;
+        *kernels += issue_frame(s, plans[i].track, plans[i].fuse, plans[i].render, plans[i].init, &ran);
+        s->stream = keep;
+        if (int rc = fetch_result(s, st)) return rc;
+    }
+    if (int rc = join_slots(b, n)) return rc;
     return check_launch();
+}
+
+int composite_step(fb_batch* b, fb_session* const* ss, int n, const FramePlan* plans) {
+    std::vector<uint64_t> key = composition(ss, n, plans);
+    auto it = b->cache.find(key);
+    if (it == b->cache.end()) {
+        if (b->cache.size() >= kBatchCacheMax) clear_cache(b);
+        cudaGraph_t graph = nullptr;
+        cudaGraphExec_t exec = nullptr;
+        int kernels = 0;
+        FB_CUDA(cudaStreamBeginCapture(b->origin, cudaStreamCaptureModeThreadLocal));
+        int rc = issue_step(b, ss, n, plans, &kernels);
+        cudaError_t e = cudaStreamEndCapture(b->origin, &graph);
+        if (rc == FB_OK && e == cudaSuccess) e = cudaGraphInstantiate(&exec, graph, 0);
+        if (graph) cudaGraphDestroy(graph);
+        if (rc) return rc;
+        FB_CUDA(e);
+        it = b->cache.emplace(key, std::make_pair(exec, kernels)).first;
+        b->captures++;
+    }
+    FB_CUDA(cudaGraphLaunch(it->second.first, b->origin));
+    // kernels per session are not separated in a composite graph: count
+    // them on the first session
+    ss[0]->launches += (uint64_t)it->second.second;
+    return FB_OK;
+}
+
+// A step that stopped with an error: nothing of it is in flight afterwards
+// (the caller may free the inputs), the first `issued` sessions' frames have
+// run and are finished without a result, and the others, planned or not, are
+// as they were before the call.
+void abandon_step(fb_batch* b, fb_session* const* ss, int n, const std::vector<FramePlan>& plans, int issued) {
+    for (cudaStream_t st : b->slots) cudaStreamSynchronize(st);
+    cudaStreamSynchronize(b->origin);
+    for (int i = 0; i < n; ++i) {
+        if (i < issued)
+            finish_frame(ss[i], plans[i], nullptr);
+        else if (i < (int)plans.size())
+            unplan_frame(ss[i]);
+        ss[i]->shared_gpu = false;
+    }
 }
 
 }  // namespace
@@ -453,60 +542,44 @@ int fb_batch_submit(fb_batch* b, fb_session* const* ss, int n, const fb_frame_in
         for (int j = 0; j < i; ++j)
             if (ss[j] == ss[i]) return FB_EINVAL;
     }
-    int rc = FB_OK;
-    // captured and fused steps: inputs first (on the origin stream; the frames
-    // fork after them)
-    for (int i = 0; i < n && b->mode != 0; ++i) {
-        rc = copy_frame_in(ss[i], in[i].depth, in[i].depth_pitch, in[i].rgb, in[i].rgb_pitch, in[i].on_device,
-                           b->origin);
-        if (rc) return rc;
-    }
-    // sessions of a step of more than kBatchSharedMin sessions run the
-    // tracking forms that leave room for the other sessions' frames (their
-    // frame graphs are the ones fb_session_prepare(s, 1) captures); smaller
-    // steps run the forms of a session alone (fb_session_prepare(s, 0)),
-    // which finish sooner.  Both give the same results.
-    // fused steps always run the group forms (clusters do not span the parts
-    // of a fused grid)
-    const bool shared = n > kBatchSharedMin || b->mode == 2;
-    for (int i = 0; i < n; ++i) ss[i]->shared_gpu = shared;
-    std::vector<FramePlan> plans(n);
-    for (int i = 0; i < n; ++i) plans[i] = plan_frame(ss[i]);
-    if (b->mode == 2) {
-        rc = fused_step(b, ss, n, plans.data());
-        if (rc) {
-            for (int i = 0; i < n; ++i) ss[i]->shared_gpu = false;
-            return rc;
-        }
-    } else if (b->mode == 1) {
-        std::vector<uint64_t> key = composition(ss, n, plans.data());
-        auto it = b->cache.find(key);
-        if (it == b->cache.end()) {
-            if (b->cache.size() >= kBatchCacheMax) clear_cache(b);
-            cudaGraph_t graph = nullptr;
-            cudaGraphExec_t exec = nullptr;
-            int kernels = 0;
-            FB_CUDA(cudaStreamBeginCapture(b->origin, cudaStreamCaptureModeThreadLocal));
-            rc = issue_step(b, ss, n, plans.data(), nullptr, &kernels);
-            cudaError_t e = cudaStreamEndCapture(b->origin, &graph);
-            if (rc == FB_OK && e == cudaSuccess) e = cudaGraphInstantiate(&exec, graph, 0);
-            if (graph) cudaGraphDestroy(graph);
-            if (rc) return rc;
-            FB_CUDA(e);
-            it = b->cache.emplace(key, std::make_pair(exec, kernels)).first;
-            b->captures++;
-        }
-        FB_CUDA(cudaGraphLaunch(it->second.first, b->origin));
-        // kernels per session are not separated in a composite graph: count
-        // them on the first session
-        ss[0]->launches += (uint64_t)it->second.second;
-    } else {
-        int kernels = 0;
-        rc = issue_step(b, ss, n, plans.data(), in, &kernels);
-        if (rc) return rc;
-    }
     if (!b->pend_done) FB_CUDA(cudaEventCreateWithFlags(&b->pend_done, cudaEventDisableTiming));
-    FB_CUDA(cudaEventRecord(b->pend_done, b->origin));
+    int rc = FB_OK, issued = 0;
+    std::vector<FramePlan> plans;
+    std::vector<char> copied;
+    // inputs: captured and fused steps' on the origin stream (the frames fork
+    // after them), else with the frames (launch_frames)
+    if (b->mode == 0)
+        rc = copy_unsure_inputs(b, ss, n, in, copied);
+    else
+        for (int i = 0; i < n && rc == FB_OK; ++i)
+            rc = copy_frame_in(ss[i], in[i].depth, in[i].depth_pitch, in[i].rgb, in[i].rgb_pitch, in[i].on_device,
+                               b->origin);
+    if (rc == FB_OK) {
+        // sessions of a step of more than kBatchSharedMin sessions run the
+        // tracking forms that leave room for the other sessions' frames (their
+        // frame graphs are the ones fb_session_prepare(s, 1) captures); smaller
+        // steps run the forms of a session alone (fb_session_prepare(s, 0)),
+        // which finish sooner.  Both give the same results.
+        // fused steps always run the group forms (clusters do not span the parts
+        // of a fused grid)
+        const bool shared = n > kBatchSharedMin || b->mode == 2;
+        plans.resize(n);
+        for (int i = 0; i < n; ++i) {
+            ss[i]->shared_gpu = shared;
+            plans[i] = plan_frame(ss[i]);
+        }
+        rc = b->mode == 2   ? fused_step(b, ss, n, plans.data())
+             : b->mode == 1 ? composite_step(b, ss, n, plans.data())
+                            : launch_frames(b, ss, n, in, copied, plans.data(), &issued);
+    }
+    if (rc == FB_OK && !cuda_ok(cudaEventRecord(b->pend_done, b->origin))) {
+        rc = FB_ECUDA;
+        issued = n;
+    }
+    if (rc) {
+        abandon_step(b, ss, n, plans, issued);
+        return rc;
+    }
     b->pend_ss.assign(ss, ss + n);
     b->pend_plans = std::move(plans);
     b->pending = true;

@@ -666,6 +666,8 @@ FramePlan plan_frame(fb_session* s) {
     return p;
 }
 
+void unplan_frame(fb_session* s) { std::swap(s->state, s->last_state); }
+
 // Captures the graph of a frame of plan p for the session's current frame
 // parity and shared-GPU flag, unless it is cached already.  The capture runs
 // on stream st (nothing executes).

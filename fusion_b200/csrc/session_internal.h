@@ -219,6 +219,7 @@ void unpack_sums(const double* s, double* A, double* b);
 int copy_frame_in(fb_session* s, const uint16_t* depth, size_t depth_pitch, const uint8_t* rgb, size_t rgb_pitch,
                   int on_device, cudaStream_t st);
 FramePlan plan_frame(fb_session* s);
+void unplan_frame(fb_session* s);   // takes back the last plan_frame of a frame that was not issued
 int capture_frame(fb_session* s, const FramePlan& p, cudaStream_t st);
 int enqueue_frame(fb_session* s, const FramePlan& p, cudaStream_t st, unsigned* ran);
 void finish_frame(fb_session* s, const FramePlan& p, fb_frame_result* out);

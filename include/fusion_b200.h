@@ -249,7 +249,10 @@ FB_API int fb_batch_reserve(fb_batch* b, size_t bytes);
  * captured graph.  Results are the same in every mode. */
 FB_API int fb_batch_set_mode(fb_batch* b, int mode);
 /* One frame for each of n distinct sessions; out[i] as fb_grab_frame's.
- * Synchronous.  A session must not be used elsewhere during the call. */
+ * Synchronous.  A session must not be used elsewhere during the call.  A call
+ * that ends with an error leaves nothing in flight; an input that is refused
+ * leaves every session as it was, and where a launch fails in mode 0 the
+ * sessions launched before it have taken their frame and the others have not. */
 FB_API int fb_batch_step(fb_batch* b, fb_session* const* sessions, int n, const fb_frame_input* in,
                          fb_frame_result* out);
 /* fb_batch_step in two halves: submit starts the step and collect waits for
