@@ -89,7 +89,7 @@ void clear_fused(fb_batch* b) {
 }
 
 // The composition of a step: each session with what decides its launches
-// (tracker mode, fusion, frame parity, map form options, raycast tile).
+// (tracker mode, fusion, frame parity, map form options, launch shapes, wait limit).
 std::vector<uint64_t> composition(fb_session* const* ss, int n, const FramePlan* plans) {
     std::vector<uint64_t> key;
     key.reserve(2 * n);
@@ -98,7 +98,8 @@ std::vector<uint64_t> composition(fb_session* const* ss, int n, const FramePlan*
         key.push_back((uint64_t)(uintptr_t)s);
         key.push_back((uint64_t)plans[i].mode | (uint64_t)plans[i].fuse << 2 | (uint64_t)s->next << 3 |
                       (uint64_t)s->shared_gpu << 5 | (uint64_t)s->mapping_disabled << 6 |
-                      (uint64_t)s->rc_bx << 8 | (uint64_t)s->rc_by << 20 | (uint64_t)s->integ_cps << 32);
+                      (uint64_t)s->rc_bx << 8 | (uint64_t)s->rc_by << 20 | (uint64_t)s->integ_cps << 32 |
+                      (uint64_t)s->wait_polls << 40);
     }
     return key;
 }

@@ -198,7 +198,7 @@ enum ErrFlag : uint32_t {
     kErrNewListFull = 1u << 4,        // more new blocks in one frame than the pool
     kErrVisibleFull = 1u << 5,        // visible list capacity exceeded
     kErrSequentialInsert = 1u << 6,   // slow exact path taken (heap/excess edge cases)
-    kErrTimeout = 1u << 7,            // a bounded device-side wait gave up (the kernel stopped early)
+    kErrTimeout = 1u << 7,            // a bounded wait of the tracker gave up (its frame is not tracked)
     kErrNormalW = 1u << 8,            // a valid normal given to integration had a w lane other than 1
 };
 

@@ -103,8 +103,10 @@ int launch_track_begin(TrackState* st, TrackSync* sync, const int iters[3], cuda
 // All Gauss-Newton iterations of a frame (lv, iters and min_count by pyramid
 // level; list: track_list_bytes of level 0) in one launch; 0 launches when the sizes do not fit it (the caller
 // then launches the iterations one by one; the results are the same).
+// polls: the limit of its waits for other blocks (fb_session_set_wait_limit).
 int launch_track_loop(const TrackLevel lv[3], const int iters[3], const int min_count[3], TrackState* st,
-                      TrackSync* sync, void* list, cudaStream_t s, bool compensated);
+                      TrackSync* sync, void* list, cudaStream_t s, bool compensated, int polls);
+constexpr int kWaitPolls = 1 << 18;
 // residual: per-warp compact segments of photometric correspondences
 // (int2: the pixel's Sobel derivatives dx | dy << 16, packed last pixel + difference), track_list_bytes;
 // counts: entries per segment (kTrackMaxBlocks * kTrackWarps ints)

@@ -68,23 +68,27 @@ FB_FUSED_KERNEL(k_init_poses, init_poses_body, 32)
 // After the frame: a tracked frame becomes the last frame (SwapFrame), and the
 // frame's result goes to `out` -- the session's pinned host memory where the
 // device can write it (a copy of the 184 bytes after the kernel took 3 us and
-// a gap of 6), else device memory.  64 threads.
+// a gap of 6), else device memory.  A tracker whose waits gave up (failed bit
+// 1) may have left a pose and errors of incomplete sums: the frame reports the
+// last pose and no errors, and kErrTimeout.  64 threads.
 __device__ __forceinline__ void commit_body(const BlockCtx&, TrackState* st, MapCounters* c, FrameOut* out,
                                             int tracked_path) {
     const int t = threadIdx.x;
+    const bool gave_up = tracked_path && (st->failed & 2);
     if (t < 16) {
-        const double v = st->pose[t];
+        const double v = gave_up ? st->last_pose[t] : st->pose[t];
         out->pose[t] = v;
         if (tracked_path && !st->failed) st->last_pose[t] = v;
     } else if (t < 16 + (int)(sizeof(DevPose) / 4)) {
         if (tracked_path && !st->failed) ((float*)&st->last)[t - 16] = ((const float*)&st->cur)[t - 16];
     } else if (t == 40) {
         out->failed = st->failed;
-        out->icp_error = st->icp_error;
-        out->icp_count = st->icp_count;
-        out->rgb_error = st->rgb_error;
-        out->rgb_count = st->rgb_count;
+        out->icp_error = gave_up ? qnan() : st->icp_error;
+        out->icp_count = gave_up ? 0.f : st->icp_count;
+        out->rgb_error = gave_up ? qnan() : st->rgb_error;
+        out->rgb_count = gave_up ? 0.f : st->rgb_count;
     } else if (t == 41) {
+        if (gave_up) c->err |= kErrTimeout;
         out->n_alloc = c->n_alloc;
         out->n_visible = c->n_visible;
         out->n_new = c->n_new;
@@ -444,7 +448,8 @@ int issue_frame(fb_session* s, bool track, bool fuse, bool render, bool init, un
         const TrackLevel lv[3] = {level_view(s, 0), level_view(s, 1), level_view(s, 2)};
         const bool comp = c.form == FB_FORM_PRECISION;
         const int one =
-            s->shared_gpu ? 0 : launch_track_loop(lv, c.iters, min_count, s->st, s->track_sync, s->residual, st, comp);
+            s->shared_gpu ? 0 : launch_track_loop(lv, c.iters, min_count, s->st, s->track_sync, s->residual, st, comp,
+                                             s->wait_polls);
         n += one;
         int last_level = -1;
         for (int l = 2; l >= 0; --l)
@@ -879,6 +884,7 @@ int fb_session_create(const fb_config* cfg, void* stream, fb_session** out) {
     s->rc_bx = 16;
     s->rc_by = 8;
     s->integ_cps = 0;
+    s->wait_polls = kWaitPolls;
     s->shared_gpu = false;
     for (int a = 0; a < 3; ++a)
         for (int b = 0; b < 2; ++b)
@@ -1071,6 +1077,14 @@ int fb_session_set_integration_grid(fb_session* s, int ctas_per_sm) {
     if (ctas_per_sm == s->integ_cps) return FB_OK;
     drop_graphs(s);
     s->integ_cps = ctas_per_sm;
+    return FB_OK;
+}
+
+int fb_session_set_wait_limit(fb_session* s, int polls) {
+    if (!s || polls < 0 || polls > kWaitPolls) return FB_EINVAL;
+    if (polls == s->wait_polls) return FB_OK;
+    drop_graphs(s);
+    s->wait_polls = polls;
     return FB_OK;
 }
 

@@ -135,6 +135,7 @@ struct fb_session {
     DevPose* scratch_pose;
     char* mesh_scratch;        // triangle counts and offsets of the pool's blocks (launch_mesh)
     std::mutex mesh_lock;      // held while a mesh uses it
+    int wait_polls;            // fb_session_set_wait_limit
     FrameOut* d_out;
     FrameOut* h_out;           // pinned
     FrameOut* h_out_dev;       // h_out's device address (cudaHostGetDevicePointer), null if none

@@ -1161,11 +1161,11 @@ __global__ void __launch_bounds__(256, kMinBlocks)
 // loaded as one 128-bit access each, so a slot that holds the expected epoch
 // holds its data: no fences, tickets or second round trips.  A slot is
 // rewritten only after everyone who needs its last value has published
-// something that the rewriting waits for.  Every wait is bounded; a wait that
-// gives up fails the frame (failed bit 1) and its block leaves.
+// something that the rewriting waits for.  Every wait is bounded (LoopArgs::
+// polls); a wait that gives up fails the frame (failed bit 1, reported by
+// k_commit as kErrTimeout with the last pose) and its block leaves.
 // The blocks must be resident together, hence the cooperative launch and the
 // size rule of launch_track_loop.
-constexpr int kLoopPolls = 1 << 18;
 constexpr int kLoopRows = 80;                       // blocks of one group range, at most
 constexpr int kLoopMaxBuf = 12;
 constexpr int kLoopScratch = kLoopRows / kTrackCluster * 32 * 8 + kLoopRows * 30 * 4;   // cluster 0's sums (14720)
@@ -1184,6 +1184,7 @@ struct LoopStage {
 struct LoopArgs {
     TrackLevel L[3];
     int iters[3], min_count[3], G[3];
+    int polls;     // loads of an exchanged value before its wait gives up
     int nbuf;      // chunk buffers
     int chunks;    // chunks of a block, at most (the list's capacity)
     unsigned char* list;   // the lists in global memory (kGlobalList)
@@ -1219,9 +1220,9 @@ __device__ __forceinline__ uint4 slot_get(const TrackSlot* p) {
     return v;
 }
 
-// Waits until the slot holds exchange e; false after kLoopPolls loads.
-__device__ __forceinline__ bool slot_wait(const TrackSlot* p, uint32_t e, uint4& v) {
-    for (int i = 0; i < kLoopPolls; ++i) {
+// Waits until the slot holds exchange e; false after `polls` loads.
+__device__ __forceinline__ bool slot_wait(const TrackSlot* p, uint32_t e, int polls, uint4& v) {
+    for (int i = polls; i > 0; --i) {
         v = slot_get(p);
         if (v.w == e) return true;
     }
@@ -1255,7 +1256,8 @@ __device__ __forceinline__ void loop_fill(LoopStage& S, uint64_t* bar, const Tra
 // ((double*)scratch)[group * 32 + value].  Whole block; false in a thread
 // whose wait gave up.
 template <bool kComp>
-__device__ __forceinline__ bool range_sums(unsigned char* scratch, const TrackSlot* src, int ng, uint32_t e) {
+__device__ __forceinline__ bool range_sums(unsigned char* scratch, const TrackSlot* src, int ng, uint32_t e,
+                                           int polls) {
     constexpr int kRowsAtOnce = 25;   // 25 x 10 slots by 250 threads
     const int t = threadIdx.x, nb = ng * kTrackCluster;
     float* const S = (float*)(scratch + kLoopRows / kTrackCluster * 32 * 8);
@@ -1271,7 +1273,7 @@ __device__ __forceinline__ bool range_sums(unsigned char* scratch, const TrackSl
         for (int j = 0; j < (kLoopRows + kRowsAtOnce - 1) / kRowsAtOnce; ++j) {
             const int r = row + kRowsAtOnce * j;
             if (r < nb) {
-                if (v[j].w != e) ok &= slot_wait(src + (size_t)r * kSumSlots, e, v[j]);
+                if (v[j].w != e) ok &= slot_wait(src + (size_t)r * kSumSlots, e, polls, v[j]);
                 float* o = S + r * 30 + 3 * col;
                 o[0] = __uint_as_float(v[j].x);
                 o[1] = __uint_as_float(v[j].y);
@@ -1387,7 +1389,7 @@ __global__ void __cluster_dims__(kTrackCluster, 1, 1) __launch_bounds__(256, 2)
                     // had no pixels, says so under an earlier number
                     uint4 v;
                     bool got = false;
-                    for (int i = 0; i < kLoopPolls && !got; ++i) {
+                    for (int i = A.polls; i > 0 && !got; --i) {
                         v = slot_get(&sync->pose[b % kPoseCopies][lane & 7]);
                         const bool lost = (lane & 7) == 7 && v.x != 0 && v.w - base - 1u < total;
                         if (__any_sync(0xffffffffu, lost)) {
@@ -1505,7 +1507,10 @@ __global__ void __cluster_dims__(kTrackCluster, 1, 1) __launch_bounds__(256, 2)
             uint32_t tc = 0, tq = 0;   // at most three blocks' sums per thread: below 2^32
             for (int j = t; j < G; j += 256) {
                 uint4 v;
-                if (!slot_wait(&sync->count[j], e + 1, v)) bad = 1;
+                if (!slot_wait(&sync->count[j], e + 1, A.polls, v)) {
+                    bad = 1;
+                    continue;
+                }
                 tc += v.x;
                 tq += v.y;
             }
@@ -1559,7 +1564,7 @@ __global__ void __cluster_dims__(kTrackCluster, 1, 1) __launch_bounds__(256, 2)
             const int NG = G / kTrackCluster, per = (NG + 3) / 4, g0 = b * per;
             const int ng = max(0, min(NG, g0 + per) - g0);
             for (int pass = 0; pass < 2; ++pass) {
-                bad |= !range_sums<kComp>(scratch, &sync->sums[g0 * kTrackCluster][10 * pass], ng, e);
+                bad |= !range_sums<kComp>(scratch, &sync->sums[g0 * kTrackCluster][10 * pass], ng, e, A.polls);
                 if (t < 32) {
                     double* dst = (double*)cl.map_shared_rank(&s_part[0][0], 0) + b * 64 + 32 * pass + t;
                     if constexpr (kComp) {
@@ -1853,9 +1858,10 @@ bool track_list_global(int n) {
 
 // k_track_loop's launch for these levels, when its grid is resident at once.
 int launch_track_loop(const TrackLevel lv[3], const int iters[3], const int min_count[3], TrackState* st,
-                      TrackSync* sync, void* list, cudaStream_t s, bool compensated) {
+                      TrackSync* sync, void* list, cudaStream_t s, bool compensated, int polls) {
     if (launch_recorder()) return 0;
     LoopArgs A{};
+    A.polls = polls;
     int grid = 0, chunks = 0;
     bool global = false;
     for (int l = 0; l < 3; ++l) {

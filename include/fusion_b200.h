@@ -49,7 +49,7 @@ extern "C" {
 #define FB_ERR_NEW_LIST_FULL 0x10u    /* more new blocks in one frame than the pool */
 #define FB_ERR_VISIBLE_FULL 0x20u     /* visible list full */
 #define FB_ERR_SEQUENTIAL_INSERT 0x40u /* pool/excess edge case: exact sequential insert used */
-#define FB_ERR_TIMEOUT 0x80u          /* a bounded device-side wait (a staged copy) gave up; integration stopped */
+#define FB_ERR_TIMEOUT 0x80u          /* a bounded device-side wait of the tracker gave up: the frame was not tracked */
 #define FB_ERR_NORMAL_W 0x100u        /* fb_fuse_map_color: a valid normal's w lane was not 1 (ComputeNMap's) */
 
 /* Runtime form of the reference's compile-time constants:
@@ -194,6 +194,13 @@ FB_API int fb_session_set_raycast_tile(fb_session* s, int bx, int by);
  * on it.  Cached frame graphs are rebuilt on the next frame.  No reference
  * counterpart: a tuning knob for the batched form's autotuner. */
 FB_API int fb_session_set_integration_grid(fb_session* s, int ctas_per_sm);
+/* The limit of the tracking kernel's waits for its other blocks, in polls of
+ * a value (0 .. 262144, the default: some hundred milliseconds; 0: every wait
+ * gives up at once).  A wait that gives up ends the kernel: the frame is not
+ * tracked, keeps the last pose, and FB_ERR_TIMEOUT is set.  Cached frame
+ * graphs are rebuilt on the next frame.  No reference counterpart: lets a
+ * program try its handling of such a frame without a fault of the GPU. */
+FB_API int fb_session_set_wait_limit(fb_session* s, int polls);
 
 /* Snapshots (System::WriteMapToDisk / ReadMapFromDisk, Core/System.cc:195-271,
  * in memory and with the tracker included): everything a session needs to
