@@ -870,6 +870,8 @@ int fb_session_create(const fb_config* cfg, void* stream, fb_session** out) {
     *out = nullptr;
     fb_session* s = new (std::nothrow) fb_session();
     if (!s) return FB_ENOMEM;
+    static std::atomic<uint64_t> sessions{0};
+    s->id = ++sessions;
     s->cfg = *cfg;
     s->h_out = nullptr;
     s->h_out_dev = nullptr;

@@ -117,6 +117,7 @@ struct Pose16 {
 using namespace fb;
 
 struct fb_session {
+    uint64_t id;               // of this session alone (addresses come again after fb_session_destroy)
     fb_config cfg;
     cudaStream_t stream;
     bool own_stream;

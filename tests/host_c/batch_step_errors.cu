@@ -76,6 +76,7 @@ static void report(const char* name) {
 }
 
 static std::vector<fb_frame_input> inputs;
+static uint64_t last_id;
 static uint16_t depth, depth_k;
 static uint8_t rgb;
 static void reset(int n) {
@@ -83,6 +84,7 @@ static void reset(int n) {
     pop.clear();
     for (int i = 0; i < n; ++i) {
         fb_session* s = new fb_session();
+        s->id = ++last_id;
         s->W[0] = 16;
         s->H[0] = 16;
         s->state = 3;        // told apart from the last state by value only
@@ -169,5 +171,21 @@ int main() {
             }
         }
     report("other_modes");
+    {
+        // a session made where a destroyed one was takes no graph of it
+        uint64_t steps, before, again, other;
+        check(fb_batch_set_mode(b, 1) == FB_OK);
+        reset(2);
+        check(good_step(b, 2));
+        fb_batch_stats(b, &steps, &before);
+        check(good_step(b, 2));
+        fb_batch_stats(b, &steps, &again);
+        check(again == before);
+        pop[0]->id = ++last_id;
+        check(good_step(b, 2));
+        fb_batch_stats(b, &steps, &other);
+        check(other == before + 1);
+    }
+    report("same_address");
     return 0;
 }

@@ -2,7 +2,8 @@
 batch code with fakes of the runtime and of the session functions): an input
 the runtime refuses leaves every session as it was, a frame that cannot be
 launched leaves the frames before it finished and the others as they were,
-nothing stays in flight, and the next step runs."""
+nothing stays in flight, and the next step runs.  A session made at the address
+of a destroyed one is another session to a batch's cached graphs."""
 import os
 import shutil
 import subprocess
@@ -24,6 +25,6 @@ def test_errors(tmp_path):
                            os.path.join(HERE, "host_c", "fake_cudart.cpp")])
     out = subprocess.run([str(exe)], capture_output=True, text=True, check=True, timeout=120).stdout
     rows = {line.split()[0]: [int(v) for v in line.split()[1:]] for line in out.splitlines()}
-    assert set(rows) == {"refused_input", "failed_launch", "other_modes"}, out
+    assert set(rows) == {"refused_input", "failed_launch", "other_modes", "same_address"}, out
     for name, (runs, failures) in rows.items():
         assert runs > 0 and failures == 0, (name, runs, failures)
