@@ -623,7 +623,7 @@ __global__ void __launch_bounds__(32 * kQG * kParts) k_match2(const float* __res
     constexpr int kQueries = kQG * kTQ, kTile = 32 * kMatchTrains * kParts;
     extern __shared__ __align__(16) float dyn_match[];
     float* const sq = dyn_match;                                  // [value][query], negated
-    float* const st = dyn_match + kKeyDesc * kQueries;            // two tiles
+    float* const st = dyn_match + kKeyDesc * kQueries;            // two tiles, or the one there is
     __shared__ Best2 s_best[kQG * kParts][kTQ];
     __shared__ Best2 s_cta[kQueries];
     cg::cluster_group cl = cg::this_cluster();
@@ -638,65 +638,70 @@ __global__ void __launch_bounds__(32 * kQG * kParts) k_match2(const float* __res
         const int r = t % kQueries, c = t / kQueries;
         sq[t] = q0 + r < nq ? -Q[(size_t)(q0 + r) * kKeyDesc + c] : 0.f;
     }
-    if (rank < tiles) stage_rows(st, T, rank * kTile, kTile, nt);
+    // rows of the tiles that a warp works on (parts beyond the last train are left out)
+    constexpr int kPart = 32 * kMatchTrains;
+    auto rows_of = [&](int tile) { return min(kTile, (nt - tile * kTile + kPart - 1) / kPart * kPart); };
+    if (rank < tiles) stage_rows(st, T, rank * kTile, rows_of(rank), nt);
     int buf = 0;
     for (int tile = rank; tile < tiles; tile += ranks, buf ^= 1) {
         if (tile + ranks < tiles) {
-            stage_rows(st + (buf ^ 1) * kTile * kMatchRow, T, (tile + ranks) * kTile, kTile, nt);
+            stage_rows(st + (buf ^ 1) * kTile * kMatchRow, T, (tile + ranks) * kTile, rows_of(tile + ranks), nt);
             asm volatile("cp.async.wait_group 1;" ::: "memory");
         } else {
             asm volatile("cp.async.wait_group 0;" ::: "memory");
         }
         __syncthreads();
-        const float* const qp = sq + qg * kTQ;
-        const float* const tp = st + (buf * kTile + part * 32 * kMatchTrains + lane) * kMatchRow;
-        unsigned long long acc2[kTQ / 2][kMatchTrains] = {};
+        const int t0 = tile * kTile + part * kPart + lane;
+        if (t0 - lane < nt) {   // the warp has trains
+            const float* const qp = sq + qg * kTQ;
+            const float* const tp = st + (buf * kTile + part * kPart + lane) * kMatchRow;
+            unsigned long long acc2[kTQ / 2][kMatchTrains] = {};
 #pragma unroll 4
-        for (int c = 0; c < kKeyDesc; c += 4) {
-            float4 t[kMatchTrains];
+            for (int c = 0; c < kKeyDesc; c += 4) {
+                float4 t[kMatchTrains];
 #pragma unroll
-            for (int b = 0; b < kMatchTrains; ++b)
-                t[b] = *reinterpret_cast<const float4*>(tp + 32 * b * kMatchRow + c);
+                for (int b = 0; b < kMatchTrains; ++b)
+                    t[b] = *reinterpret_cast<const float4*>(tp + 32 * b * kMatchRow + c);
 #pragma unroll
-            for (int e = 0; e < 4; ++e) {
-                unsigned long long q[kTQ / 2];
-                if constexpr (kTQ == 4) {
-                    const ulonglong2 v = *reinterpret_cast<const ulonglong2*>(qp + (c + e) * kQueries);
-                    q[0] = v.x;
-                    q[kTQ / 2 - 1] = v.y;
-                } else {
-                    q[0] = *reinterpret_cast<const unsigned long long*>(qp + (c + e) * kQueries);
-                }
+                for (int e = 0; e < 4; ++e) {
+                    unsigned long long q[kTQ / 2];
+                    if constexpr (kTQ == 4) {
+                        const ulonglong2 v = *reinterpret_cast<const ulonglong2*>(qp + (c + e) * kQueries);
+                        q[0] = v.x;
+                        q[kTQ / 2 - 1] = v.y;
+                    } else {
+                        q[0] = *reinterpret_cast<const unsigned long long*>(qp + (c + e) * kQueries);
+                    }
 #pragma unroll
-                for (int b = 0; b < kMatchTrains; ++b) {
-                    const unsigned long long tt = twice(e == 0 ? t[b].x : e == 1 ? t[b].y : e == 2 ? t[b].z : t[b].w);
+                    for (int b = 0; b < kMatchTrains; ++b) {
+                        const unsigned long long tt = twice(e == 0 ? t[b].x : e == 1 ? t[b].y : e == 2 ? t[b].z : t[b].w);
 #pragma unroll
-                    for (int a = 0; a < kTQ / 2; ++a) add_square(acc2[a][b], tt, q[a]);
+                        for (int a = 0; a < kTQ / 2; ++a) add_square(acc2[a][b], tt, q[a]);
+                    }
                 }
             }
-        }
-        float acc[kTQ][kMatchTrains];
+            float acc[kTQ][kMatchTrains];
 #pragma unroll
-        for (int a = 0; a < kTQ / 2; ++a)
+            for (int a = 0; a < kTQ / 2; ++a)
 #pragma unroll
-            for (int b = 0; b < kMatchTrains; ++b)
-                asm("mov.b64 {%0, %1}, %2;" : "=f"(acc[2 * a][b]), "=f"(acc[2 * a + 1][b]) : "l"(acc2[a][b]));
-        // a lane's trains come in ascending order: a tie keeps the earlier
-        const int t0 = tile * kTile + part * 32 * kMatchTrains + lane;
+                for (int b = 0; b < kMatchTrains; ++b)
+                    asm("mov.b64 {%0, %1}, %2;" : "=f"(acc[2 * a][b]), "=f"(acc[2 * a + 1][b]) : "l"(acc2[a][b]));
+            // a lane's trains come in ascending order: a tie keeps the earlier
 #pragma unroll
-        for (int b = 0; b < kMatchTrains; ++b) {
-            const int ti = t0 + 32 * b;
-            if (ti >= nt) break;
+            for (int b = 0; b < kMatchTrains; ++b) {
+                const int ti = t0 + 32 * b;
+                if (ti >= nt) break;
 #pragma unroll
-            for (int a = 0; a < kTQ; ++a) {
-                const float v = acc[a][b];
-                if (v < best[a].d2) {
-                    const bool first = v < best[a].d1;
-                    best[a].d2 = first ? best[a].d1 : v;
-                    best[a].i2 = first ? best[a].i1 : ti;
-                    if (first) {
-                        best[a].d1 = v;
-                        best[a].i1 = ti;
+                for (int a = 0; a < kTQ; ++a) {
+                    const float v = acc[a][b];
+                    if (v < best[a].d2) {
+                        const bool first = v < best[a].d1;
+                        best[a].d2 = first ? best[a].d1 : v;
+                        best[a].i2 = first ? best[a].i1 : ti;
+                        if (first) {
+                            best[a].d1 = v;
+                            best[a].i1 = ti;
+                        }
                     }
                 }
             }
@@ -830,7 +835,10 @@ int launch_backproject(const KeyScratch& ks, int n, const float* depth, int dp, 
 // queries x 256 trains by 256 threads for fewer queries than fill the chip so.
 // The cluster size is the one whose waves of resident clusters take the
 // fewest tiles (clusters of 5 leave SMs of a GPC unused, and so on: the
-// runtime knows how many of a size are resident).
+// runtime knows how many of a size are resident).  Trains of one tile: the small
+// shape, with shared memory for the rows there are, so that three or four CTAs
+// share an SM (a call of 3000 queries x 100 trains 26 us; with the two buffers
+// of the other shapes, one CTA per SM, 37).
 int launch_match2(const float* q, int nq, const float* t, int nt, int2* idx, float2* dist, cudaStream_t st) {
     if (nq <= 0) return FB_OK;
     constexpr int kTile = 256;
@@ -839,9 +847,10 @@ int launch_match2(const float* q, int nq, const float* t, int nt, int2* idx, flo
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
         return FB_ECUDA;
     const int tiles = (nt + kTile - 1) / kTile;
-    const bool wide = (nq + 31) / 32 * std::min(8, std::max(tiles, 1)) >= sms;
+    const bool wide = tiles > 1 && (nq + 31) / 32 * std::min(8, tiles) >= sms;
     const int queries = wide ? 32 : 8, threads = wide ? 512 : 256, groups = (nq + queries - 1) / queries;
-    const size_t smem = ((size_t)queries * kKeyDesc + 2 * kTile * kMatchRow) * sizeof(float);
+    auto smem_of = [&](int rows) { return ((size_t)queries * kKeyDesc + (size_t)rows * kMatchRow) * sizeof(float); };
+    const size_t smem = smem_of(2 * kTile);
     const void* k = wide ? (const void*)k_match2<4, 8, 2> : (const void*)k_match2<2, 4, 2>;
     cudaLaunchConfig_t cfg = {};
     cfg.blockDim = dim3(threads);
@@ -880,6 +889,7 @@ int launch_match2(const float* q, int nq, const float* t, int nt, int2* idx, flo
     }
     at[0].val.clusterDim.x = (unsigned)ranks;
     cfg.gridDim = dim3((unsigned)(groups * ranks));
+    if (tiles <= 1) cfg.dynamicSmemBytes = smem_of((nt + 127) / 128 * 128);
     cfg.stream = st;
     void* args[] = {&q, &nq, &t, &nt, &idx, &dist};
     return cudaLaunchKernelExC(&cfg, k, args) == cudaSuccess ? FB_OK : FB_ECUDA;
