@@ -471,15 +471,15 @@ int issue_frame(fb_session* s, bool track, bool fuse, bool render, bool init, un
         // Mapping::FuseColor(LastFrame) after the swap (Mapping.cc:76-90):
         // raw depth, colour and level-0 normals of the frame just tracked
         launch_slot(kSlotAllocate);
-        n += launch_allocate(s->map, N.raw, s->W[0], s->W[0], s->H[0], s->K[0], pose, skip, st, render);
+        // (the z ranges and the dense block index of the raycast that follows,
+        // as it does every fused frame, are made on the way)
+        n += launch_allocate(s->map, N.raw, s->W[0], s->W[0], s->H[0], s->K[0], pose, skip, st, true);
         mark(4);
         launch_slot(kSlotVisibility);
-        // a rendered frame's z ranges and dense block index are made on the way
-        n += render ? launch_view(s->map, s->W[0], s->H[0], s->K[0], pose, skip, st, tiles)
-                    : launch_visibility(s->map, s->W[0], s->H[0], s->K[0], pose, skip, st, true);
+        n += launch_view(s->map, s->W[0], s->H[0], s->K[0], pose, skip, st, tiles);
         mark(5);
         launch_slot(kSlotIntegrate);
-        n += launch_integrate(s->map, s->W[0], s->H[0], s->K[0], pose, skip, st, s->integ_cps, render);
+        n += launch_integrate(s->map, s->W[0], s->H[0], s->K[0], pose, skip, st, s->integ_cps, true);
         *ran |= 7u << 3;
     } else {
         mark(4);
