@@ -290,8 +290,12 @@ int fused_step(fb_batch* b, fb_session* const* ss, int n, const FramePlan* plans
 }
 
 
-// Steps of at most this many sessions run each frame as a session alone
-// (served p50 at 64 clients on B200: 2.50 ms with 1, 2.25 with 2, 1.67 with 3).
+// Steps of at most this many sessions run each frame as a session alone.  The
+// tracking loops of several sessions run one after another from 320x240 up
+// (each wants nearly every cluster slot), the group forms beside each other.
+// us a step with the loop / with the group forms, at 160x120, 320x240, 640x480:
+// two sessions 322/636, 536/780, 900/1455; three 351/666, 760/873, 1235/1607;
+// four 475/702, 994/907, 1579/1703; six 559/790, 1433/1000, 2310/2025.
 constexpr int kBatchSharedMin = 3;
 
 int ensure_slots(fb_batch* b, int n) {

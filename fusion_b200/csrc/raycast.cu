@@ -727,8 +727,8 @@ __global__ void __launch_bounds__(128, 8) k_raycast(MapView m, float4* __restric
                                                  const int* __restrict__ skip) {
     raycast_body<VR>(own_ctx(), m, vmap, nmap, vp, W, H, k, posep, skip);
 }
-// (the fused form keeps the compiler's register count: its spills at nine
-// CTAs per SM cost more in batched steps than the occupancy gains)
+// (the fused form keeps the compiler's register count, seven CTAs per SM: with
+// eight, fused steps of 8 and 16 ragged sessions took the same time within 1 %)
 template <class VR>
 __global__ void __launch_bounds__(128)
     k_raycast_fused(const __grid_constant__ FusedParams<ArgsOf<decltype(&k_raycast<VR>)>> fp) {

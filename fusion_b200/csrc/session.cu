@@ -631,9 +631,10 @@ cudaGraphExec_t take_exec(const ExecKey& key) {
 namespace fb {
 
 // One image of H rows of `row` bytes into dense device memory.  Dense sources
-// go as one linear copy: the copy engine takes a 2-D copy row by row and moved
-// pinned rows of 854 to 1920 bytes at 8-27 GB/s (a 640x480 frame's two images
-// 115 us, a 427x319 frame's 86 us), a linear copy of them at PCIe rate.
+// go as one linear copy: the copy engine takes a 2-D copy row by row, which
+// costs where rows are short or odd (both images from pinned memory: 160x120 37
+// us, 17 as linear copies; 427x319 88, 25-42); from 640x480 up the bus bounds
+// both (41-99 us by the box).
 static cudaError_t copy_rows(void* dst, const void* src, size_t pitch, size_t row, size_t H, cudaMemcpyKind kind,
                              cudaStream_t st) {
     if (pitch == row) return cudaMemcpyAsync(dst, src, row * H, kind, st);
