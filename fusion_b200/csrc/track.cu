@@ -1161,8 +1161,8 @@ __global__ void __launch_bounds__(256, kMinBlocks)
 // loaded as one 128-bit access each, so a slot that holds the expected epoch
 // holds its data: no fences, tickets or second round trips.  A slot is
 // rewritten only after everyone who needs its last value has published
-// something that the rewriting waits for.  Every wait is bounded (LoopArgs::
-// polls); a wait that gives up fails the frame (failed bit 1, reported by
+// something that the rewriting waits for.  Every wait is bounded (kWaitPolls;
+// for counts and sums LoopArgs::polls); a wait that gives up fails the frame (failed bit 1, reported by
 // k_commit as kErrTimeout with the last pose) and its block leaves.
 // The blocks must be resident together, hence the cooperative launch and the
 // size rule of launch_track_loop.
@@ -1184,7 +1184,7 @@ struct LoopStage {
 struct LoopArgs {
     TrackLevel L[3];
     int iters[3], min_count[3], G[3];
-    int polls;     // loads of an exchanged value before its wait gives up
+    int polls;     // loads of a count or sum before its wait gives up
     int nbuf;      // chunk buffers
     int chunks;    // chunks of a block, at most (the list's capacity)
     unsigned char* list;   // the lists in global memory (kGlobalList)
@@ -1386,10 +1386,11 @@ __global__ void __cluster_dims__(kTrackCluster, 1, 1) __launch_bounds__(256, 2)
             if (e != base && b != 0) {
                 if (wid == 0) {
                     // a frame that failed at a coarser level, where this block
-                    // had no pixels, says so under an earlier number
+                    // had no pixels, says so under an earlier number (the limit
+                    // is constant here: a variable one spills)
                     uint4 v;
                     bool got = false;
-                    for (int i = A.polls; i > 0 && !got; --i) {
+                    for (int i = 0; i < kWaitPolls && !got; ++i) {
                         v = slot_get(&sync->pose[b % kPoseCopies][lane & 7]);
                         const bool lost = (lane & 7) == 7 && v.x != 0 && v.w - base - 1u < total;
                         if (__any_sync(0xffffffffu, lost)) {

@@ -194,9 +194,9 @@ FB_API int fb_session_set_raycast_tile(fb_session* s, int bx, int by);
  * on it.  Cached frame graphs are rebuilt on the next frame.  No reference
  * counterpart: a tuning knob for the batched form's autotuner. */
 FB_API int fb_session_set_integration_grid(fb_session* s, int ctas_per_sm);
-/* The limit of the tracking kernel's waits for its other blocks, in polls of
- * a value (0 .. 262144, the default: some hundred milliseconds; 0: every wait
- * gives up at once).  A wait that gives up ends the kernel: the frame is not
+/* The limit of the tracking kernel's waits for its other blocks' sums, in
+ * polls of a value (0 .. 262144, the default: some hundred milliseconds; 0: they
+ * give up at once).  A wait that gives up ends the kernel: the frame is not
  * tracked, keeps the last pose, and FB_ERR_TIMEOUT is set.  Cached frame
  * graphs are rebuilt on the next frame.  No reference counterpart: lets a
  * program try its handling of such a frame without a fault of the GPU. */

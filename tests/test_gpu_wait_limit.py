@@ -1,5 +1,5 @@
 """The waits of the tracking kernel's blocks for one another end: with a limit
-of no polls every wait gives up, the kernel returns, and the frame is reported
+of no polls every wait for sums gives up, the kernel returns, and the frame is reported
 as not tracked with FB_ERR_TIMEOUT and the last pose.  The frames that follow
 are those of a session whose tracker failed that frame by its counts (a frame
 without depth), bit for bit: alone, and beside another session in a batch step.
